@@ -132,6 +132,19 @@ __device__ __forceinline__ V qrot(const Q& q, const V& p) {
   return V{r.x, r.y, r.z};
 }
 
+// Three-input float min/max (PTX ISA 8.8, sm_100 and later); same NaN rules as
+// the two-input forms.
+__device__ __forceinline__ float fmin3f(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float fmax3f(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 struct Tf { Q R; V t; };
 
 // Transform composition T1 * T2 (Transform.tcc:34-42): t = R1*t2 + t1, R = R1*R2.
@@ -161,53 +174,58 @@ __device__ __forceinline__ Tf load_tf(const rmg_transform& T) {
 // inputs, as the paper prescribes.
 // Accepts 0 < t <= tfar, both windings.
 // ----------------------------------------------------------------------------
+// The test runs for the few lanes of a warp that stand at a leaf (5 to 7 of 32
+// on the 1M-triangle terrain), so what bounds it is its instruction count.  The
+// vertices are read component by component, at byte offsets that put the ray's
+// axes in (kx, ky, kz) order, and the origin is kept in that order: nine 4-byte
+// loads in place of three 16-byte ones and 18 selects with their predicates.
+// 128 x 1024 rays on that terrain, ranges: 3,759 -> 3,340 warp instructions per
+// 32 rays, 200 poses with all attributes 3,459 -> 3,170 us; 500 scans of a 16 x
+// 360 lidar in the box room 353 -> 324 us, 64 x 10,000 scattered directions on a
+// 525,000-triangle terrain 216 -> 184 us.
 struct RayW {
-  float ox, oy, oz;
-  int kx, ky, kz;
+  float ox, oy, oz;        // origin components kx, ky, kz
+  uint32_t bx, by, bz;     // byte offsets of components kx, ky, kz in a vertex
   float Sx, Sy, Sz;
 };
 
-__device__ __forceinline__ float comp(const float3& v, int k) {
-  return k == 0 ? v.x : (k == 1 ? v.y : v.z);
-}
+__device__ __forceinline__ float comp(const V& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
-__device__ __forceinline__ RayW make_rayw(V o, V d) {
+__device__ __forceinline__ RayW make_rayw(const V& o, const V& d) {
   RayW r;
-  r.ox = o.x; r.oy = o.y; r.oz = o.z;
   const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   int kz = 0;
   if (ay > ax) kz = 1;
   if (az > fmaxf(ax, ay)) kz = 2;
   int kx = kz + 1; if (kx == 3) kx = 0;
   int ky = kx + 1; if (ky == 3) ky = 0;
-  const float dz = kz == 0 ? d.x : (kz == 1 ? d.y : d.z);
+  const float dz = comp(d, kz);
   if (dz < 0.0f) { const int t = kx; kx = ky; ky = t; }
-  const float dx = kx == 0 ? d.x : (kx == 1 ? d.y : d.z);
-  const float dy = ky == 0 ? d.x : (ky == 1 ? d.y : d.z);
-  r.kx = kx; r.ky = ky; r.kz = kz;
-  r.Sx = __fdiv_rn(dx, dz);
-  r.Sy = __fdiv_rn(dy, dz);
+  r.ox = comp(o, kx); r.oy = comp(o, ky); r.oz = comp(o, kz);
+  r.bx = 4u * (uint32_t)kx; r.by = 4u * (uint32_t)ky; r.bz = 4u * (uint32_t)kz;
+  r.Sx = __fdiv_rn(comp(d, kx), dz);
+  r.Sy = __fdiv_rn(comp(d, ky), dz);
   r.Sz = __fdiv_rn(1.0f, dz);
   return r;
 }
 
 // Returns true and sets t when the ray hits the triangle with 0 < t <= tfar.
-__device__ __forceinline__ bool tri_hit(const RayW& r, const float4& p0, const float4& p1,
-                                        const float4& p2, float tfar, float& t_out) {
-  const float3 A = make_float3(sub(p0.x, r.ox), sub(p0.y, r.oy), sub(p0.z, r.oz));
-  const float3 B = make_float3(sub(p1.x, r.ox), sub(p1.y, r.oy), sub(p1.z, r.oz));
-  const float3 C = make_float3(sub(p2.x, r.ox), sub(p2.y, r.oy), sub(p2.z, r.oz));
-  const float Akz = comp(A, r.kz), Bkz = comp(B, r.kz), Ckz = comp(C, r.kz);
-  const float Ax = __fmaf_rn(-r.Sx, Akz, comp(A, r.kx));
-  const float Ay = __fmaf_rn(-r.Sy, Akz, comp(A, r.ky));
-  const float Bx = __fmaf_rn(-r.Sx, Bkz, comp(B, r.kx));
-  const float By = __fmaf_rn(-r.Sy, Bkz, comp(B, r.ky));
-  const float Cx = __fmaf_rn(-r.Sx, Ckz, comp(C, r.kx));
-  const float Cy = __fmaf_rn(-r.Sy, Ckz, comp(C, r.ky));
+__device__ __forceinline__ bool tri_hit(const RayW& r, const Tri* tri, float tfar, float& t_out) {
+  const char* tp = reinterpret_cast<const char*>(tri);
+  const float* px = reinterpret_cast<const float*>(tp + r.bx);
+  const float* py = reinterpret_cast<const float*>(tp + r.by);
+  const float* pz = reinterpret_cast<const float*>(tp + r.bz);
+  const float Akz = sub(__ldg(pz), r.oz), Bkz = sub(__ldg(pz + 4), r.oz), Ckz = sub(__ldg(pz + 8), r.oz);
+  const float Ax = __fmaf_rn(-r.Sx, Akz, sub(__ldg(px), r.ox));
+  const float Ay = __fmaf_rn(-r.Sy, Akz, sub(__ldg(py), r.oy));
+  const float Bx = __fmaf_rn(-r.Sx, Bkz, sub(__ldg(px + 4), r.ox));
+  const float By = __fmaf_rn(-r.Sy, Bkz, sub(__ldg(py + 4), r.oy));
+  const float Cx = __fmaf_rn(-r.Sx, Ckz, sub(__ldg(px + 8), r.ox));
+  const float Cy = __fmaf_rn(-r.Sy, Ckz, sub(__ldg(py + 8), r.oy));
   float U = sub(mul(Cx, By), mul(Cy, Bx));
   float Vv = sub(mul(Ax, Cy), mul(Ay, Cx));
   float W = sub(mul(Bx, Ay), mul(By, Ax));
-  if (U == 0.0f || Vv == 0.0f || W == 0.0f) {
+  if (fmin3f(fabsf(U), fabsf(Vv), fabsf(W)) == 0.0f) {
     const double CxBy = (double)Cx * (double)By, CyBx = (double)Cy * (double)Bx;
     U = (float)(CxBy - CyBx);
     const double AxCy = (double)Ax * (double)Cy, AyCx = (double)Ay * (double)Cx;
@@ -215,7 +233,8 @@ __device__ __forceinline__ bool tri_hit(const RayW& r, const float4& p0, const f
     const double BxAy = (double)Bx * (double)Ay, ByAx = (double)By * (double)Ax;
     W = (float)(BxAy - ByAx);
   }
-  if ((U < 0.0f || Vv < 0.0f || W < 0.0f) && (U > 0.0f || Vv > 0.0f || W > 0.0f)) return false;
+  // (min and max pass over a NaN as the six comparisons they stand for do)
+  if (fmin3f(U, Vv, W) < 0.0f && fmax3f(U, Vv, W) > 0.0f) return false;
   const float det = add(add(U, Vv), W);
   if (det == 0.0f) return false;
   const float Az = mul(r.Sz, Akz), Bz = mul(r.Sz, Bkz), Cz = mul(r.Sz, Ckz);

@@ -99,19 +99,6 @@ __device__ __forceinline__ RayBox make_raybox(const V& o, const V& d) {
   return r;
 }
 
-// Three-input float min/max (PTX ISA 8.8, sm_100 and later); same NaN rules as
-// the two-input forms.
-__device__ __forceinline__ float fmin3f(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ float fmax3f(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-
 #if RMG_SLAB_F32X2
 // (lo, hi) * (1/d, 1/d) + (lo addend, hi addend) for one axis in one packed
 // FMA (fma.rn.f32x2, sm_100 and later: two IEEE single-precision FMAs).
@@ -146,10 +133,9 @@ __device__ __forceinline__ bool visit(float tmin, float tmax, float best) {
 
 __device__ __forceinline__ void test_tri(const DeviceMap& map, const RayW& rw, int k, Hit& h) {
   const Tri* tp = map.tris + k;
-  const float4 p0 = __ldg(&tp->v0), p1 = __ldg(&tp->v1), p2 = __ldg(&tp->v2);
   float t;
-  if (tri_hit(rw, p0, p1, p2, h.t, t)) {
-    const uint32_t f = __float_as_uint(p0.w);
+  if (tri_hit(rw, tp, h.t, t)) {
+    const uint32_t f = __float_as_uint(__ldg(&tp->v0.w));
     if (t < h.t || f < h.face) { h.t = t; h.tri = k; h.face = f; }
   }
 }
@@ -500,12 +486,7 @@ __device__ __forceinline__ void leaf_exact(const DeviceMap& map, const RayW& rw,
   const float z1 = __fmaf_rn(fmaxf(fmaxf(p0.z, p1.z), p2.z), iz, __fadd_rn(nz, sz));
   const float tmin = fmax3f(fminf(x0, x1), fminf(y0, y1), fmaxf(fminf(z0, z1), 0.0f));
   const float tmax = fmin3f(fmaxf(x0, x1), fmaxf(y0, y1), fmaxf(z0, z1));
-  if (!visit(tmin, tmax, h.t)) return;
-  float t;
-  if (tri_hit(rw, p0, p1, p2, h.t, t)) {
-    const uint32_t f = __float_as_uint(p0.w);
-    if (t < h.t || f < h.face) { h.t = t; h.tri = k; h.face = f; }
-  }
+  if (visit(tmin, tmax, h.t)) test_tri(map, rw, k, h);
 }
 
 // Closest hit through the 8-wide quantized tree (wide8.cu).  Every child box
