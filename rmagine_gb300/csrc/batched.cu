@@ -47,6 +47,7 @@ struct BatchParams {
   unsigned budget;
   int trail_bits;
   int full_stack;
+  int wide;  // walk the 4-wide tree
 };
 
 template <int OK, int SS, int TB>
@@ -76,12 +77,8 @@ __device__ __forceinline__ void batched_ray(const BatchParams& B, const JobDev& 
   write_attributes<OK>(P, gid, h, dir_s, orig_s, Tsm);
 }
 
-#ifndef RMG_BATCHED_MIN_BLOCKS
-#define RMG_BATCHED_MIN_BLOCKS 5
-#endif
-
 template <int SS, int TB>
-__global__ void __launch_bounds__(256, RMG_BATCHED_MIN_BLOCKS) k_trace_batched(const BatchParams B) {
+__global__ void __maxnreg__((trace_regs<TB>())) k_trace_batched(const BatchParams B) {
   __shared__ unsigned long long s_begin[kMaxJobsShared + 1];
   const bool in_smem = B.n_jobs <= kMaxJobsShared;
   if (in_smem) {
@@ -119,6 +116,10 @@ __global__ void __launch_bounds__(256, RMG_BATCHED_MIN_BLOCKS) k_trace_batched(c
 
 template <int SS>
 cudaError_t launch_batched_tb(const BatchParams& B, unsigned grid, unsigned block, cudaStream_t st) {
+  if (SS > 0 && B.wide) {
+    k_trace_batched<0, kWideTB><<<grid, block, 0, st>>>(B);
+    return cudaGetLastError();
+  }
   if (SS > 0 && B.full_stack) {
     k_trace_batched<kFullStack, 0><<<grid, block, 0, st>>>(B);
     return cudaGetLastError();
@@ -142,6 +143,7 @@ cudaError_t launch_batched(const BatchParams& B, int ss, unsigned grid, unsigned
 
 template <int SS>
 const void* batched_fn(int tb) {
+  if (tb == kWideTB) return reinterpret_cast<const void*>(k_trace_batched<0, kWideTB>);
   if (tb == 0) return reinterpret_cast<const void*>(k_trace_batched<kFullStack, 0>);
   return tb == 32 ? reinterpret_cast<const void*>(k_trace_batched<SS, 32>)
                   : tb == 64 ? reinterpret_cast<const void*>(k_trace_batched<SS, 64>)
@@ -254,6 +256,7 @@ BatchParams params(const rmg_batch* b) {
   B.budget = 2u * b->map->n_nodes + 64u;
   B.trail_bits = trail_bits_for_depth(b->map->depth);
   B.full_stack = b->map->depth <= (unsigned)kFullStack ? 1 : 0;
+  B.wide = have_wide4(b->map) ? 1 : 0;
   return B;
 }
 
@@ -261,8 +264,10 @@ BatchParams params(const rmg_batch* b) {
 int launch_direct(rmg_batch* b, cudaStream_t st) {
   if (b->total_tiles == 0) return RMG_OK;
   unsigned grid = 0;
-  const bool full = b->cfg.stack_depth > 0 && b->map->depth <= (unsigned)kFullStack;
-  int s = persistent_grid(b->cfg, full ? 0 : trail_bits_for_depth(b->map->depth), grid);
+  const bool stack = b->cfg.stack_depth > 0;
+  const bool full = stack && b->map->depth <= (unsigned)kFullStack;
+  int s = persistent_grid(b->cfg, stack && have_wide4(b->map) ? kWideTB
+                                  : full ? 0 : trail_bits_for_depth(b->map->depth), grid);
   if (s != RMG_OK) return s;
   RMG_CUDA_TRY(cudaMemsetAsync(b->counter, 0, sizeof(unsigned long long), st));
   return cuda_status(launch_batched(params(b), (int)b->cfg.stack_depth, grid, 32u * b->cfg.block_warps, st),

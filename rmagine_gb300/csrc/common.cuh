@@ -41,10 +41,11 @@ struct __align__(16) Tri {
 };
 
 // 4-wide node, 128 B (one cache line), collapsed from the binary tree:
-// the four child boxes as structure of arrays (component k = child k), the
+// the four child boxes as structure of arrays (component k = slot k), the
 // child links (>= 0 wide node, < 0 leaf ~packed triangle, kEmpty4 = no child,
-// whose box is a point at 1e30 that no ray reaches), and meta = (children,
-// parent wide node or -1, 0, 0).
+// whose box is a point at 1e30), and meta = (base, leaf slots as bits 0-3 |
+// internal slots as bits 4-7, 0, 0).  Internal children take the first slots
+// and are consecutive nodes: slot k's is node base + k.
 constexpr int kEmpty4 = (int)0x80000000;
 
 struct __align__(16) Node4 {

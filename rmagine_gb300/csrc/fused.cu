@@ -33,9 +33,6 @@
 namespace rmg {
 namespace {
 
-#ifndef RMG_FUSED_MIN_BLOCKS
-#define RMG_FUSED_MIN_BLOCKS 5
-#endif
 // tiles (32 rays) each warp reduces before its CTA writes one partial record
 #ifndef RMG_FUSED_TILES_PER_WARP
 #define RMG_FUSED_TILES_PER_WARP 8
@@ -83,7 +80,7 @@ __device__ __forceinline__ double raw_moment(const float v[16], uint32_t k, cons
 }
 
 template <bool P2L, int OK, int SS, int TB>
-__global__ void __launch_bounds__(256, RMG_FUSED_MIN_BLOCKS) k_trace_stats(const FusedParams F) {
+__global__ void __maxnreg__((trace_regs<TB>())) k_trace_stats(const FusedParams F) {
   const TraceParams& P = F.T;
   const uint32_t pose = blockIdx.x / F.ctas_per_pose;
   const uint32_t cta = blockIdx.x - pose * F.ctas_per_pose;
@@ -201,6 +198,10 @@ __global__ void k_compose(const rmg_transform* a, uint32_t a_stride, const rmg_t
 
 template <bool P2L, int OK>
 cudaError_t launch_fused_ok(const FusedParams& F, unsigned grid, unsigned block, cudaStream_t st) {
+  if (F.T.wide) {
+    k_trace_stats<P2L, OK, 0, kWideTB><<<grid, block, 0, st>>>(F);
+    return cudaGetLastError();
+  }
   if (F.T.full_stack) {
     k_trace_stats<P2L, OK, kFullStack, 0><<<grid, block, 0, st>>>(F);
     return cudaGetLastError();

@@ -33,12 +33,8 @@ struct GradParams {
   uint32_t warps_per_pose;
 };
 
-#ifndef RMG_GRAD_MIN_BLOCKS
-#define RMG_GRAD_MIN_BLOCKS 5
-#endif
-
 template <int OK, int SS, int TB>
-__global__ void __launch_bounds__(256, RMG_GRAD_MIN_BLOCKS) k_range_grad(const GradParams G) {
+__global__ void __maxnreg__((trace_regs<TB>())) k_range_grad(const GradParams G) {
   const TraceParams& P = G.T;
   const uint32_t pose = blockIdx.y;
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -127,6 +123,10 @@ __global__ void k_grad_final(const float* partial, uint32_t n_poses, uint32_t wa
 
 template <int OK, int SS>
 cudaError_t launch_grad_tb(const GradParams& G, dim3 grid, unsigned block, cudaStream_t st) {
+  if (G.T.wide) {
+    k_range_grad<OK, 0, kWideTB><<<grid, block, 0, st>>>(G);
+    return cudaGetLastError();
+  }
   if (G.T.full_stack) {
     k_range_grad<OK, kFullStack, 0><<<grid, block, 0, st>>>(G);
     return cudaGetLastError();

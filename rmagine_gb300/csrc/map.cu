@@ -823,10 +823,7 @@ extern "C" int rmg_map_debug_set_child(rmg_map* m, uint32_t node, uint32_t which
         return fail(RMG_ERR_INVALID_ARG, "rmg_map_debug_set_child: wide node/slot out of range");
       if (child >= 0 ? (uint32_t)child >= m->n_nodes4 : (uint32_t)(~child) >= m->n_faces)
         return fail(RMG_ERR_INVALID_ARG, "rmg_map_debug_set_child: child out of range");
-      const size_t off = offsetof(Node4, child) + sizeof(int) * (which - 2);
-      RMG_CUDA_TRY(cudaMemcpy(reinterpret_cast<char*>(m->d_nodes4 + node) + off, &child, sizeof(int),
-                              cudaMemcpyHostToDevice));
-      return RMG_OK;
+      return wide_set_child(m, node, which - 2, child);
     }
     if (node >= m->n_nodes)
       return fail(RMG_ERR_INVALID_ARG, "rmg_map_debug_set_child: node/which out of range");
@@ -835,7 +832,7 @@ extern "C" int rmg_map_debug_set_child(rmg_map* m, uint32_t node, uint32_t which
     const size_t off = offsetof(Node, d) + (which ? sizeof(int) : 0);
     RMG_CUDA_TRY(cudaMemcpy(reinterpret_cast<char*>(m->d_nodes + node) + off, &child, sizeof(int),
                             cudaMemcpyHostToDevice));
-    wide_free(m);  // the binary tree is the one damaged: walk it from now on
+    m->depth4 = 0xffffffffu;  // the binary tree is the one damaged: walk it from now on (see have_wide4)
     return RMG_OK;
   });
 }

@@ -7,22 +7,9 @@
 #include "launch.h"
 #include "trace.cuh"
 
-// Walk the 4-wide tree when the launch config leaves the choice open.  Off:
-// on the 1M-triangle terrain the binary walk is faster (spherical 6,296 vs
-// 5,736 Mrays/s, pinhole 9,200 vs 8,035); the 4-wide walk wins on small maps
-// (2,412-triangle room: 3,563 vs 3,281) and is chosen there with bvh_width = 4.
-#ifndef RMG_DEFAULT_WIDE
-#define RMG_DEFAULT_WIDE 0
-#endif
-
 // 8-wide quantized walk when the launch config leaves the width open.
 #ifndef RMG_DEFAULT_WIDE8
 #define RMG_DEFAULT_WIDE8 0
-#endif
-
-// Warp-synchronous packet walk when the launch config leaves the choice open.
-#ifndef RMG_DEFAULT_PACKET
-#define RMG_DEFAULT_PACKET 0
 #endif
 
 namespace rmg {
@@ -97,10 +84,10 @@ int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_tr
   P.budget = 2u * map->n_nodes + 64u;
   P.trail_bits = trail_bits_for_depth(map->depth);
   P.full_stack = map->depth <= (unsigned)kFullStack ? 1 : 0;
-  // 4-wide walk: 3 pushes per level at most, so 21 levels fit its 64-entry stack
-  P.wide = (cfg.bvh_width != 2 && cfg.refill == 0 && map->d_nodes4 && 3 * map->depth4 <= (unsigned)kStack4 &&
-            RMG_DEFAULT_WIDE) ? 1 : 0;
-  if (cfg.bvh_width == 4 && cfg.refill == 0 && map->d_nodes4 && 3 * map->depth4 <= (unsigned)kStack4) P.wide = 1;
+  // 4-wide walk unless another walk is asked for (a width, the packet walk, or a
+  // short stack other than the default's)
+  P.wide = (have_wide4(map) && cfg.refill == 0 &&
+            (cfg.bvh_width == 4 || (cfg.bvh_width == 0 && cfg.packet != 1 && cfg.stack_depth == 16))) ? 1 : 0;
   // 8-wide quantized walk: a pending-children stack of kStack8 entries holds trees of kStack8 + 1 levels
   const bool have8 = map->d_nodes8 && map->depth8 <= (unsigned)kStack8 + 1u;
   P.wide8 = (have8 && cfg.refill == 0 && (cfg.bvh_width == 8 || (cfg.bvh_width == 0 && RMG_DEFAULT_WIDE8))) ? 1 : 0;
@@ -109,8 +96,7 @@ int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_tr
     P.map.tris = map->d_tris8;  // h.tri of this walk indexes the 8-wide triangle copy
   }
   // warp-synchronous packet walk: binary tree, full stack
-  const bool want_packet = cfg.packet == 1 || (cfg.packet == 2 && RMG_DEFAULT_PACKET);
-  P.packet = (want_packet && !P.wide && !P.wide8 && cfg.refill == 0 && P.full_stack) ? 1 : 0;
+  P.packet = (cfg.packet == 1 && !P.wide && !P.wide8 && cfg.refill == 0 && P.full_stack) ? 1 : 0;
   return RMG_OK;
 }
 

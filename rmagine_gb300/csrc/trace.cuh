@@ -27,6 +27,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "internal.h"
 
 namespace rmg {
 
@@ -348,73 +349,136 @@ constexpr int kWideTB = 4;
 // the budget error.
 constexpr int kStack4 = 64;
 
-__device__ __forceinline__ void cswap(float& ta, int& ca, float& tb, int& cb) {
-  const bool s = tb < ta;
-  const float t = s ? tb : ta;
-  const int c = s ? cb : ca;
-  tb = s ? ta : tb;
-  cb = s ? ca : cb;
-  ta = t;
-  ca = c;
+// Whether a map's 4-wide tree can be walked.
+inline bool have_wide4(const rmg_map* m) { return m->d_nodes4 && m->depth4 <= (unsigned)kStack4 / 3u; }
+
+// One axis of two children at once: (near0, near1) planes times (1/d, 1/d)
+// plus the plane's addend, each an IEEE single FMA.
+__device__ __forceinline__ void plane2(unsigned long long p, unsigned long long inv, unsigned long long add,
+                                       float& t0, float& t1) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(p), "l"(inv), "l"(add));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(r));
 }
 
-// Closest hit through the 4-wide tree.  Same boxes, same culling rule
-// (tmin <= min(tmax, best) * (1 + 2^-22)) and the same triangle test and tie
-// rule as the binary walk, so the hit (t, face) is identical; only the order
-// of visits differs.  Leaf children are tested as soon as their box is hit;
-// internal children are visited nearest first (a 4-element sorting network on
-// the entry distances), the others pushed far to near.
+// Closest hit through the 4-wide tree, the default walk.  Same boxes, same slab
+// arithmetic and culling rule (tmin <= min(tmax, best) * (1 + 2^-22)) and the
+// same triangle test and tie rule as the binary walk, so the hit (t, face) is
+// identical; only the order of visits differs.
+//
+// What bounds it is instruction issue and the half-rate min/max/compare pipe
+// (65% and 54% busy on the 1M-triangle terrain; L1 68%), so a visit is built to
+// spend little there: the near and far planes are picked by address from the
+// ray's signs (no min/max of a plane pair), two children share an FMA
+// (fma.rn.f32x2), the hits are a 4-bit mask, and entry distances are ordered
+// only where two or more internal children are hit (23% of the visits), the
+// nearest first and the others as they come (a third hit is rare).  Internal
+// children are consecutive nodes, so no link is read for them.  12.7 visits per
+// ray against 24.9 binary ones there.  Both walks, us a pass: that terrain with
+// a 128 x 1024 lidar 3,221 (binary) / 3,126, a 2.1M-triangle terrain with a
+// 640 x 480 camera 1,558 / 1,466, the box room with a 16 x 360 lidar 318 / 299,
+// one 16 x 900 scan there 32.5 / 29.3, scattered directions 204 / 184.  Sorting
+// all four distances, postponing the leaf tests until every lane has one,
+// 32-bit node offsets and a pointer per plane all measured slower.
 __device__ __forceinline__ void trace_ray4(const DeviceMap& map, const V& o, const V& d, float tfar,
                                            unsigned budget, Hit& h, bool& over_budget) {
   h.t = tfar;
   h.tri = -1;
   h.face = 0xffffffffu;
   if (map.root < 0) return;
+  // A ray with a NaN or infinite component hits no triangle (its edge functions
+  // or its quotient are NaN), but a box test with NaN planes admits everything.
+  float z = o.x * 0.0f;
+  z = fmaf(o.y, 0.0f, z); z = fmaf(o.z, 0.0f, z);
+  z = fmaf(d.x, 0.0f, z); z = fmaf(d.y, 0.0f, z); z = fmaf(d.z, 0.0f, z);
+  if (z != 0.0f) return;
   const RayW rw = make_rayw(o, d);
   const RayBox rb = make_raybox(o, d);
-  int stk_node[kStack4];
-  float stk_t[kStack4];
+  const bool bx = rb.ix < 0.f, by = rb.iy < 0.f, bz = rb.iz < 0.f;
+  const unsigned long long pix = pack2(rb.ix, rb.ix), piy = pack2(rb.iy, rb.iy), piz = pack2(rb.iz, rb.iz);
+  const float nxa = bx ? rb.chx : rb.clx, fxa = bx ? rb.clx : rb.chx;
+  const float nya = by ? rb.chy : rb.cly, fya = by ? rb.cly : rb.chy;
+  const float nza = bz ? rb.chz : rb.clz, fza = bz ? rb.clz : rb.chz;
+  const unsigned long long cnx = pack2(nxa, nxa), cfx = pack2(fxa, fxa), cny = pack2(nya, nya),
+                           cfy = pack2(fya, fya), cnz = pack2(nza, nza), cfz = pack2(fza, fza);
+  // byte offsets of the near planes in a node; the far planes are at ^ 16
+  const uint32_t ox = bx ? 16u : 0u, oy = by ? 48u : 32u, oz = bz ? 80u : 64u;
+  uint2 stack[kStack4];
   int sp = 0;
   int node = 0;
   unsigned steps = 0;
   while (true) {
     if (++steps > budget) { over_budget = true; break; }
-    const Node4* np = map.nodes4 + node;
-    const float4 lox = __ldg(&np->lox), hix = __ldg(&np->hix), loy = __ldg(&np->loy), hiy = __ldg(&np->hiy);
-    const float4 loz = __ldg(&np->loz), hiz = __ldg(&np->hiz);
-    const int4 ch = __ldg(&np->child);
-    float t0, t1, t2, t3, m0, m1, m2, m3;
-    slab(rb, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x, t0, m0);
-    slab(rb, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y, t1, m1);
-    slab(rb, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z, t2, m2);
-    slab(rb, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w, t3, m3);
-    bool v0 = visit(t0, m0, h.t), v1 = visit(t1, m1, h.t), v2 = visit(t2, m2, h.t), v3 = visit(t3, m3, h.t);
-    if (v0 && ch.x < 0) { if (ch.x != kEmpty4) test_tri(map, rw, ~ch.x, h); v0 = false; }
-    if (v1 && ch.y < 0) { if (ch.y != kEmpty4) test_tri(map, rw, ~ch.y, h); v1 = false; }
-    if (v2 && ch.z < 0) { if (ch.z != kEmpty4) test_tri(map, rw, ~ch.z, h); v2 = false; }
-    if (v3 && ch.w < 0) { if (ch.w != kEmpty4) test_tri(map, rw, ~ch.w, h); v3 = false; }
-    const float cull = h.t * kWiden;
-    const float inf = __int_as_float(0x7f800000);
-    float k0 = v0 && t0 <= cull ? t0 : inf, k1 = v1 && t1 <= cull ? t1 : inf;
-    float k2 = v2 && t2 <= cull ? t2 : inf, k3 = v3 && t3 <= cull ? t3 : inf;
-    int c0 = ch.x, c1 = ch.y, c2 = ch.z, c3 = ch.w;
-    cswap(k0, c0, k1, c1);
-    cswap(k2, c2, k3, c3);
-    cswap(k0, c0, k2, c2);
-    cswap(k1, c1, k3, c3);
-    cswap(k1, c1, k2, c2);
-    if (k0 < inf) {
-      if (sp + 3 > kStack4) { over_budget = true; break; }  // only a corrupt tree gets this deep
-      if (k3 < inf) { stk_node[sp] = c3; stk_t[sp] = k3; ++sp; }
-      if (k2 < inf) { stk_node[sp] = c2; stk_t[sp] = k2; ++sp; }
-      if (k1 < inf) { stk_node[sp] = c1; stk_t[sp] = k1; ++sp; }
-      node = c0;
+    const char* np = reinterpret_cast<const char*>(map.nodes4 + node);
+    const ulonglong2 qnx = __ldg(reinterpret_cast<const ulonglong2*>(np + ox));
+    const ulonglong2 qfx = __ldg(reinterpret_cast<const ulonglong2*>(np + (ox ^ 16u)));
+    const ulonglong2 qny = __ldg(reinterpret_cast<const ulonglong2*>(np + oy));
+    const ulonglong2 qfy = __ldg(reinterpret_cast<const ulonglong2*>(np + (oy ^ 16u)));
+    const ulonglong2 qnz = __ldg(reinterpret_cast<const ulonglong2*>(np + oz));
+    const ulonglong2 qfz = __ldg(reinterpret_cast<const ulonglong2*>(np + (oz ^ 16u)));
+    const int2 meta = __ldg(reinterpret_cast<const int2*>(np + 112));
+    float t[4], m[4];
+    {
+      float x0, x1, y0, y1, z0, z1;
+      plane2(qnx.x, pix, cnx, x0, x1); plane2(qny.x, piy, cny, y0, y1); plane2(qnz.x, piz, cnz, z0, z1);
+      t[0] = fmax3f(x0, y0, fmaxf(z0, 0.0f));
+      t[1] = fmax3f(x1, y1, fmaxf(z1, 0.0f));
+      plane2(qnx.y, pix, cnx, x0, x1); plane2(qny.y, piy, cny, y0, y1); plane2(qnz.y, piz, cnz, z0, z1);
+      t[2] = fmax3f(x0, y0, fmaxf(z0, 0.0f));
+      t[3] = fmax3f(x1, y1, fmaxf(z1, 0.0f));
+      plane2(qfx.x, pix, cfx, x0, x1); plane2(qfy.x, piy, cfy, y0, y1); plane2(qfz.x, piz, cfz, z0, z1);
+      m[0] = fmin3f(x0, y0, fminf(z0, h.t));
+      m[1] = fmin3f(x1, y1, fminf(z1, h.t));
+      plane2(qfx.y, pix, cfx, x0, x1); plane2(qfy.y, piy, cfy, y0, y1); plane2(qfz.y, piz, cfz, z0, z1);
+      m[2] = fmin3f(x0, y0, fminf(z0, h.t));
+      m[3] = fmin3f(x1, y1, fminf(z1, h.t));
+    }
+    uint32_t hit = 0;
+    if (t[0] <= m[0] * kWiden) hit |= 0x11u;
+    if (t[1] <= m[1] * kWiden) hit |= 0x22u;
+    if (t[2] <= m[2] * kWiden) hit |= 0x44u;
+    if (t[3] <= m[3] * kWiden) hit |= 0x88u;
+    hit &= (uint32_t)meta.y;
+    uint32_t lm = hit & 15u, im = hit >> 4;
+    if (lm) {
+      const int* cp = reinterpret_cast<const int*>(np + 96);
+      do {
+        const int s = __ffs((int)lm) - 1;
+        lm &= lm - 1u;
+        test_tri(map, rw, ~__ldg(cp + s), h);
+      } while (lm);
+      const float cull = h.t * kWiden;
+      if (!(t[0] <= cull)) im &= ~1u;
+      if (!(t[1] <= cull)) im &= ~2u;
+      if (!(t[2] <= cull)) im &= ~4u;
+      if (!(t[3] <= cull)) im &= ~8u;
+    }
+    if (im) {
+      uint32_t s = (im >> 1) - (im >> 3);  // the slot of a single bit
+      if (im & (im - 1u)) {
+        // entry distance and slot in one word: ordered as the distances (>= 0)
+        // are, rounded down to 4 ulp, which keeps the later culls conservative
+        const uint32_t k0 = im & 1u ? (__float_as_uint(t[0]) & ~3u) : 0xffffffffu;
+        const uint32_t k1 = im & 2u ? (__float_as_uint(t[1]) & ~3u) | 1u : 0xffffffffu;
+        const uint32_t k2 = im & 4u ? (__float_as_uint(t[2]) & ~3u) | 2u : 0xffffffffu;
+        const uint32_t k3 = im & 8u ? (__float_as_uint(t[3]) & ~3u) | 3u : 0xffffffffu;
+        const uint32_t kn = min(min(k0, k1), min(k2, k3));
+        s = kn & 3u;
+        if (sp + 3 > kStack4) { over_budget = true; break; }  // only a corrupt tree gets this deep
+        im &= ~(1u << s);
+        if (im & 8u) stack[sp++] = make_uint2(k3, (uint32_t)meta.x + 3u);
+        if (im & 4u) stack[sp++] = make_uint2(k2, (uint32_t)meta.x + 2u);
+        if (im & 2u) stack[sp++] = make_uint2(k1, (uint32_t)meta.x + 1u);
+        if (im & 1u) stack[sp++] = make_uint2(k0, (uint32_t)meta.x);
+      }
+      node = meta.x + (int)s;
       continue;
     }
     bool found = false;
+    const float cull = h.t * kWiden;
     while (sp > 0) {
-      --sp;
-      if (stk_t[sp] <= h.t * kWiden) { node = stk_node[sp]; found = true; break; }
+      const uint2 e = stack[--sp];
+      if (__uint_as_float(e.x & ~3u) <= cull) { node = (int)e.y; found = true; break; }
     }
     if (!found) break;
   }
@@ -816,28 +880,20 @@ __device__ __forceinline__ void setup_ray(const SensorDev& sen, const Tf& Tsm, u
   }
 }
 
-// One warp = one tile of tile_h x tile_w rays of one pose.
-// Minimum resident CTAs per SM requested from the compiler for k_trace: 5
-// CTAs of 256 threads cap the kernel at 48 registers (a few bytes of spills
-// to L1-cached local memory) and lift occupancy from 50% to 62.5%; measured
-// 9% faster than the unconstrained 62-register build on the 1M-triangle
-// terrain (6,179 vs 5,661 Mrays/s), while 6 CTAs (40 registers) spill more
-// and lose again.
-#ifndef RMG_TRACE_MIN_BLOCKS
-#define RMG_TRACE_MIN_BLOCKS 5
-#endif
-
-// The 8-wide walk holds a node's twenty words and three axes of plane
-// addends at once: it gets 64 registers (4 CTAs of 256 threads per SM).
-#ifndef RMG_TRACE8_MIN_BLOCKS
-#define RMG_TRACE8_MIN_BLOCKS 4
-#endif
-
+// Registers of the traversal kernels, by walk.  The binary walk at 48 (40 warps
+// per SM, a few bytes of spills to L1-cached local memory) is 9% faster than
+// unconstrained at 62 (1M-triangle terrain, 5,661 -> 6,179 Mrays/s then), 40
+// registers lose again.  The 4-wide walk holds twice the planes per visit; on
+// the same terrain 48 / 56 / 64 / 72 registers take 3,778 / 3,297 / 3,351 /
+// 3,589 us, in the box room 362 / 322 / 324 / 338.  The 8-wide walk holds a
+// node's twenty words and three axes of plane addends at once.
 template <int TB>
-constexpr int trace_min_blocks() { return TB == kWide8TB ? RMG_TRACE8_MIN_BLOCKS : RMG_TRACE_MIN_BLOCKS; }
+constexpr int trace_regs() { return TB == kWide8TB ? 64 : (TB == kWideTB ? 56 : 48); }
 
+// One warp = one tile of tile_h x tile_w rays of one pose.
 template <int OK, int SS, int TB>
-__global__ void __launch_bounds__(256, trace_min_blocks<TB>()) k_trace(const TraceParams P) {
+__global__ void __maxnreg__((trace_regs<TB>()))
+k_trace(const TraceParams P) {
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp >= P.n_tiles) return;
   const uint32_t lane = threadIdx.x & 31;

@@ -8,8 +8,9 @@
 // packets", RT 2008, and of most wide-BVH builders since).  Every slot keeps
 // the binary record its box came from (parent node and side), so after a
 // binary refit the wide boxes are refreshed by one copy kernel.  Node indices
-// are allocated level by level with an atomic counter; their order does not
-// affect any result (the traversal's closest hit is order-independent).
+// are allocated level by level with an atomic counter, a node's internal
+// children as one block; their order does not affect any result (the traversal's closest hit is order-independent).
+#include <algorithm>
 #include <vector>
 
 #include "internal.h"
@@ -44,7 +45,7 @@ __device__ __forceinline__ float half_area(const Cand& c) {
   return ex * ey + ey * ez + ez * ex;
 }
 
-__device__ __forceinline__ void set_slot(Node4& w, int k, const float lo[3], const float hi[3]) {
+__host__ __device__ __forceinline__ void set_slot(Node4& w, int k, const float lo[3], const float hi[3]) {
   float* lox = &w.lox.x; float* hix = &w.hix.x; float* loy = &w.loy.x;
   float* hiy = &w.hiy.x; float* loz = &w.loz.x; float* hiz = &w.hiz.x;
   lox[k] = lo[0]; hix[k] = hi[0]; loy[k] = lo[1]; hiy[k] = hi[1]; loz[k] = lo[2]; hiz[k] = hi[2];
@@ -52,8 +53,8 @@ __device__ __forceinline__ void set_slot(Node4& w, int k, const float lo[3], con
 
 // One level of the collapse: wide nodes [lo4, hi4), whose binary roots are
 // bin_of[j], get their children; internal children receive new wide indices.
-__global__ void k_collapse(const Node* __restrict__ bn, int* bin_of, int* parent4, uint32_t lo4, uint32_t hi4,
-                           Node4* w4, int* src4, unsigned int* count4) {
+__global__ void k_collapse(const Node* __restrict__ bn, int* bin_of, uint32_t lo4, uint32_t hi4, Node4* w4,
+                           int* src4, unsigned int* count4) {
   const uint32_t j = lo4 + blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= hi4) return;
   const int b = bin_of[j];
@@ -78,6 +79,18 @@ __global__ void k_collapse(const Node* __restrict__ bn, int* bin_of, int* parent
     c[best] = cand_of(nb, id, 0);
     c[n++] = cand_of(nb, id, 1);
   }
+  // internal children take the first slots and get consecutive wide indices, so
+  // a walk finds child `slot` at base + slot without reading the links
+  int ni = 0;
+  for (int k = 0; k < n; ++k) {
+    if (c[k].id >= 0) {
+      const Cand t = c[ni];
+      c[ni] = c[k];
+      c[k] = t;
+      ++ni;
+    }
+  }
+  const int base = ni > 0 ? (int)atomicAdd(count4, (unsigned int)ni) : 0;
   Node4 w;
   const float far[3] = {1e30f, 1e30f, 1e30f};
   int child[4];
@@ -87,10 +100,8 @@ __global__ void k_collapse(const Node* __restrict__ bn, int* bin_of, int* parent
       if (c[k].id < 0) {
         child[k] = c[k].id;
       } else {
-        const unsigned int k4 = atomicAdd(count4, 1u);
-        bin_of[k4] = c[k].id;
-        parent4[k4] = (int)j;
-        child[k] = (int)k4;
+        bin_of[base + k] = c[k].id;
+        child[k] = base + k;
       }
       src4[4 * j + k] = c[k].src;
     } else {
@@ -100,7 +111,7 @@ __global__ void k_collapse(const Node* __restrict__ bn, int* bin_of, int* parent
     }
   }
   w.child = make_int4(child[0], child[1], child[2], child[3]);
-  w.meta = make_int4(n, parent4[j], 0, 0);
+  w.meta = make_int4(base, (((1 << n) - 1) ^ ((1 << ni) - 1)) | (((1 << ni) - 1) << 4), 0, 0);
   w4[j] = w;
 }
 
@@ -136,23 +147,20 @@ int wide_build(rmg_map* m, cudaStream_t st) {
   if (m->n_faces == 0) return RMG_OK;
   const uint32_t cap = std::max<uint32_t>(m->n_nodes, 1u);
   int* bin_of = nullptr;
-  int* parent4 = nullptr;
   unsigned int* count4 = nullptr;
   int s = dev_alloc(&m->d_nodes4, cap, "wide nodes");
   if (s == RMG_OK) s = dev_alloc(&m->d_src4, 4 * (size_t)cap, "wide sources");
   if (s == RMG_OK) s = dev_alloc(&bin_of, cap, "wide roots");
-  if (s == RMG_OK) s = dev_alloc(&parent4, cap, "wide parents");
   if (s == RMG_OK) s = dev_alloc(&count4, 1, "wide counter");
-  const int zero = 0, minus1 = -1;
+  const int zero = 0;
   const unsigned int one = 1;
   if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(bin_of, &zero, 4, cudaMemcpyHostToDevice, st), "wide init");
-  if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(parent4, &minus1, 4, cudaMemcpyHostToDevice, st), "wide init");
   if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(count4, &one, 4, cudaMemcpyHostToDevice, st), "wide init");
   uint32_t lo4 = 0, hi4 = 1, levels = 0;
   while (s == RMG_OK && lo4 < hi4) {
     const uint32_t n = hi4 - lo4;
-    k_collapse<<<(n + kBlock4 - 1) / kBlock4, kBlock4, 0, st>>>(m->d_nodes, bin_of, parent4, lo4, hi4, m->d_nodes4,
-                                                                m->d_src4, count4);
+    k_collapse<<<(n + kBlock4 - 1) / kBlock4, kBlock4, 0, st>>>(m->d_nodes, bin_of, lo4, hi4, m->d_nodes4, m->d_src4,
+                                                                count4);
     s = cuda_status(cudaGetLastError(), "k_collapse");
     unsigned int c = 0;
     if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&c, count4, 4, cudaMemcpyDeviceToHost, st), "wide count");
@@ -163,11 +171,57 @@ int wide_build(rmg_map* m, cudaStream_t st) {
     if (hi4 > cap) s = fail(RMG_ERR_CUDA, "wide build: node count exceeds the binary tree");
   }
   cudaFree(bin_of);
-  cudaFree(parent4);
   cudaFree(count4);
   if (s != RMG_OK) { wide_free(m); return s; }
   m->n_nodes4 = hi4;
   m->depth4 = levels;
+  return RMG_OK;
+}
+
+// Test hook: slot `slot` of wide node `node` gets the link `child` (range-checked
+// by the caller).  The walk takes internal children as consecutive nodes, so the
+// node's slots are put in order again (internal ones first) and its internal
+// children are copied to a new block behind the last node.  Synchronises.
+int wide_set_child(rmg_map* m, uint32_t node, uint32_t slot, int child) {
+  const uint32_t n4 = m->n_nodes4;
+  std::vector<Node4> w(n4);
+  std::vector<int> src(4 * (size_t)n4);
+  RMG_CUDA_TRY(cudaMemcpy(w.data(), m->d_nodes4, sizeof(Node4) * n4, cudaMemcpyDeviceToHost));
+  RMG_CUDA_TRY(cudaMemcpy(src.data(), m->d_src4, sizeof(int) * src.size(), cudaMemcpyDeviceToHost));
+  const Node4 old = w[node];
+  const int old_src[4] = {src[4 * node], src[4 * node + 1], src[4 * node + 2], src[4 * node + 3]};
+  int link[4] = {old.child.x, old.child.y, old.child.z, old.child.w};
+  link[slot] = child;
+  int order[4], n = 0, ni = 0;
+  for (int pass = 0; pass < 3; ++pass)  // internal, leaf, empty
+    for (int k = 0; k < 4; ++k)
+      if ((link[k] >= 0 ? 0 : (link[k] == kEmpty4 ? 2 : 1)) == pass) {
+        order[n++] = k;
+        if (pass == 0) ++ni;
+      }
+  if ((uint64_t)n4 + ni > std::max<uint32_t>(m->n_nodes, 1u))
+    return fail(RMG_ERR_INVALID_ARG, "rmg_map_debug_set_child: no room for the changed node's children");
+  Node4 nw = old;
+  uint32_t leaves = 0;
+  for (int j = 0; j < 4; ++j) {
+    const int k = order[j];
+    const float lo[3] = {(&old.lox.x)[k], (&old.loy.x)[k], (&old.loz.x)[k]};
+    const float hi[3] = {(&old.hix.x)[k], (&old.hiy.x)[k], (&old.hiz.x)[k]};
+    set_slot(nw, j, lo, hi);
+    (&nw.child.x)[j] = j < ni ? (int)n4 + j : link[k];
+    if (link[k] < 0 && link[k] != kEmpty4) leaves |= 1u << j;
+    src[4 * node + j] = old_src[k];
+  }
+  nw.meta = make_int4((int)n4, (int)leaves | (((1 << ni) - 1) << 4), 0, 0);
+  w[node] = nw;
+  for (int j = 0; j < ni; ++j) {
+    const int from = link[order[j]];
+    w.push_back(Node4(w[from]));
+    for (int k = 0; k < 4; ++k) src.push_back(int(src[4 * from + k]));
+  }
+  RMG_CUDA_TRY(cudaMemcpy(m->d_nodes4, w.data(), sizeof(Node4) * w.size(), cudaMemcpyHostToDevice));
+  RMG_CUDA_TRY(cudaMemcpy(m->d_src4, src.data(), sizeof(int) * src.size(), cudaMemcpyHostToDevice));
+  m->n_nodes4 = (uint32_t)w.size();
   return RMG_OK;
 }
 
