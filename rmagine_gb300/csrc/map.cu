@@ -436,21 +436,12 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
   
     const uint32_t n = n_faces;
     if (builder == RMG_BUILD_SAH) {
-      s = sah_build_topology(m, st, m->d_leaf_order);
-      if (s == RMG_OK) s = repack_and_refit(m, st, m->d_leaf_order);
-      unsigned int* d_depth = nullptr;
-      if (s == RMG_OK) s = dev_alloc(&d_depth, 1, "depth");
-      if (s == RMG_OK) s = cuda_status(cudaMemsetAsync(d_depth, 0, 4, st), "memset");
+      s = sah_build(m, st, m->d_leaf_order);
       if (s == RMG_OK) {
-        k_depth<<<grid_for(n), kBlock, 0, st>>>(m->d_nodes, m->d_leaf_parent, n, d_depth);
-        s = cuda_status(cudaGetLastError(), "depth");
+        k_pack<<<grid_for(n), kBlock, 0, st>>>(m->d_vertices, m->d_faces, m->d_leaf_order, n, m->d_tris, nullptr);
+        s = cuda_status(cudaGetLastError(), "k_pack");
       }
-      unsigned int depth = 0;
-      if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&depth, d_depth, 4, cudaMemcpyDeviceToHost, st), "depth copy");
-      if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "sync");
-      cudaFree(d_depth);
       if (s != RMG_OK) { free_map(m); return s; }
-      m->depth = depth;
       s = wide_build(m, st);
       if (s != RMG_OK) { free_map(m); return s; }
       update_info(m, st);
