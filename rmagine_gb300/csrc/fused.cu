@@ -151,16 +151,18 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_trace_stats(const FusedParams 
   }
 }
 
-// One warp per pose: lanes 0..15 add moment k over the pose's partial records
-// in order; lane 0 forms the statistics and the Umeyama transform.
-__global__ void k_fused_final(const double* partial, uint32_t n_poses, uint32_t ctas, rmg_cross_stats* stats,
-                              rmg_transform* transforms) {
-  const uint32_t pose = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31;
-  if (pose >= n_poses) return;
+// One warp, one CTA per pose: each half warp adds moment k over every other
+// partial record of the pose, in order; lane 0 forms the statistics and the
+// Umeyama transform.  The solve is one thread's binary64 chain, so the poses are
+// spread over as many SMs as there are.
+__global__ void __launch_bounds__(32) k_fused_final(const double* partial, uint32_t ctas, rmg_cross_stats* stats,
+                                                    rmg_transform* transforms) {
+  const uint32_t pose = blockIdx.x, lane = threadIdx.x;
   double s = 0.0;
-  if (lane < 16)
-    for (uint32_t c = 0; c < ctas; ++c) s += partial[16ull * ((uint64_t)pose * ctas + c) + lane];
+  const double* p = partial + 16ull * pose * ctas + (lane & 15u);
+#pragma unroll 4
+  for (uint32_t c = lane >> 4; c < ctas; c += 2) s += __ldg(p + 16ull * c);
+  s += __shfl_down_sync(0xffffffffu, s, 16);
   double S[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) S[k] = __shfl_sync(0xffffffffu, s, k);
@@ -272,9 +274,7 @@ extern "C" int rmg_simulate_statistics(const rmg_map* map, const rmg_sensor* sen
                                          : launch_fused<false>(F, sensor->model.kind, (unsigned)grid, block, st);
     int s = cuda_status(e, "k_trace_stats");
     if (s == RMG_OK) {
-      const uint64_t threads = 32ull * n_poses;
-      k_fused_final<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(partial, n_poses, F.ctas_per_pose, stats,
-                                                                       transforms);
+      k_fused_final<<<n_poses, 32, 0, st>>>(partial, F.ctas_per_pose, stats, transforms);
       s = cuda_status(cudaGetLastError(), "k_fused_final");
     }
     cudaFreeAsync(partial, st);

@@ -106,14 +106,27 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_range_grad(const GradParams G)
   }
 }
 
-// Per pose and component, the warps' sums in slot order in binary64 (a fixed
-// order: the result does not depend on scheduling).
-__global__ void k_grad_final(const float* partial, uint32_t n_poses, uint32_t warps, float* grad, float* loss) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 7u * n_poses) return;
-  const uint32_t pose = i / 7, k = i - pose * 7;
+// One CTA per pose sums its warps' slots in binary64: thread t adds component
+// t & 7 of the slots t >> 3, t >> 3 + 32, ...  (a warp reads four whole slots at
+// a time), then the 32 strands are added in order.  A fixed order: the result
+// does not depend on scheduling.  A thread per pose and component read 2,048
+// slots 32 B apart one after the other: 298 us for 150 poses of 64 x 1024 rays,
+// a sixth of the whole call; this takes 16.
+constexpr int kFinalThreads = 256;
+
+__global__ void __launch_bounds__(kFinalThreads) k_grad_final(const float* partial, uint32_t n_poses, uint32_t warps,
+                                                              float* grad, float* loss) {
+  __shared__ double acc[kFinalThreads / 8][8];
+  const uint32_t pose = blockIdx.x, k = threadIdx.x & 7, strand = threadIdx.x >> 3;
+  const float* p = partial + 8ull * pose * warps + k;
   double s = 0.0;
-  for (uint32_t c = 0; c < warps; ++c) s += partial[8ull * ((uint64_t)pose * warps + c) + k];
+#pragma unroll 8
+  for (uint32_t c = strand; c < warps; c += kFinalThreads / 8) s += (double)__ldg(p + 8ull * c);
+  acc[strand][k] = s;
+  __syncthreads();
+  if (threadIdx.x >= 7) return;
+  s = 0.0;
+  for (int j = 0; j < kFinalThreads / 8; ++j) s += acc[j][k];
   if (k < 6) {
     if (grad) grad[6ull * pose + k] = (float)s;
   } else if (loss) {
@@ -198,7 +211,7 @@ extern "C" int rmg_range_pose_grad(const rmg_map* map, const rmg_sensor* sensor,
     }
     int s = cuda_status(e, "k_range_grad");
     if (s == RMG_OK) {
-      k_grad_final<<<(7 * n_poses + 255) / 256, 256, 0, st>>>(partial, n_poses, G.warps_per_pose, grad, loss);
+      k_grad_final<<<n_poses, kFinalThreads, 0, st>>>(partial, n_poses, G.warps_per_pose, grad, loss);
       s = cuda_status(cudaGetLastError(), "k_grad_final");
     }
     cudaFreeAsync(partial, st);

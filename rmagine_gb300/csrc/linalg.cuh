@@ -61,53 +61,70 @@ __host__ __device__ inline double m3_det(const M3d& m) {
          m.a[0][2] * (m.a[1][0] * m.a[2][1] - m.a[1][1] * m.a[2][0]);
 }
 
+__host__ __device__ inline double rsqrt_d(double x) {
+#ifdef __CUDA_ARCH__
+  return rsqrt(x);
+#else
+  return 1.0 / sqrt(x);
+#endif
+}
+
+// One Jacobi rotation of a symmetric 3x3 matrix on its axes p and q (r the
+// third): zeroes apq, V <- V J.  Everything stays in registers, and the chain
+// has three long operations (square root, division, reciprocal square root):
+// t = 2 apq / (d + sign(d) sqrt(d^2 + 4 apq^2)), d = aqq - app.  (An angle found
+// in binary32 with a binary64 normalisation measured slower: conversions and
+// one sweep more.)
+__host__ __device__ inline void jacobi_rotate(double& app, double& aqq, double& apq, double& arp, double& arq,
+                                              double vp[3], double vq[3]) {
+  if (fabs(apq) <= 1e-300) return;
+  const double d = aqq - app;
+  const double t = 2.0 * apq / (d + copysign(sqrt(d * d + 4.0 * apq * apq), d));
+  const double c = rsqrt_d(t * t + 1.0), s = t * c;
+  app -= t * apq;
+  aqq += t * apq;
+  apq = 0.0;
+  const double x = arp, y = arq;
+  arp = c * x - s * y;
+  arq = s * x + c * y;
+  for (int k = 0; k < 3; ++k) {
+    const double vx = vp[k], vy = vq[k];
+    vp[k] = c * vx - s * vy;
+    vq[k] = s * vx + c * vy;
+  }
+}
+
+__host__ __device__ inline void swap_columns(double& lx, double& ly, double x[3], double y[3]) {
+  if (!(lx < ly)) return;
+  double t = lx; lx = ly; ly = t;
+  for (int k = 0; k < 3; ++k) { t = x[k]; x[k] = y[k]; y[k] = t; }
+}
+
 // C = U diag(s) V^T with U, V proper rotations; s[0] >= s[1] >= |s[2]|, s[2] signed.
+//
+// One thread solves one matrix, so what counts is the latency of its binary64
+// chain.  400 matrices: 41 us with indexed arrays in local memory, five
+// divisions and square roots per rotation and four warps to an SM's narrow
+// binary64 pipe; 26 us in registers, with three, one warp to a CTA.
 __host__ __device__ inline void svd3_rot(const M3d& C, M3d& U, double s[3], M3d& V) {
-  M3d A = m3_mul_tn(C, C);
-  V = m3_eye();
-  double scale = 0.0;
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) scale = fmax(scale, fabs(A.a[i][j]));
+  const M3d A = m3_mul_tn(C, C);
+  double a00 = A.a[0][0], a11 = A.a[1][1], a22 = A.a[2][2], a01 = A.a[0][1], a02 = A.a[0][2], a12 = A.a[1][2];
+  double v0[3] = {1.0, 0.0, 0.0}, v1[3] = {0.0, 1.0, 0.0}, v2[3] = {0.0, 0.0, 1.0};  // columns of V
+  const double scale = fmax(fmax(fmax(fabs(a00), fabs(a11)), fmax(fabs(a22), fabs(a01))), fmax(fabs(a02), fabs(a12)));
   if (scale > 0.0) {
     for (int sweep = 0; sweep < 24; ++sweep) {
-      const double off = A.a[0][1] * A.a[0][1] + A.a[0][2] * A.a[0][2] + A.a[1][2] * A.a[1][2];
+      const double off = a01 * a01 + a02 * a02 + a12 * a12;
       if (off <= 1e-36 * scale * scale) break;
-      for (int p = 0; p < 2; ++p) {
-        for (int q = p + 1; q < 3; ++q) {
-          const double apq = A.a[p][q];
-          if (fabs(apq) <= 1e-300) continue;
-          const double theta = (A.a[q][q] - A.a[p][p]) / (2.0 * apq);
-          const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-          const double c = 1.0 / sqrt(t * t + 1.0), s_ = t * c;
-          for (int k = 0; k < 3; ++k) {  // A <- A J
-            const double akp = A.a[k][p], akq = A.a[k][q];
-            A.a[k][p] = c * akp - s_ * akq;
-            A.a[k][q] = s_ * akp + c * akq;
-          }
-          for (int k = 0; k < 3; ++k) {  // A <- J^T A
-            const double apk = A.a[p][k], aqk = A.a[q][k];
-            A.a[p][k] = c * apk - s_ * aqk;
-            A.a[q][k] = s_ * apk + c * aqk;
-          }
-          for (int k = 0; k < 3; ++k) {  // V <- V J
-            const double vkp = V.a[k][p], vkq = V.a[k][q];
-            V.a[k][p] = c * vkp - s_ * vkq;
-            V.a[k][q] = s_ * vkp + c * vkq;
-          }
-        }
-      }
+      jacobi_rotate(a00, a11, a01, a02, a12, v0, v1);
+      jacobi_rotate(a00, a22, a02, a01, a12, v0, v2);
+      jacobi_rotate(a11, a22, a12, a01, a02, v1, v2);
     }
   }
-  // sort eigenvalues descending (swap V columns)
-  double lam[3] = {A.a[0][0], A.a[1][1], A.a[2][2]};
-  for (int i = 0; i < 2; ++i) {
-    for (int j = 0; j < 2 - i; ++j) {
-      if (lam[j] < lam[j + 1]) {
-        const double t = lam[j]; lam[j] = lam[j + 1]; lam[j + 1] = t;
-        for (int k = 0; k < 3; ++k) { const double v = V.a[k][j]; V.a[k][j] = V.a[k][j + 1]; V.a[k][j + 1] = v; }
-      }
-    }
-  }
+  // eigenvalues descending
+  swap_columns(a00, a11, v0, v1);
+  swap_columns(a11, a22, v1, v2);
+  swap_columns(a00, a11, v0, v1);
+  for (int k = 0; k < 3; ++k) { V.a[k][0] = v0[k]; V.a[k][1] = v1[k]; V.a[k][2] = v2[k]; }
   if (m3_det(V) < 0.0)
     for (int k = 0; k < 3; ++k) V.a[k][2] = -V.a[k][2];
   // B = C V: columns b_i = s_i u_i
@@ -119,20 +136,20 @@ __host__ __device__ inline void svd3_rot(const M3d& C, M3d& U, double s[3], M3d&
     s[0] = s[1] = s[2] = 0.0;
     return;
   }
-  for (int k = 0; k < 3; ++k) u1[k] /= n1;
+  const double r1 = 1.0 / n1;
+  for (int k = 0; k < 3; ++k) u1[k] *= r1;
   double u2[3] = {B.a[0][1], B.a[1][1], B.a[2][1]};
   double d12 = u1[0] * u2[0] + u1[1] * u2[1] + u1[2] * u2[2];
   for (int k = 0; k < 3; ++k) u2[k] -= d12 * u1[k];
   double n2 = sqrt(u2[0] * u2[0] + u2[1] * u2[1] + u2[2] * u2[2]);
   if (!(n2 > 1e-12 * n1)) {  // rank 1: any unit vector orthogonal to u1
     const int k = (fabs(u1[0]) <= fabs(u1[1]) && fabs(u1[0]) <= fabs(u1[2])) ? 0 : (fabs(u1[1]) <= fabs(u1[2]) ? 1 : 2);
-    double e[3] = {0.0, 0.0, 0.0};
-    e[k] = 1.0;
-    d12 = u1[k];
-    for (int j = 0; j < 3; ++j) u2[j] = e[j] - d12 * u1[j];
+    d12 = k == 0 ? u1[0] : (k == 1 ? u1[1] : u1[2]);
+    for (int j = 0; j < 3; ++j) u2[j] = (j == k ? 1.0 : 0.0) - d12 * u1[j];
     n2 = sqrt(u2[0] * u2[0] + u2[1] * u2[1] + u2[2] * u2[2]);
   }
-  for (int k = 0; k < 3; ++k) u2[k] /= n2;
+  const double r2 = 1.0 / n2;
+  for (int k = 0; k < 3; ++k) u2[k] *= r2;
   const double u3[3] = {u1[1] * u2[2] - u1[2] * u2[1], u1[2] * u2[0] - u1[0] * u2[2], u1[0] * u2[1] - u1[1] * u2[0]};
   for (int k = 0; k < 3; ++k) { U.a[k][0] = u1[k]; U.a[k][1] = u2[k]; U.a[k][2] = u3[k]; }
   s[0] = n1;
@@ -145,33 +162,21 @@ __host__ __device__ inline void svd3_rot(const M3d& C, M3d& U, double s[3], M3d&
 // so both pick the same of the two signs q / -q.
 __host__ __device__ inline void rot_to_quat(const M3d& R, double q[4]) {
   const double tr = R.a[0][0] + R.a[1][1] + R.a[2][2];
-  if (tr > 0.0) {
-    const double S = sqrt(tr + 1.0) * 2.0;
-    q[3] = 0.25 * S;
-    q[0] = (R.a[2][1] - R.a[1][2]) / S;
-    q[1] = (R.a[0][2] - R.a[2][0]) / S;
-    q[2] = (R.a[1][0] - R.a[0][1]) / S;
-  } else if (R.a[0][0] > R.a[1][1] && R.a[0][0] > R.a[2][2]) {
-    const double S = sqrt(1.0 + R.a[0][0] - R.a[1][1] - R.a[2][2]) * 2.0;
-    q[3] = (R.a[2][1] - R.a[1][2]) / S;
-    q[0] = 0.25 * S;
-    q[1] = (R.a[0][1] + R.a[1][0]) / S;
-    q[2] = (R.a[0][2] + R.a[2][0]) / S;
-  } else if (R.a[1][1] > R.a[2][2]) {
-    const double S = sqrt(1.0 + R.a[1][1] - R.a[0][0] - R.a[2][2]) * 2.0;
-    q[3] = (R.a[0][2] - R.a[2][0]) / S;
-    q[0] = (R.a[0][1] + R.a[1][0]) / S;
-    q[1] = 0.25 * S;
-    q[2] = (R.a[1][2] + R.a[2][1]) / S;
-  } else {
-    const double S = sqrt(1.0 + R.a[2][2] - R.a[0][0] - R.a[1][1]) * 2.0;
-    q[3] = (R.a[1][0] - R.a[0][1]) / S;
-    q[0] = (R.a[0][2] + R.a[2][0]) / S;
-    q[1] = (R.a[1][2] + R.a[2][1]) / S;
-    q[2] = 0.25 * S;
-  }
-  const double n = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
-  for (int k = 0; k < 4; ++k) q[k] /= n;
+  // S^2 / 4 and which component it is; the others are sums over S
+  const int big = tr > 0.0 ? 3 : (R.a[0][0] > R.a[1][1] && R.a[0][0] > R.a[2][2]) ? 0 : (R.a[1][1] > R.a[2][2] ? 1 : 2);
+  const double x = R.a[2][1] - R.a[1][2], y = R.a[0][2] - R.a[2][0], z = R.a[1][0] - R.a[0][1];
+  const double xy = R.a[0][1] + R.a[1][0], xz = R.a[0][2] + R.a[2][0], yz = R.a[1][2] + R.a[2][1];
+  const double arg = big == 3 ? tr + 1.0
+                              : big == 0 ? 1.0 + R.a[0][0] - R.a[1][1] - R.a[2][2]
+                                         : big == 1 ? 1.0 + R.a[1][1] - R.a[0][0] - R.a[2][2]
+                                                    : 1.0 + R.a[2][2] - R.a[0][0] - R.a[1][1];
+  const double S = sqrt(arg) * 2.0, rS = 1.0 / S;
+  if (big == 3) { q[3] = 0.25 * S; q[0] = x * rS; q[1] = y * rS; q[2] = z * rS; }
+  else if (big == 0) { q[3] = x * rS; q[0] = 0.25 * S; q[1] = xy * rS; q[2] = xz * rS; }
+  else if (big == 1) { q[3] = y * rS; q[0] = xy * rS; q[1] = 0.25 * S; q[2] = yz * rS; }
+  else { q[3] = z * rS; q[0] = xz * rS; q[1] = yz * rS; q[2] = 0.25 * S; }
+  const double n = 1.0 / sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+  for (int k = 0; k < 4; ++k) q[k] *= n;
 }
 
 // Umeyama / Kabsch: R = U V^T, t = m - R d.  n == 0 or a non-finite result

@@ -31,6 +31,10 @@ namespace rmg {
 namespace {
 
 constexpr int kStatsThreads = 256;
+// Threads of the CTAs that solve one 3x3 problem per thread: one warp, so that
+// a few hundred problems reach as many SMs as there are and no two warps share
+// an SM's narrow binary64 pipe.
+constexpr int kSolveThreads = 32;
 constexpr int kFold = 8;  // vector groups (4 correspondences) per binary32 run
 
 struct StatsParams {
@@ -60,15 +64,19 @@ __device__ __forceinline__ Tf batch_pre(const StatsParams& P, uint32_t b) {
   return load_tf(P.pre[P.pre_stride ? b : 0]);
 }
 
+__device__ __forceinline__ bool passes(const StatsParams& P, uint64_t i) {
+  if (P.dmask && P.dmask[i] == 0) return false;
+  if (P.mmask && P.mmask[i] == 0) return false;
+  if (P.dids && P.dids[i] != P.dataset_id) return false;
+  return !(P.mids && P.mids[i] != P.model_id);
+}
+
 // PRE = false: no pre-transform (rotating by the identity quaternion is exact, so
 // skipping it changes no bit).
 template <bool P2L, bool PRE = true>
 __device__ __forceinline__ bool correspondence(const StatsParams& P, const Tf& pre, uint64_t i, const V& dpt,
                                                const V& mpt, const V& npt, V& D, V& M) {
-  if (P.dmask && P.dmask[i] == 0) return false;
-  if (P.mmask && P.mmask[i] == 0) return false;
-  if (P.dids && P.dids[i] != P.dataset_id) return false;
-  if (P.mids && P.mids[i] != P.model_id) return false;
+  if (!passes(P, i)) return false;
   D = PRE ? tf_point(pre, dpt) : dpt;
   return match<P2L>(D, mpt, npt, P.max_dist, M);
 }
@@ -157,40 +165,71 @@ __global__ void __launch_bounds__(kStatsThreads, 3) k_stats(const StatsParams P)
   f.zero();
   const V zero{0.f, 0.f, 0.f};
   if (VEC) {
-    // thread t takes groups of 4 consecutive correspondences: 3 x 16-byte loads per array
-    const uint32_t g0 = lo / 4, g1 = (hi + 3) / 4;
+    // Thread t takes groups of 4 consecutive correspondences -- 3 x 16-byte loads
+    // per array, one word of masks -- counted over the whole array, so that they
+    // are aligned whatever n_per is; a batch's first and last group may hold
+    // neighbours of other batches, which are skipped, and the array's last group
+    // is read one by one if it is cut short.  400 batches of 10,007 with masks and
+    // pre-transforms: 46 us, one correspondence at a time 51.
+    const uint64_t e0 = base + lo, e1 = base + hi, total = (uint64_t)P.n_batches * P.n_per;
+    const uint64_t g0 = e0 / 4, g1 = lo < hi ? (e1 + 3) / 4 : g0;
     int run = 0;
     // warp-uniform trip count (lanes past the end skip the loads)
-    const uint32_t iters = (g1 - g0 + blockDim.x - 1) / blockDim.x;
+    const uint32_t iters = (uint32_t)((g1 - g0 + blockDim.x - 1) / blockDim.x);
     for (uint32_t it = 0; it < iters; ++it) {
-      const uint32_t g = g0 + threadIdx.x + it * blockDim.x;
+      const uint64_t g = g0 + threadIdx.x + (uint64_t)it * blockDim.x;
       if (g < g1) {
-      const uint64_t e = base + 4ull * g;
-      const float4* dv = reinterpret_cast<const float4*>(P.dp + 3 * e);
-      const float4* mv = reinterpret_cast<const float4*>(P.mp + 3 * e);
-      float dd[12], mmv[12], nn[12];
-      *reinterpret_cast<float4*>(dd + 0) = __ldg(dv + 0);
-      *reinterpret_cast<float4*>(dd + 4) = __ldg(dv + 1);
-      *reinterpret_cast<float4*>(dd + 8) = __ldg(dv + 2);
-      *reinterpret_cast<float4*>(mmv + 0) = __ldg(mv + 0);
-      *reinterpret_cast<float4*>(mmv + 4) = __ldg(mv + 1);
-      *reinterpret_cast<float4*>(mmv + 8) = __ldg(mv + 2);
-      if (P2L) {
-        const float4* nv = reinterpret_cast<const float4*>(P.mn + 3 * e);
-        *reinterpret_cast<float4*>(nn + 0) = __ldg(nv + 0);
-        *reinterpret_cast<float4*>(nn + 4) = __ldg(nv + 1);
-        *reinterpret_cast<float4*>(nn + 8) = __ldg(nv + 2);
-      }
+        const uint64_t e = 4 * g;
+        float dd[12], mmv[12], nn[12];
+        uint32_t keep = 0;  // bit k: correspondence e + k is this CTA's and passes the masks and ids
+        if (e + 4 <= total) {
+          const float4* dv = reinterpret_cast<const float4*>(P.dp + 3 * e);
+          const float4* mv = reinterpret_cast<const float4*>(P.mp + 3 * e);
+          *reinterpret_cast<float4*>(dd + 0) = __ldg(dv + 0);
+          *reinterpret_cast<float4*>(dd + 4) = __ldg(dv + 1);
+          *reinterpret_cast<float4*>(dd + 8) = __ldg(dv + 2);
+          *reinterpret_cast<float4*>(mmv + 0) = __ldg(mv + 0);
+          *reinterpret_cast<float4*>(mmv + 4) = __ldg(mv + 1);
+          *reinterpret_cast<float4*>(mmv + 8) = __ldg(mv + 2);
+          if (P2L) {
+            const float4* nv = reinterpret_cast<const float4*>(P.mn + 3 * e);
+            *reinterpret_cast<float4*>(nn + 0) = __ldg(nv + 0);
+            *reinterpret_cast<float4*>(nn + 4) = __ldg(nv + 1);
+            *reinterpret_cast<float4*>(nn + 8) = __ldg(nv + 2);
+          }
+          const uint32_t dm = P.dmask ? __ldg(reinterpret_cast<const uint32_t*>(P.dmask + e)) : 0x01010101u;
+          const uint32_t mm = P.mmask ? __ldg(reinterpret_cast<const uint32_t*>(P.mmask + e)) : 0x01010101u;
+          const uint4 di = P.dids ? __ldg(reinterpret_cast<const uint4*>(P.dids + e))
+                                  : make_uint4(P.dataset_id, P.dataset_id, P.dataset_id, P.dataset_id);
+          const uint4 mi = P.mids ? __ldg(reinterpret_cast<const uint4*>(P.mids + e))
+                                  : make_uint4(P.model_id, P.model_id, P.model_id, P.model_id);
+          const bool id[4] = {di.x == P.dataset_id && mi.x == P.model_id, di.y == P.dataset_id && mi.y == P.model_id,
+                              di.z == P.dataset_id && mi.z == P.model_id, di.w == P.dataset_id && mi.w == P.model_id};
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t j = 4 * g + k;
-        if (j < lo || j >= hi) continue;
-        V D, M;
-        const V np = P2L ? V{nn[3 * k], nn[3 * k + 1], nn[3 * k + 2]} : zero;
-        if (correspondence<P2L, PRE>(P, pre, base + j, V{dd[3 * k], dd[3 * k + 1], dd[3 * k + 2]},
-                                V{mmv[3 * k], mmv[3 * k + 1], mmv[3 * k + 2]}, np, D, M))
-          f.add_pt(D, M, sd, sm);
-      }
+          for (int k = 0; k < 4; ++k)
+            if (id[k] && (dm & (0xffu << (8 * k))) != 0 && (mm & (0xffu << (8 * k))) != 0 && e + k >= e0 && e + k < e1)
+              keep |= 1u << k;
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (e + k >= e1 || e + k < e0) continue;
+            const uint64_t i = e + k;
+            const V d3 = ldv(P.dp, i), m3 = ldv(P.mp, i), n3 = P2L ? ldv(P.mn, i) : zero;
+            dd[3 * k] = d3.x; dd[3 * k + 1] = d3.y; dd[3 * k + 2] = d3.z;
+            mmv[3 * k] = m3.x; mmv[3 * k + 1] = m3.y; mmv[3 * k + 2] = m3.z;
+            if (P2L) { nn[3 * k] = n3.x; nn[3 * k + 1] = n3.y; nn[3 * k + 2] = n3.z; }
+            if (passes(P, i)) keep |= 1u << k;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (!(keep >> k & 1u)) continue;
+          const V dpt{dd[3 * k], dd[3 * k + 1], dd[3 * k + 2]};
+          const V np = P2L ? V{nn[3 * k], nn[3 * k + 1], nn[3 * k + 2]} : zero;
+          const V D = PRE ? tf_point(pre, dpt) : dpt;
+          V M;
+          if (match<P2L>(D, V{mmv[3 * k], mmv[3 * k + 1], mmv[3 * k + 2]}, np, P.max_dist, M)) f.add_pt(D, M, sd, sm);
+        }
       }
       if (++run == kFold) { fold(acc, f); run = 0; }
     }
@@ -396,9 +435,12 @@ int fill_params(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
   return RMG_OK;
 }
 
+// The 4-correspondence loads need aligned arrays (16 bytes; 4 for byte masks),
+// nothing of the batch size.
 bool vec_ok(const StatsParams& P, bool p2l) {
   auto al = [](const void* p, uintptr_t a) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) % a) == 0; };
-  return (P.n_per % 4 == 0) && al(P.dp, 16) && al(P.mp, 16) && (!p2l || al(P.mn, 16));
+  return al(P.dp, 16) && al(P.mp, 16) && (!p2l || al(P.mn, 16)) && al(P.dmask, 4) && al(P.mmask, 4) &&
+         al(P.dids, 16) && al(P.mids, 16);
 }
 
 int launch_stats(StatsParams& P, bool p2l, cudaStream_t st) {
@@ -447,7 +489,7 @@ int stats_entry(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
   }
   s = launch_stats(P, p2l, st);
   if (s == RMG_OK && transforms) {
-    k_umeyama_dstats<<<(n_batches + 127) / 128, 128, 0, st>>>(dstats, n_batches, transforms);
+    k_umeyama_dstats<<<(n_batches + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, st>>>(dstats, n_batches, transforms);
     s = cuda_status(cudaGetLastError(), "k_umeyama_dstats");
   }
   if (dstats) cudaFreeAsync(dstats, st);
@@ -531,8 +573,8 @@ extern "C" int rmg_svd3(const float* A, float* U, float* W, float* w, float* V, 
     if (n == 0) return RMG_OK;
     if (!A) return fail(RMG_ERR_INVALID_ARG, "rmg_svd3: A is NULL");
     if (!U && !W && !w && !V) return RMG_OK;
-    const uint64_t grid = (n + 127ull) / 128ull;
-    k_svd3<<<(unsigned)grid, 128, 0, as_stream(stream)>>>(A, U, W, w, V, n, rotations);
+    const uint64_t grid = ((uint64_t)n + kSolveThreads - 1) / kSolveThreads;
+    k_svd3<<<(unsigned)grid, kSolveThreads, 0, as_stream(stream)>>>(A, U, W, w, V, n, rotations);
     return cuda_status(cudaGetLastError(), "k_svd3");
   });
 }
@@ -541,7 +583,7 @@ extern "C" int rmg_umeyama_transform(const rmg_cross_stats* stats, uint32_t n, r
   return guarded("rmg_umeyama_transform", [&]() -> int {
     if (n == 0) return RMG_OK;
     if (!stats || !out) return fail(RMG_ERR_INVALID_ARG, "rmg_umeyama_transform: NULL argument");
-    k_umeyama_stats<<<(n + 127) / 128, 128, 0, as_stream(stream)>>>(stats, n, out);
+    k_umeyama_stats<<<(n + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, as_stream(stream)>>>(stats, n, out);
     return cuda_status(cudaGetLastError(), "k_umeyama_stats");
   });
 }
@@ -564,7 +606,7 @@ extern "C" int rmg_umeyama_backward(const rmg_transform* pre_transforms, uint32_
     cudaStream_t st = as_stream(stream);
     Coef* coef = nullptr;
     RMG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&coef), sizeof(Coef) * (size_t)n_batches, st));
-    k_umeyama_bwd_coef<<<(n_batches + 127) / 128, 128, 0, st>>>(stats, grad_R, grad_t, n_batches, coef);
+    k_umeyama_bwd_coef<<<(n_batches + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, st>>>(stats, grad_R, grad_t, n_batches, coef);
     s = cuda_status(cudaGetLastError(), "k_umeyama_bwd_coef");
     if (s == RMG_OK) {
       B.coef = coef;
