@@ -50,9 +50,12 @@ struct BatchParams {
   int wide;  // walk the 4-wide tree
 };
 
+// A warp's tile of one job.  The composed pose (formed by lane 0) waits in
+// shared memory and the job's record in global memory while the rays walk: kept
+// in registers they were spilled into the walk.
 template <int OK, int SS, int TB>
 __device__ __forceinline__ void batched_ray(const BatchParams& B, const JobDev& J, uint64_t tile_in_job,
-                                            uint32_t lane) {
+                                            uint32_t lane, Tf* s_tsm) {
   const uint32_t pose = (uint32_t)(tile_in_job / J.tiles_per_pose);
   const uint32_t r = (uint32_t)(tile_in_job - (uint64_t)pose * J.tiles_per_pose);
   const uint32_t ty = r / J.tiles_x, tx = r - ty * J.tiles_x;
@@ -60,21 +63,23 @@ __device__ __forceinline__ void batched_ray(const BatchParams& B, const JobDev& 
   const uint32_t vid = ty * J.tile_h + (lane >> J.tile_w_log2);
   const uint32_t hid = tx * tile_w + (lane & (tile_w - 1));
   const uint32_t W = J.sen.width, H = J.sen.height;
+  __syncwarp();
+  if (lane == 0) *s_tsm = tmul(load_tf(J.Tbm[pose]), J.Tsb);
+  __syncwarp();
   if (vid >= H || hid >= W) return;
   const uint32_t loc = visit_loc(J.sen, vid * W + hid);
   const uint64_t gid = (uint64_t)pose * W * H + loc;
-  const Tf Tsm = tmul(load_tf(J.Tbm[pose]), J.Tsb);
-  V dir_s, orig_s, o, d;
-  setup_ray<OK>(J.sen, Tsm, loc, dir_s, orig_s, o, d);
   Hit h;
   bool over = false;
-  trace_ray<SS, TB>(B.map, o, d, J.sen.range_max, B.budget, h, over);
+  {
+    V dir_s, orig_s, o, d;
+    setup_ray<OK>(J.sen, reread(s_tsm), loc, dir_s, orig_s, o, d);
+    trace_ray<SS, TB>(B.map, o, d, J.sen.range_max, B.budget, h, over);
+  }
   if (over) atomicExch(B.map.status, (unsigned)RMG_ERR_TRAVERSAL_BUDGET);
-  TraceParams P;  // the epilogue reads only map, sensor range and outputs
-  P.map = B.map;
-  P.sen = J.sen;
-  P.out = J.out;
-  write_attributes<OK>(P, gid, h, dir_s, orig_s, Tsm);
+  V dir_s, orig_s;
+  reread_ray<OK>(J.sen, loc, dir_s, orig_s);
+  write_attributes<OK>(B.map, J.sen.range_min, J.sen.range_max, J.out, gid, h, dir_s, orig_s, reread(s_tsm));
 }
 
 template <int SS, int TB>
@@ -86,7 +91,9 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_trace_batched(const BatchParam
     if (threadIdx.x == 0) s_begin[B.n_jobs] = B.total_tiles;
   }
   __syncthreads();
+  __shared__ Tf s_tsm[8];
   const uint32_t lane = threadIdx.x & 31;
+  Tf* tsm = s_tsm + (threadIdx.x >> 5);
   for (;;) {
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(B.counter, (unsigned long long)B.grab);
@@ -106,9 +113,9 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_trace_batched(const BatchParam
       const uint64_t t = tile - J.tile_begin;
       switch (J.sen.kind) {
         case RMG_MODEL_SPHERICAL:
-        case RMG_MODEL_PINHOLE: batched_ray<ORIGIN_POSE, SS, TB>(B, J, t, lane); break;
-        case RMG_MODEL_O1DN: batched_ray<ORIGIN_SINGLE, SS, TB>(B, J, t, lane); break;
-        default: batched_ray<ORIGIN_TABLE, SS, TB>(B, J, t, lane); break;
+        case RMG_MODEL_PINHOLE: batched_ray<ORIGIN_POSE, SS, TB>(B, J, t, lane, tsm); break;
+        case RMG_MODEL_O1DN: batched_ray<ORIGIN_SINGLE, SS, TB>(B, J, t, lane, tsm); break;
+        default: batched_ray<ORIGIN_TABLE, SS, TB>(B, J, t, lane, tsm); break;
       }
     }
   }

@@ -192,7 +192,11 @@ struct RayW {
 
 __device__ __forceinline__ float comp(const V& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
-__device__ __forceinline__ RayW make_rayw(const V& o, const V& d) {
+// 1/d per component, correctly rounded: shared by the slab constants and the
+// triangle test.
+__device__ __forceinline__ V reciprocal(const V& d) { return V{__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)}; }
+
+__device__ __forceinline__ RayW make_rayw(const V& o, const V& d, const V& inv) {
   RayW r;
   const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   int kz = 0;
@@ -206,7 +210,7 @@ __device__ __forceinline__ RayW make_rayw(const V& o, const V& d) {
   r.bx = 4u * (uint32_t)kx; r.by = 4u * (uint32_t)ky; r.bz = 4u * (uint32_t)kz;
   r.Sx = __fdiv_rn(comp(d, kx), dz);
   r.Sy = __fdiv_rn(comp(d, ky), dz);
-  r.Sz = __fdiv_rn(1.0f, dz);
+  r.Sz = comp(inv, kz);  // = 1 / dz
   return r;
 }
 

@@ -86,15 +86,18 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_trace_stats(const FusedParams 
   const uint32_t cta = blockIdx.x - pose * F.ctas_per_pose;
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const uint32_t W = P.sen.width, H = P.sen.height;
-  const Tf Tsm = tmul(load_tf(P.Tbm[pose]), P.Tsb);
-  const Tf pre = F.pre ? load_tf(F.pre[F.pre_stride ? pose : 0]) : Tf{Q{0.f, 0.f, 0.f, 1.f}, V{0.f, 0.f, 0.f}};
+  // the pose's transforms wait in shared memory, not in registers, while rays walk
+  __shared__ Tf s_tsm, s_pre;
+  if (threadIdx.x == 0) s_tsm = tmul(load_tf(P.Tbm[pose]), P.Tsb);
+  if (threadIdx.x == 32 % blockDim.x && F.pre) s_pre = load_tf(F.pre[F.pre_stride ? pose : 0]);
+  __syncthreads();
   const uint64_t dbase = (uint64_t)pose * F.d_stride;
   const uint32_t tile_w = 1u << P.tile_w_log2;
   double acc = 0.0;
   const uint32_t t0 = cta * F.tiles_per_cta;
   const uint32_t t1 = min(P.tiles_per_pose, t0 + F.tiles_per_cta);
   for (uint32_t tile = t0 + wib; tile < t1; tile += nw) {  // warp-uniform
-    const uint32_t ty = tile / P.tiles_x, tx = tile - ty * P.tiles_x;
+    const uint32_t ty = P.by_tiles_x(tile), tx = tile - ty * P.tiles_x;
     const uint32_t vid = ty * P.tile_h + (lane >> P.tile_w_log2);
     const uint32_t hid = tx * tile_w + (lane & (tile_w - 1));
     bool ok = false;
@@ -103,17 +106,21 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_trace_stats(const FusedParams 
       const uint32_t loc = visit_loc(P.sen, vid * W + hid);
       const uint64_t di = dbase + loc;
       if ((!F.dmask || F.dmask[di] != 0) && (!F.dids || F.dids[di] == F.dataset_id)) {
-        V dir_s, orig_s, o, d;
-        setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
         Hit h;
         bool over = false;
-        trace_ray<SS, TB>(P.map, o, d, P.sen.range_max, P.budget, h, over);
+        {
+          V dir_s, orig_s, o, d;
+          setup_ray<OK>(P.sen, reread(&s_tsm), loc, dir_s, orig_s, o, d);
+          trace_ray<SS, TB>(P.map, o, d, P.sen.range_max, P.budget, h, over);
+        }
         if (over) atomicExch(P.map.status, (unsigned)RMG_ERR_TRAVERSAL_BUDGET);
         if (h.tri >= 0 && h.t >= P.sen.range_min) {
+          V dir_s, orig_s;
+          reread_ray<OK>(P.sen, loc, dir_s, orig_s);
           const V mpt = hit_point<OK>(dir_s, orig_s, h.t);
-          const V npt = P2L ? hit_normal(P.map, h, dir_s, Tsm) : V{0.f, 0.f, 0.f};
+          const V npt = P2L ? hit_normal(P.map, h, dir_s, reread(&s_tsm)) : V{0.f, 0.f, 0.f};
           const V dpt{__ldg(F.dp + 3 * di), __ldg(F.dp + 3 * di + 1), __ldg(F.dp + 3 * di + 2)};
-          D = F.pre ? tf_point(pre, dpt) : dpt;
+          D = F.pre ? tf_point(reread(&s_pre), dpt) : dpt;
           ok = match<P2L>(D, mpt, npt, F.max_dist, M);
         }
       }

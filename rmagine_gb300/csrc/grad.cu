@@ -36,27 +36,33 @@ struct GradParams {
 template <int OK, int SS, int TB>
 __global__ void __maxnreg__((trace_regs<TB>())) k_range_grad(const GradParams G) {
   const TraceParams& P = G.T;
+  __shared__ Tf s_tsm;
   const uint32_t pose = blockIdx.y;
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t tile = blockIdx.x * (blockDim.x >> 5) + wib;
+  if (threadIdx.x == 0) s_tsm = tmul(load_tf(P.Tbm[pose]), P.Tsb);
+  __syncthreads();
   float acc[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (tile < P.tiles_per_pose) {
-    const uint32_t ty = tile / P.tiles_x, tx = tile - ty * P.tiles_x;
+    const uint32_t ty = P.by_tiles_x(tile), tx = tile - ty * P.tiles_x;
     const uint32_t tile_w = 1u << P.tile_w_log2;
     const uint32_t vid = ty * P.tile_h + (lane >> P.tile_w_log2);
     const uint32_t hid = tx * tile_w + (lane & (tile_w - 1));
     const uint32_t W = P.sen.width, H = P.sen.height;
     if (vid < H && hid < W) {
       const uint32_t loc = visit_loc(P.sen, vid * W + hid);
-      const uint64_t gid = (uint64_t)pose * W * H + loc;
-      const Tf Tbm = load_tf(P.Tbm[pose]);
-      const Tf Tsm = tmul(Tbm, P.Tsb);
-      V dir_s, orig_s, o, d;
-      setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
       Hit h;
       bool over = false;
-      trace_ray<SS, TB>(P.map, o, d, P.sen.range_max, P.budget, h, over);
+      {
+        const Tf Tsm = s_tsm;
+        V dir_s, orig_s, o, d;
+        setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
+        trace_ray<SS, TB>(P.map, o, d, P.sen.range_max, P.budget, h, over);
+      }
       if (over) atomicExch(P.map.status, (unsigned)RMG_ERR_TRAVERSAL_BUDGET);
+      const uint64_t gid = (uint64_t)pose * W * H + loc;
+      V dir_s, orig_s;
+      reread_ray<OK>(P.sen, loc, dir_s, orig_s);
       if (P.out.ranges) P.out.ranges[gid] = h.tri >= 0 ? h.t : add(P.sen.range_max, 1.0f);
       if (P.out.face_ids) P.out.face_ids[gid] = h.tri >= 0 ? h.face : 0xffffffffu;
       const float obs = __ldg(G.r_obs + gid);
@@ -71,7 +77,8 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_range_grad(const GradParams G)
         const float e1x = p1.x - p0.x, e1y = p1.y - p0.y, e1z = p1.z - p0.z;
         const float e2x = p2.x - p0.x, e2y = p2.y - p0.y, e2z = p2.z - p0.z;
         const V nm{e1y * e2z - e1z * e2y, e1z * e2x - e1x * e2z, e1x * e2y - e1y * e2x};
-        const V nb = qrot(qconj(Tbm.R), nm);
+        const rmg_quat& q = P.Tbm[pose].R;
+        const V nb = qrot(qconj(Q{q.x, q.y, q.z, q.w}), nm);
         const V db = qrot(P.Tsb.R, dir_s);
         V ob = P.Tsb.t;
         if (OK != ORIGIN_POSE) {

@@ -176,7 +176,7 @@ __device__ __forceinline__ void trace_scene(const SceneParams& S, const V& o, co
     }
     return;
   }
-  const RayBox rb = make_raybox(o, d);
+  const RayBox rb = make_raybox(o, d, reciprocal(d));
   int stk_node[kFullStack];
   float stk_t[kFullStack];
   int sp = 0;

@@ -81,6 +81,8 @@ int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_tr
   const uint32_t tiles_y = (sensor->height + th - 1) / th;
   P.tiles_per_pose = P.tiles_x * tiles_y;
   P.n_tiles = (uint64_t)P.tiles_per_pose * n_poses;
+  P.by_tiles_per_pose = fast_div(P.tiles_per_pose);
+  P.by_tiles_x = fast_div(P.tiles_x);
   P.budget = 2u * map->n_nodes + 64u;
   P.trail_bits = trail_bits_for_depth(map->depth);
   P.full_stack = map->depth <= (unsigned)kFullStack ? 1 : 0;

@@ -76,11 +76,11 @@ __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
 }
 #endif
 
-__device__ __forceinline__ RayBox make_raybox(const V& o, const V& d) {
+__device__ __forceinline__ RayBox make_raybox(const V& o, const V& d, const V& inv) {
   RayBox r;
-  r.ix = fabsf(d.x) > 1e-20f ? __frcp_rn(d.x) : copysignf(1e20f, d.x);
-  r.iy = fabsf(d.y) > 1e-20f ? __frcp_rn(d.y) : copysignf(1e20f, d.y);
-  r.iz = fabsf(d.z) > 1e-20f ? __frcp_rn(d.z) : copysignf(1e20f, d.z);
+  r.ix = fabsf(d.x) > 1e-20f ? inv.x : copysignf(1e20f, d.x);
+  r.iy = fabsf(d.y) > 1e-20f ? inv.y : copysignf(1e20f, d.y);
+  r.iz = fabsf(d.z) > 1e-20f ? inv.z : copysignf(1e20f, d.z);
   // explicit roundings: the 8-wide walk's leaf test (leaf_exact) repeats these operations
   const float oix = __fmul_rn(o.x, r.ix), oiy = __fmul_rn(o.y, r.iy), oiz = __fmul_rn(o.z, r.iz);
   const float kE = 4.76837158e-7f;  // 2^-21
@@ -228,8 +228,9 @@ struct RayTrav {
     trail = Trail<TB>();
     node = map.root;
     if (map.root < 0) return false;
-    rw = make_rayw(o, d);
-    rb = make_raybox(o, d);
+    const V inv = reciprocal(d);
+    rw = make_rayw(o, d, inv);
+    rb = make_raybox(o, d, inv);
     return true;
   }
 
@@ -392,8 +393,9 @@ __device__ __forceinline__ void trace_ray4(const DeviceMap& map, const V& o, con
   z = fmaf(o.y, 0.0f, z); z = fmaf(o.z, 0.0f, z);
   z = fmaf(d.x, 0.0f, z); z = fmaf(d.y, 0.0f, z); z = fmaf(d.z, 0.0f, z);
   if (z != 0.0f) return;
-  const RayW rw = make_rayw(o, d);
-  const RayBox rb = make_raybox(o, d);
+  const V inv = reciprocal(d);
+  const RayW rw = make_rayw(o, d, inv);
+  const RayBox rb = make_raybox(o, d, inv);
   const bool bx = rb.ix < 0.f, by = rb.iy < 0.f, bz = rb.iz < 0.f;
   const unsigned long long pix = pack2(rb.ix, rb.ix), piy = pack2(rb.iy, rb.iy), piz = pack2(rb.iz, rb.iz);
   const float nxa = bx ? rb.chx : rb.clx, fxa = bx ? rb.clx : rb.chx;
@@ -568,10 +570,11 @@ __device__ __forceinline__ void trace_ray8(const DeviceMap& map, const V& o, con
   h.tri = -1;
   h.face = 0xffffffffu;
   if (map.root < 0) return;
-  const RayW rw = make_rayw(o, d);
-  const float ix = fabsf(d.x) > 1e-20f ? __frcp_rn(d.x) : copysignf(1e20f, d.x);
-  const float iy = fabsf(d.y) > 1e-20f ? __frcp_rn(d.y) : copysignf(1e20f, d.y);
-  const float iz = fabsf(d.z) > 1e-20f ? __frcp_rn(d.z) : copysignf(1e20f, d.z);
+  const V inv = reciprocal(d);
+  const RayW rw = make_rayw(o, d, inv);
+  const float ix = fabsf(d.x) > 1e-20f ? inv.x : copysignf(1e20f, d.x);
+  const float iy = fabsf(d.y) > 1e-20f ? inv.y : copysignf(1e20f, d.y);
+  const float iz = fabsf(d.z) > 1e-20f ? inv.z : copysignf(1e20f, d.z);
   const float nx = -__fmul_rn(o.x, ix), ny = -__fmul_rn(o.y, iy), nz = -__fmul_rn(o.z, iz);
   const float kE = 4.76837158e-7f;  // 2^-21
   const float ex = fabsf(nx) * kE, ey = fabsf(ny) * kE, ez = fabsf(nz) * kE;
@@ -680,8 +683,9 @@ __device__ __forceinline__ void trace_ray_packet(const DeviceMap& map, const V& 
     h.t = tfar;
     return;
   }
-  const RayW rw = make_rayw(o, d);
-  const RayBox rb = make_raybox(o, d);
+  const V inv = reciprocal(d);
+  const RayW rw = make_rayw(o, d, inv);
+  const RayBox rb = make_raybox(o, d, inv);
   int stk_node[kFullStack];
   float stk_t[kFullStack];
   int sp = 0;
@@ -764,6 +768,23 @@ __device__ __forceinline__ void trace_ray(const DeviceMap& map, const V& o, cons
   }
 }
 
+// n / d for 32-bit n by a multiplication (Granlund and Montgomery, "Division by
+// Invariant Integers using Multiplication", PLDI 1994).
+struct FastDiv {
+  uint32_t mul, s1, s2;
+  __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
+    const uint32_t t = __umulhi(n, mul);
+    return (t + ((n - t) >> s1)) >> s2;
+  }
+};
+
+inline FastDiv fast_div(uint32_t d) {
+  uint32_t l = 0;
+  while ((1ull << l) < d) ++l;
+  const uint64_t m = ((((1ull << l) - d) << 32) / d) + 1;
+  return FastDiv{(uint32_t)m, l < 1 ? l : 1u, l > 0 ? l - 1 : 0u};
+}
+
 struct TraceParams {
   DeviceMap map;
   SensorDev sen;
@@ -776,6 +797,7 @@ struct TraceParams {
   uint32_t tiles_x;
   uint32_t tiles_per_pose;
   uint64_t n_tiles;
+  FastDiv by_tiles_per_pose, by_tiles_x;
   unsigned budget;
   int trail_bits;
   int full_stack;  // internal depth < kFullStack: the traversal may keep every pending child on a stack
@@ -824,10 +846,9 @@ __device__ __forceinline__ V hit_normal(const DeviceMap& map, const Hit& h, cons
 
 // Writes all requested attributes of one ray (SphereSimulatorEmbree.tcc:104-249).
 template <int OK>
-__device__ __forceinline__ void write_attributes(const TraceParams& P, uint64_t gid, const Hit& h,
-                                                 const V& dir_s, const V& orig_s, const Tf& Tsm) {
-  const rmg_outputs& out = P.out;
-  const float rmin = P.sen.range_min, rmax = P.sen.range_max;
+__device__ __forceinline__ void write_attributes(const DeviceMap& map, float rmin, float rmax, const rmg_outputs& out,
+                                                 uint64_t gid, const Hit& h, const V& dir_s, const V& orig_s,
+                                                 const Tf& Tsm) {
   if (h.tri >= 0) {
     const float t = h.t;
     if (out.hits) out.hits[gid] = t >= rmin ? 1 : 0;
@@ -838,7 +859,7 @@ __device__ __forceinline__ void write_attributes(const TraceParams& P, uint64_t 
       po[0] = p.x; po[1] = p.y; po[2] = p.z;
     }
     if (out.normals) {
-      const V n = hit_normal(P.map, h, dir_s, Tsm);
+      const V n = hit_normal(map, h, dir_s, Tsm);
       float* no = reinterpret_cast<float*>(out.normals) + 3 * gid;
       no[0] = n.x; no[1] = n.y; no[2] = n.z;
     }
@@ -880,26 +901,68 @@ __device__ __forceinline__ void setup_ray(const SensorDev& sen, const Tf& Tsm, u
   }
 }
 
+// Loads that the compiler does not merge with an earlier one of the same address.
+__device__ __forceinline__ V reread_v(const float* table, uint32_t loc) {
+  V v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v.x) : "l"(table + 3 * loc));
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v.y) : "l"(table + 3 * loc + 1));
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v.z) : "l"(table + 3 * loc + 2));
+  return v;
+}
+__device__ __forceinline__ Tf reread(const Tf* t) {
+  const volatile float* f = reinterpret_cast<const volatile float*>(t);
+  return Tf{Q{f[0], f[1], f[2], f[3]}, V{f[4], f[5], f[6]}};
+}
+
+// A ray's sensor-frame direction and origin again, after its walk.
+template <int OK>
+__device__ __forceinline__ void reread_ray(const SensorDev& sen, uint32_t loc, V& dir_s, V& orig_s) {
+  dir_s = reread_v(sen.dirs, loc);
+  orig_s = V{0.0f, 0.0f, 0.0f};
+  if (OK == ORIGIN_SINGLE) orig_s = V{sen.orig.x, sen.orig.y, sen.orig.z};
+  if (OK == ORIGIN_TABLE) orig_s = reread_v(sen.origs, loc);
+}
+
 // Registers of the traversal kernels, by walk.  The binary walk at 48 (40 warps
 // per SM, a few bytes of spills to L1-cached local memory) is 9% faster than
 // unconstrained at 62 (1M-triangle terrain, 5,661 -> 6,179 Mrays/s then), 40
 // registers lose again.  The 4-wide walk holds twice the planes per visit; on
-// the same terrain 48 / 56 / 64 / 72 registers take 3,778 / 3,297 / 3,351 /
-// 3,589 us, in the box room 362 / 322 / 324 / 338.  The 8-wide walk holds a
+// the same terrain 48 / 56 / 64 registers take 3,573 / 3,040 / 3,195 us, in the
+// box room 341 / 292 / 301.  The 8-wide walk holds a
 // node's twenty words and three axes of plane addends at once.
 template <int TB>
 constexpr int trace_regs() { return TB == kWide8TB ? 64 : (TB == kWideTB ? 56 : 48); }
 
-// One warp = one tile of tile_h x tile_w rays of one pose.
+// A warp's pose and its tile within the pose.
+__device__ __forceinline__ uint32_t tile_pose(const TraceParams& P, uint64_t tile, uint32_t& r) {
+  uint32_t pose;
+  if (P.n_tiles <= 0xffffffffull) {
+    pose = P.by_tiles_per_pose((uint32_t)tile);
+    r = (uint32_t)tile - pose * P.tiles_per_pose;
+  } else {
+    pose = (uint32_t)(tile / P.tiles_per_pose);
+    r = (uint32_t)(tile - (uint64_t)pose * P.tiles_per_pose);
+  }
+  return pose;
+}
+
+// One warp = one tile of tile_h x tile_w rays of one pose.  The CTA's poses are
+// composed by one lane each of its first warp (84 operations that every thread
+// repeated before) and shared.
 template <int OK, int SS, int TB>
-__global__ void __maxnreg__((trace_regs<TB>()))
-k_trace(const TraceParams P) {
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__global__ void __maxnreg__((trace_regs<TB>())) k_trace(const TraceParams P) {
+  __shared__ Tf s_tsm[8];
+  const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint64_t warp0 = (uint64_t)blockIdx.x * nw, warp = warp0 + wib;
+  if (threadIdx.x < nw && warp0 + threadIdx.x < P.n_tiles) {
+    uint32_t r;
+    s_tsm[threadIdx.x] = tmul(load_tf(P.Tbm[tile_pose(P, warp0 + threadIdx.x, r)]), P.Tsb);
+  }
+  __syncthreads();
   if (warp >= P.n_tiles) return;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t pose = (uint32_t)(warp / P.tiles_per_pose);
-  const uint32_t r = (uint32_t)(warp - (uint64_t)pose * P.tiles_per_pose);
-  const uint32_t ty = r / P.tiles_x, tx = r - ty * P.tiles_x;
+  uint32_t r;
+  const uint32_t pose = tile_pose(P, warp, r);
+  const uint32_t ty = P.by_tiles_x(r), tx = r - ty * P.tiles_x;
   const uint32_t tile_w = 1u << P.tile_w_log2;
   const uint32_t vid = ty * P.tile_h + (lane >> P.tile_w_log2);
   const uint32_t hid = tx * tile_w + (lane & (tile_w - 1));
@@ -907,21 +970,31 @@ k_trace(const TraceParams P) {
   const bool inside = vid < H && hid < W;
   if (TB != kPacketTB && !inside) return;  // the packet walk needs every lane
   const uint32_t loc = inside ? visit_loc(P.sen, vid * W + hid) : 0;
-  const uint64_t gid = (uint64_t)pose * W * H + loc;
 
-  const Tf Tsm = tmul(load_tf(P.Tbm[pose]), P.Tsb);
-  V dir_s, orig_s, o, d;
-  setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
   Hit h;
   bool over = false;
-  if constexpr (TB == kPacketTB) {
-    trace_ray_packet(P.map, o, d, P.sen.range_max, inside, P.budget, h, over);
-    if (!inside) return;
-  } else {
-    trace_ray<SS, TB>(P.map, o, d, P.sen.range_max, P.budget, h, over);
+  {
+    const Tf Tsm = s_tsm[wib];
+    V dir_s, orig_s, o, d;
+    setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
+    if constexpr (TB == kPacketTB) {
+      trace_ray_packet(P.map, o, d, P.sen.range_max, inside, P.budget, h, over);
+      if (!inside) return;
+    } else {
+      trace_ray<SS, TB>(P.map, o, d, P.sen.range_max, P.budget, h, over);
+    }
   }
   if (over) atomicExch(P.map.status, (unsigned)RMG_ERR_TRAVERSAL_BUDGET);
-  write_attributes<OK>(P, gid, h, dir_s, orig_s, Tsm);
+  // The attributes' inputs are read again instead of being kept through the walk:
+  // 10 to 13 registers that were spilled into its loop.  With the shared pose and
+  // the divisions by multiplication, us a pass: lidar on the 1M-triangle terrain
+  // 3,148 -> 3,040, camera on 2.1M 1,484 -> 1,418, box room 303 -> 292, scattered
+  // directions 186 -> 177.
+  const Tf Tsm = reread(s_tsm + wib);
+  V dir_s, orig_s;
+  reread_ray<OK>(P.sen, loc, dir_s, orig_s);
+  write_attributes<OK>(P.map, P.sen.range_min, P.sen.range_max, P.out, (uint64_t)pose * W * H + loc, h, dir_s, orig_s,
+                       Tsm);
 }
 
 }  // namespace rmg
@@ -993,7 +1066,7 @@ __global__ void __launch_bounds__(256) k_trace_refill(const TraceParams P, unsig
             setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
             active = true;
             if (!R.init(P.map, o, d, P.sen.range_max)) {  // empty map: finished at once
-              write_attributes<OK>(P, gid, R.h, dir_s, orig_s, Tsm);
+              write_attributes<OK>(P.map, P.sen.range_min, P.sen.range_max, P.out, gid, R.h, dir_s, orig_s, Tsm);
               active = false;
             }
           }
@@ -1014,7 +1087,7 @@ __global__ void __launch_bounds__(256) k_trace_refill(const TraceParams P, unsig
       const Tf Tsm = tmul(load_tf(P.Tbm[pose]), P.Tsb);
       V dir_s, orig_s, o, d;
       setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
-      write_attributes<OK>(P, gid, R.h, dir_s, orig_s, Tsm);
+      write_attributes<OK>(P.map, P.sen.range_min, P.sen.range_max, P.out, gid, R.h, dir_s, orig_s, Tsm);
       active = false;
     }
   }
