@@ -22,7 +22,7 @@
 //   small: k_small, one CTA per task, builds the whole subtree in shared
 //     memory: warps bin and partition tasks of more than 32 triangles, and
 //     finish those of up to 32 with one lane per triangle, where every lane
-//     evaluates the split after its own triangle's bin.
+//     evaluates the planes after its own triangle's centre (no bins).
 // A triangle travels as its box and id (32 B).  Every task writes its own box
 // into its parent's record when it is split, so no refit follows.
 //
@@ -44,7 +44,7 @@ namespace {
 constexpr int kNB = RMG_SAH_BINS;     // bins per axis
 static_assert(kNB >= 2 && kNB <= 16, "a half warp scans one axis");
 constexpr int kBins = 3 * kNB;
-constexpr int kBinWords = 7;          // count, box lo, box hi
+constexpr int kBinWords = 7;          // count, box lo, box hi; odd, so that bins lie in different banks
 constexpr uint32_t kMaxDepth = 32;    // leaves at most this many edges below the root
 constexpr uint32_t kChunk = 1024;     // positions of a large task handled by one CTA
 constexpr uint32_t kSmall = 512;      // largest task built in shared memory
@@ -144,19 +144,31 @@ __device__ __forceinline__ void write_links(Node* nodes, int node, int parent, u
   nodes[node].d = make_int4(l, r, parent, 0);
 }
 
-// Bins of one task in words [bin][count, lo, hi].  min / max first look at the
-// bin: after a few triangles most would not change it.
+// Adds a triangle to the bins of its three axes.  Minima and maxima first look
+// at the bins: after a few triangles most would not change them.  A single warp
+// (AHEAD) reads all eighteen words at once; where many warps share the bins a
+// look just before the update saves more updates (k_bin 197 against 228 us).
+template <bool AHEAD>
 __device__ __forceinline__ void bin_add(int* bins, const Rec& r, const float3& c, const float clo[3], const float chi[3]) {
   const int lo[3] = {f2o(r.a.x), f2o(r.a.y), f2o(r.a.z)}, hi[3] = {f2o(r.b.x), f2o(r.b.y), f2o(r.b.z)};
   const float cc[3] = {c.x, c.y, c.z};
+  int* B[3];
+  int now[3][6];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    int* B = bins + kBinWords * (a * kNB + bin_of(cc[a], clo[a], chi[a]));
-    atomicAdd(B, 1);
+    B[a] = bins + kBinWords * (a * kNB + bin_of(cc[a], clo[a], chi[a]));
+    if (AHEAD) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) now[a][k] = B[a][1 + k];
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    atomicAdd(B[a], 1);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      if (lo[k] < *(volatile int*)(B + 1 + k)) atomicMin(B + 1 + k, lo[k]);
-      if (hi[k] > *(volatile int*)(B + 4 + k)) atomicMax(B + 4 + k, hi[k]);
+      if (lo[k] < (AHEAD ? now[a][k] : *(volatile int*)(B[a] + 1 + k))) atomicMin(B[a] + 1 + k, lo[k]);
+      if (hi[k] > (AHEAD ? now[a][3 + k] : *(volatile int*)(B[a] + 4 + k))) atomicMax(B[a] + 4 + k, hi[k]);
     }
   }
 }
@@ -182,7 +194,7 @@ __device__ __forceinline__ Choice warp_split(const int* bins, uint32_t count, ui
   ch.bin = -1;
   ch.left = count / 2;
   float best = INFINITY;
-#pragma unroll 1
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
     uint32_t pc = 0, sc = 0;
     float pl[3] = {INFINITY, INFINITY, INFINITY}, ph[3] = {-INFINITY, -INFINITY, -INFINITY}, sl[3], sh[3];
@@ -310,7 +322,7 @@ __global__ void __launch_bounds__(kBlk) k_bin(Build* B, uint32_t par, const Task
     const uint32_t i = (threadIdx.x & 31) * (kChunk / 32) + k;
     if (i < len) {
       const Rec r = r0[i];
-      bin_add(sb, r, centre(r.a, r.b), clo, chi);
+      bin_add<false>(sb, r, centre(r.a, r.b), clo, chi);
     }
   }
   __syncthreads();
@@ -503,7 +515,7 @@ struct Sub {  // a task inside k_small's range
 struct SmallShared {
   Rec rec[kSmall];
   uint16_t perm[2][kSmall];
-  int bins[kSmallWarps][kBins * kBinWords];
+  __align__(16) int bins[kSmallWarps][kBins * kBinWords];
   Sub mid[2][kSmall / 33 + 1];  // tasks of more than 32 triangles, by level
   Sub tiny[kSmall / 2];
   uint32_t n_mid[2], n_tiny, task;
@@ -516,12 +528,12 @@ struct SmallOut {
 };
 
 // A task of up to 32 triangles, one lane each: all its subtasks, level by
-// level.  Every lane evaluates the three splits that put the bins up to its own
-// triangle's on the left -- other planes give the same sides as one of these --
-// by walking over its subtask's triangles; the least (cost, axis, bin) wins, as
-// in the scan over all planes.  The lanes' records live in `slot` (32 of them).
-__device__ void build_tiny(Rec* slot, uint16_t* perm, const Rec* rec, const Sub& t, uint32_t first, const SmallOut& out,
-                           uint32_t& max_depth) {
+// level.  No bins here: every lane evaluates, on each axis, the plane just after
+// its own box centre (centres up to it go left) by walking over its subtask's
+// triangles -- the full sweep over all planes -- and the least (cost, axis,
+// lane) wins.  The lanes' records live in `slot` (32 of them).
+__device__ void build_tiny(Rec* slot, const uint16_t* perm, const Rec* rec, const Sub& t, uint32_t first,
+                           const SmallOut& out, uint32_t& max_depth) {
   const uint32_t lane = threadIdx.x & 31, m = t.count;
   const bool live = lane < m;
   __syncwarp();
@@ -534,38 +546,26 @@ __device__ void build_tiny(Rec* slot, uint16_t* perm, const Rec* rec, const Sub&
     const bool on = e - s > 1;
     Rec me;
     float3 c;
-    float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    uint32_t mine = 0;
-    if (on) {
-      me = slot[lane];
-      for (uint32_t j = s; j < e; ++j) {
-        const float3 x = centre(slot[j].a, slot[j].b);
-        clo[0] = fminf(clo[0], x.x); clo[1] = fminf(clo[1], x.y); clo[2] = fminf(clo[2], x.z);
-        chi[0] = fmaxf(chi[0], x.x); chi[1] = fmaxf(chi[1], x.y); chi[2] = fmaxf(chi[2], x.z);
-      }
-      c = centre(me.a, me.b);
-      mine = (uint32_t)bin_of(c.x, clo[0], chi[0]) | (uint32_t)bin_of(c.y, clo[1], chi[1]) << 8 |
-             (uint32_t)bin_of(c.z, clo[2], chi[2]) << 16;
-    }
-    __syncwarp();
-    if (on) slot[lane].b.w = __uint_as_float(mine);
-    __syncwarp();
     float cost = INFINITY;
     uint32_t key = 0;
     float lo[3], hi[3];
     if (on) {
+      me = slot[lane];
+      c = centre(me.a, me.b);
       float ll[3][3], lh[3][3], rl[3][3], rh[3][3];
       uint32_t lc = 0;  // left counts, one byte per axis
 #pragma unroll
       for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int k = 0; k < 3; ++k) { ll[a][k] = rl[a][k] = INFINITY; lh[a][k] = rh[a][k] = -INFINITY; }
+#pragma unroll 2
       for (uint32_t j = s; j < e; ++j) {
         const float4 ja = slot[j].a, jb = slot[j].b;
-        const uint32_t jbins = __float_as_uint(jb.w);
+        const float3 jc = centre(ja, jb);
+        const bool left[3] = {jc.x <= c.x, jc.y <= c.y, jc.z <= c.z};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          if (((jbins >> (8 * a)) & 255u) <= ((mine >> (8 * a)) & 255u)) {
+          if (left[a]) {
             lc += 1u << (8 * a);
             ll[a][0] = fminf(ll[a][0], ja.x); ll[a][1] = fminf(ll[a][1], ja.y); ll[a][2] = fminf(ll[a][2], ja.z);
             lh[a][0] = fmaxf(lh[a][0], jb.x); lh[a][1] = fmaxf(lh[a][1], jb.y); lh[a][2] = fmaxf(lh[a][2], jb.z);
@@ -578,28 +578,35 @@ __device__ void build_tiny(Rec* slot, uint16_t* perm, const Rec* rec, const Sub&
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const uint32_t l = (lc >> (8 * a)) & 255u, r = e - s - l;
-        if (r == 0 || too_deep(depth, l, r)) continue;
+        if (l == 0 || r == 0 || too_deep(depth, l, r)) continue;
         const float x = half_area(ll[a], lh[a]) * (float)l + half_area(rl[a], rh[a]) * (float)r;
-        if (x < cost) { cost = x; key = (uint32_t)a << 8 | ((mine >> (8 * a)) & 255u); }
+        if (x < cost) { cost = x; key = (uint32_t)a << 8 | lane; }
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k) { lo[k] = fminf(ll[0][k], rl[0][k]); hi[k] = fmaxf(lh[0][k], rh[0][k]); }
     }
-    // least (cost, axis, bin) of the subtask (a.w and b.w hold the id and the bins:
-    // both are in registers)
+    // least (cost, axis, lane) of the subtask (the spare words of the slots carry
+    // them; the id stays in the lane's register)
     __syncwarp();
     if (on) { slot[lane].a.w = cost; slot[lane].b.w = __uint_as_float(key); }
     __syncwarp();
+    bool left = false;
     if (on) {
+#pragma unroll 4
       for (uint32_t j = s; j < e; ++j) {
         const float x = slot[j].a.w;
         const uint32_t k = __float_as_uint(slot[j].b.w);
         if (x < cost || (x == cost && k < key)) { cost = x; key = k; }
       }
+      if (!(cost < INFINITY)) {
+        left = lane - s < (e - s) / 2;  // halved by position
+      } else {
+        const Rec& w = slot[key & 255u];
+        const float3 wc = centre(w.a, w.b);
+        const uint32_t axis = key >> 8;
+        left = axis == 0 ? c.x <= wc.x : (axis == 1 ? c.y <= wc.y : c.z <= wc.z);
+      }
     }
-    const bool halved = !(cost < INFINITY);
-    const uint32_t axis = key >> 8;
-    const bool left = on && (halved ? lane - s < (e - s) / 2 : ((mine >> (8 * axis)) & 255u) <= (key & 255u));
     const unsigned bal = __ballot_sync(0xffffffffu, left);
     uint32_t p = lane, L = 0;
     if (on) {
@@ -683,7 +690,7 @@ __global__ void __launch_bounds__(kSmallBlk) k_small(Build* B, const Task* small
         __syncwarp();
         for (uint32_t i = lane; i < t.count; i += 32) {
           const Rec r = S.rec[perm[i]];
-          bin_add(bins, r, centre(r.a, r.b), clo, chi);
+          bin_add<true>(bins, r, centre(r.a, r.b), clo, chi);
         }
         __syncwarp();
         const Choice ch = warp_split(bins, t.count, depth);

@@ -19,6 +19,7 @@ namespace rmg {
 namespace {
 
 constexpr int kBlock4 = 256;
+constexpr int kMaxLevels4 = 192;  // a binary tree's depth at most (128 for the trail walks) and some more
 
 struct Cand {
   int id;        // binary child link: >= 0 internal node, < 0 leaf ~k
@@ -51,68 +52,125 @@ __host__ __device__ __forceinline__ void set_slot(Node4& w, int k, const float l
   lox[k] = lo[0]; hix[k] = hi[0]; loy[k] = lo[1]; hiy[k] = hi[1]; loz[k] = lo[2]; hiz[k] = hi[2];
 }
 
-// One level of the collapse: wide nodes [lo4, hi4), whose binary roots are
-// bin_of[j], get their children; internal children receive new wide indices.
-__global__ void k_collapse(const Node* __restrict__ bn, int* bin_of, uint32_t lo4, uint32_t hi4, Node4* w4,
-                           int* src4, unsigned int* count4) {
-  const uint32_t j = lo4 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= hi4) return;
-  const int b = bin_of[j];
-  const Node root = bn[b];
-  Cand c[4];
-  c[0] = cand_of(root, b, 0);
-  c[1] = cand_of(root, b, 1);
-  int n = 2;
-  if (root.d.x == root.d.y) n = 1;  // the one-triangle tree: both links name leaf 0
-  while (n < 4) {
-    int best = -1;
-    float ba = -1.f;
-    for (int k = 0; k < n; ++k) {
-      if (c[k].id >= 0) {
-        const float a = half_area(c[k]);
-        if (a > ba) { ba = a; best = k; }
+// The collapse's counters in device memory.
+struct WideBuild {
+  unsigned int count;            // wide nodes allocated
+  unsigned int levels;           // levels that held nodes
+  unsigned int end[kMaxLevels4 + 2];   // level l: nodes [end[l], end[l + 1])
+  unsigned int done[kMaxLevels4];      // CTAs of the level's launch that have finished
+};
+
+__device__ __forceinline__ void swap_cand(Cand& x, Cand& y, bool yes) {
+  if (!yes) return;
+  const Cand t = x;
+  x = y;
+  y = t;
+}
+
+// Level `level` of the collapse: its wide nodes, whose binary roots are
+// bin_of[j], get their children; internal children receive new wide indices, a
+// CTA's with one addition to the counter.  The last CTA to finish closes the
+// next level, so the launches follow one another without the host.  530,000
+// triangles, 13 levels: 188 us with all allocations made, where a host
+// synchronisation per level and an atomic per node took 330.
+__global__ void __launch_bounds__(kBlock4) k_collapse(const Node* __restrict__ bn, int* bin_of, WideBuild* B, int level,
+                                                      uint32_t cap, Node4* w4, int* src4) {
+  const uint32_t lo4 = B->end[level], hi4 = min(B->end[level + 1], cap);
+  if (lo4 >= hi4 && blockIdx.x != 0) return;
+  __shared__ uint32_t s_sum[kBlock4 / 32], s_base;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t j0 = lo4 + blockIdx.x * kBlock4; j0 < hi4; j0 += gridDim.x * kBlock4) {
+    const uint32_t j = j0 + threadIdx.x;
+    Cand c[4];
+    int n = 0, ni = 0;
+    if (j < hi4) {
+      const int b = bin_of[j];
+      const Node root = bn[b];
+      c[0] = cand_of(root, b, 0);
+      c[1] = cand_of(root, b, 1);
+      n = root.d.x == root.d.y ? 1 : 2;  // the one-triangle tree: both links name leaf 0
+#pragma unroll
+      for (int open = 0; open < 2; ++open) {  // the internal child of largest area gives way to its two
+        int best = -1;
+        float ba = -1.f;
+#pragma unroll
+        for (int k = 0; k < 2 + open; ++k) {
+          if (k < n && c[k].id >= 0) {
+            const float a = half_area(c[k]);
+            if (a > ba) { ba = a; best = k; }
+          }
+        }
+        if (best >= 0) {
+          int id = 0;
+#pragma unroll
+          for (int k = 0; k < 2 + open; ++k)
+            if (k == best) id = c[k].id;
+          const Node nb = bn[id];
+          const Cand l = cand_of(nb, id, 0);
+#pragma unroll
+          for (int k = 0; k < 2 + open; ++k)
+            if (k == best) c[k] = l;
+          // n == 2 + open here: the earlier opening succeeded too, or this is the first
+          c[2 + open] = cand_of(nb, id, 1);
+          ++n;
+        } else {
+          break;
+        }
       }
+      // internal children take the first slots and get consecutive wide indices, so
+      // a walk finds child `slot` at base + slot without reading the links
+#pragma unroll
+      for (int pass = 0; pass < 3; ++pass)
+#pragma unroll
+        for (int k = 0; k < 3 - pass; ++k) swap_cand(c[k], c[k + 1], k + 1 < n && c[k].id < 0 && c[k + 1].id >= 0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ni += k < n && c[k].id >= 0 ? 1 : 0;
     }
-    if (best < 0) break;
-    const int id = c[best].id;
-    const Node nb = bn[id];
-    c[best] = cand_of(nb, id, 0);
-    c[n++] = cand_of(nb, id, 1);
-  }
-  // internal children take the first slots and get consecutive wide indices, so
-  // a walk finds child `slot` at base + slot without reading the links
-  int ni = 0;
-  for (int k = 0; k < n; ++k) {
-    if (c[k].id >= 0) {
-      const Cand t = c[ni];
-      c[ni] = c[k];
-      c[k] = t;
-      ++ni;
+    uint32_t at = (uint32_t)ni;  // inclusive prefix over the CTA
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= (uint32_t)o) at += u;
     }
-  }
-  const int base = ni > 0 ? (int)atomicAdd(count4, (unsigned int)ni) : 0;
-  Node4 w;
-  const float far[3] = {1e30f, 1e30f, 1e30f};
-  int child[4];
-  for (int k = 0; k < 4; ++k) {
-    if (k < n) {
-      set_slot(w, k, c[k].lo, c[k].hi);
-      if (c[k].id < 0) {
-        child[k] = c[k].id;
+    if (lane == 31) s_sum[warp] = at;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (uint32_t w = 0; w < kBlock4 / 32; ++w) { if (w < warp) before += s_sum[w]; total += s_sum[w]; }
+    if (threadIdx.x == 0) s_base = total ? atomicAdd(&B->count, total) : 0;
+    __syncthreads();
+    const int base = ni > 0 ? (int)(s_base + before + at - (uint32_t)ni) : 0;
+    __syncthreads();
+    if (j >= hi4 || (uint32_t)(base + ni) > cap) continue;  // more nodes than the binary tree has: never
+    Node4 w;
+    const float far[3] = {1e30f, 1e30f, 1e30f};
+    int child[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k < n) {
+        set_slot(w, k, c[k].lo, c[k].hi);
+        if (c[k].id < 0) {
+          child[k] = c[k].id;
+        } else {
+          bin_of[base + k] = c[k].id;
+          child[k] = base + k;
+        }
       } else {
-        bin_of[base + k] = c[k].id;
-        child[k] = base + k;
+        set_slot(w, k, far, far);
+        child[k] = kEmpty4;
+        c[k].src = -1;
       }
-      src4[4 * j + k] = c[k].src;
-    } else {
-      set_slot(w, k, far, far);
-      child[k] = kEmpty4;
-      src4[4 * j + k] = -1;
     }
+    reinterpret_cast<int4*>(src4)[j] = make_int4(c[0].src, c[1].src, c[2].src, c[3].src);
+    w.child = make_int4(child[0], child[1], child[2], child[3]);
+    w.meta = make_int4(base, (((1 << n) - 1) ^ ((1 << ni) - 1)) | (((1 << ni) - 1) << 4), 0, 0);
+    w4[j] = w;
   }
-  w.child = make_int4(child[0], child[1], child[2], child[3]);
-  w.meta = make_int4(base, (((1 << n) - 1) ^ ((1 << ni) - 1)) | (((1 << ni) - 1) << 4), 0, 0);
-  w4[j] = w;
+  __threadfence();
+  __syncthreads();
+  const uint32_t ctas = lo4 >= hi4 ? 1u : gridDim.x;
+  if (threadIdx.x == 0 && atomicAdd(&B->done[level], 1u) == ctas - 1) {
+    B->end[level + 2] = atomicAdd(&B->count, 0u);
+    if (lo4 < hi4) B->levels = (unsigned int)level + 1u;
+  }
 }
 
 // Boxes of every slot from the (refitted) binary records.
@@ -141,40 +199,42 @@ void wide_free(rmg_map* m) {
   m->depth4 = 0;
 }
 
-// Builds the 4-wide tree of a map whose binary tree is complete.  Synchronises.
+// Builds the 4-wide tree of a map whose binary tree is complete (its depth
+// known).  Synchronises once.
 int wide_build(rmg_map* m, cudaStream_t st) {
   wide_free(m);
   if (m->n_faces == 0) return RMG_OK;
   const uint32_t cap = std::max<uint32_t>(m->n_nodes, 1u);
   int* bin_of = nullptr;
-  unsigned int* count4 = nullptr;
+  WideBuild* B = nullptr;
   int s = dev_alloc(&m->d_nodes4, cap, "wide nodes");
   if (s == RMG_OK) s = dev_alloc(&m->d_src4, 4 * (size_t)cap, "wide sources");
   if (s == RMG_OK) s = dev_alloc(&bin_of, cap, "wide roots");
-  if (s == RMG_OK) s = dev_alloc(&count4, 1, "wide counter");
-  const int zero = 0;
-  const unsigned int one = 1;
-  if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(bin_of, &zero, 4, cudaMemcpyHostToDevice, st), "wide init");
-  if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(count4, &one, 4, cudaMemcpyHostToDevice, st), "wide init");
-  uint32_t lo4 = 0, hi4 = 1, levels = 0;
-  while (s == RMG_OK && lo4 < hi4) {
-    const uint32_t n = hi4 - lo4;
-    k_collapse<<<(n + kBlock4 - 1) / kBlock4, kBlock4, 0, st>>>(m->d_nodes, bin_of, lo4, hi4, m->d_nodes4, m->d_src4,
-                                                                count4);
+  if (s == RMG_OK) s = dev_alloc(&B, 1, "wide counters");
+  WideBuild h{};
+  h.count = 1;
+  h.end[1] = 1;
+  if (s == RMG_OK) s = cuda_status(cudaMemsetAsync(bin_of, 0, 4, st), "wide init");
+  if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(B, &h, sizeof h, cudaMemcpyHostToDevice, st), "wide init");
+  // every wide level descends at least one binary level
+  const int levels = (int)std::min<unsigned>(std::max(m->depth, 1u), (unsigned)kMaxLevels4);
+  for (int l = 0; s == RMG_OK && l < levels; ++l) {
+    const uint64_t most = std::min<uint64_t>(cap, 1ull << std::min(2 * l, 62));
+    const unsigned grid = (unsigned)std::min<uint64_t>((most + kBlock4 - 1) / kBlock4, 4ull * device_sm_count());
+    k_collapse<<<grid, kBlock4, 0, st>>>(m->d_nodes, bin_of, B, l, cap, m->d_nodes4, m->d_src4);
     s = cuda_status(cudaGetLastError(), "k_collapse");
-    unsigned int c = 0;
-    if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&c, count4, 4, cudaMemcpyDeviceToHost, st), "wide count");
-    if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "wide sync");
-    ++levels;
-    lo4 = hi4;
-    hi4 = c;
-    if (hi4 > cap) s = fail(RMG_ERR_CUDA, "wide build: node count exceeds the binary tree");
   }
+  if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "wide count");
+  if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "wide sync");
+  if (s == RMG_OK && h.count > cap) s = fail(RMG_ERR_CUDA, "wide build: node count exceeds the binary tree");
   cudaFree(bin_of);
-  cudaFree(count4);
+  cudaFree(B);
   if (s != RMG_OK) { wide_free(m); return s; }
-  m->n_nodes4 = hi4;
-  m->depth4 = levels;
+  // a tree deeper than kMaxLevels4 keeps no 4-wide form (its walk takes at most
+  // 21 levels anyway, see have_wide4)
+  if (h.end[levels + 1] != h.end[levels]) { wide_free(m); return RMG_OK; }
+  m->n_nodes4 = h.count;
+  m->depth4 = h.levels;
   return RMG_OK;
 }
 
