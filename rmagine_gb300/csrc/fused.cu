@@ -274,17 +274,18 @@ extern "C" int rmg_simulate_statistics(const rmg_map* map, const rmg_sensor* sen
     if (grid > 0x7fffffffull) return fail(RMG_ERR_INVALID_ARG, "rmg_simulate_statistics: too many rays for one launch");
     cudaStream_t st = as_stream(stream);
     double* partial = nullptr;
-    RMG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&partial), 16 * sizeof(double) * (size_t)grid, st));
+    int s = pool_alloc(&partial, 16 * (size_t)grid, st, "fused partials");
+    if (s != RMG_OK) return s;
     F.partial = partial;
     const unsigned block = 32u * cfg.block_warps;
     const cudaError_t e = point_to_plane ? launch_fused<true>(F, sensor->model.kind, (unsigned)grid, block, st)
                                          : launch_fused<false>(F, sensor->model.kind, (unsigned)grid, block, st);
-    int s = cuda_status(e, "k_trace_stats");
+    s = cuda_status(e, "k_trace_stats");
     if (s == RMG_OK) {
       k_fused_final<<<n_poses, 32, 0, st>>>(partial, F.ctas_per_pose, stats, transforms);
       s = cuda_status(cudaGetLastError(), "k_fused_final");
     }
-    cudaFreeAsync(partial, st);
+    pool_free(partial, st);
     return s;
   });
 }

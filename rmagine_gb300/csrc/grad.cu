@@ -204,8 +204,8 @@ extern "C" int rmg_range_pose_grad(const rmg_map* map, const rmg_sensor* sensor,
     G.warps_per_pose = ctas_per_pose * cfg.block_warps;
     cudaStream_t st = as_stream(stream);
     float* partial = nullptr;
-    RMG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&partial),
-                                 8 * sizeof(float) * (size_t)n_poses * G.warps_per_pose, st));
+    int s = pool_alloc(&partial, 8 * (size_t)n_poses * G.warps_per_pose, st, "gradient partials");
+    if (s != RMG_OK) return s;
     G.partial = partial;
     const dim3 grid(ctas_per_pose, n_poses);
     const unsigned block = 32u * cfg.block_warps;
@@ -216,12 +216,12 @@ extern "C" int rmg_range_pose_grad(const rmg_map* map, const rmg_sensor* sensor,
       case RMG_MODEL_O1DN: e = launch_grad<ORIGIN_SINGLE>(G, (int)cfg.stack_depth, grid, block, st); break;
       default: e = launch_grad<ORIGIN_TABLE>(G, (int)cfg.stack_depth, grid, block, st); break;
     }
-    int s = cuda_status(e, "k_range_grad");
+    s = cuda_status(e, "k_range_grad");
     if (s == RMG_OK) {
       k_grad_final<<<n_poses, kFinalThreads, 0, st>>>(partial, n_poses, G.warps_per_pose, grad, loss);
       s = cuda_status(cudaGetLastError(), "k_grad_final");
     }
-    cudaFreeAsync(partial, st);
+    pool_free(partial, st);
     return s;
   });
 }

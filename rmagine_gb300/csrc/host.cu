@@ -790,6 +790,7 @@ extern "C" int rmg_host_staging_trim(void) {
     std::lock_guard<std::mutex> lock(g_pool_mu);
     for (int d = 0; d < kMaxDevices; ++d)
       if (g_pool[d]) RMG_CUDA_TRY(cudaMemPoolTrimTo(g_pool[d], 0));
+    pool_trim();
     return RMG_OK;
   });
 }

@@ -17,7 +17,8 @@ struct rmg_map {
   uint32_t n_nodes;
   uint32_t depth;
   float lo[3], hi[3];
-  // device arrays
+  // device arrays, all in one allocation from the pool
+  void* d_arena;
   float* d_vertices;          // 3*n_vertices
   uint32_t* d_faces;          // 3*n_faces
   rmg::Node* d_nodes;         // n_nodes
@@ -26,7 +27,7 @@ struct rmg_map {
   int* d_leaf_parent;         // n_faces: parent node of each leaf
   unsigned int* d_flags;      // n_nodes refit visit counters
   unsigned int* d_status;     // 1 word: device error status
-  // 4-wide tree collapsed from the binary one (wide.cu)
+  // 4-wide tree collapsed from the binary one (wide.cu), in one allocation that starts at d_nodes4
   rmg::Node4* d_nodes4;       // n_nodes4
   int* d_src4;                // 4*n_nodes4: binary record (2*parent + side) of each slot, -1 empty
   uint32_t n_nodes4;
@@ -75,6 +76,19 @@ int dev_alloc(T** p, size_t count, const char* what) {
                 std::string("cudaMalloc failed for ") + what);
   }
   return RMG_OK;
+}
+
+// Device memory from the library's stream-ordered pool of the current device
+// (runtime.cu): what a call or a map gives back is kept for the next one, up to
+// kPoolKeepBytes, instead of going through the driver.  pool_free takes NULL.
+int pool_alloc_bytes(void** p, size_t bytes, cudaStream_t st, const char* what);
+void pool_free(void* p, cudaStream_t st);
+void pool_trim();  // gives back what the pools of all devices hold unused
+
+template <typename T>
+int pool_alloc(T** p, size_t count, cudaStream_t st, const char* what) {
+  *p = nullptr;
+  return count == 0 ? RMG_OK : pool_alloc_bytes(reinterpret_cast<void**>(p), count * sizeof(T), st, what);
 }
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }

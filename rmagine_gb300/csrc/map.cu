@@ -20,6 +20,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -260,18 +261,57 @@ void single_node(const float* v, const uint32_t* f, Node* out) {
   out->d = make_int4(-1, -1, -1, 0);
 }
 
+std::atomic<long> g_live_maps{0};
+
+// A map's record, its device's arrays still to be allocated.
+rmg_map* new_map() {
+  rmg_map* m = new (std::nothrow) rmg_map;
+  if (!m) return nullptr;
+  std::memset(m, 0, sizeof(*m));
+  cudaGetDevice(&m->device);
+  g_live_maps.fetch_add(1);
+  return m;
+}
+
+// Waits for the device (work on any stream may use the map), as freeing its
+// arrays one by one did, and hands them back to the pool.
 void free_map(rmg_map* m) {
   if (!m) return;
-  cudaFree(m->d_vertices);
-  cudaFree(m->d_faces);
-  cudaFree(m->d_nodes);
-  cudaFree(m->d_tris);
-  cudaFree(m->d_leaf_order);
-  cudaFree(m->d_leaf_parent);
-  cudaFree(m->d_flags);
-  cudaFree(m->d_status);
+  int cur = m->device;
+  cudaGetDevice(&cur);
+  if (cur != m->device) cudaSetDevice(m->device);
+  cudaDeviceSynchronize();
   wide_free(m);
+  pool_free(m->d_arena, nullptr);
+  if (g_live_maps.fetch_sub(1) == 1) {
+    cudaStreamSynchronize(nullptr);
+    pool_trim();
+  }
+  if (cur != m->device) cudaSetDevice(cur);
   delete m;
+}
+
+// The arrays of a map of the given counts (cleared status word), on `st`.
+int alloc_arrays(rmg_map* m, cudaStream_t st) {
+  const size_t nv = m->n_vertices, nf = m->n_faces, nn = m->n_nodes;
+  size_t off = 0;
+  auto carve = [&](size_t bytes) { const size_t at = off; off = (off + bytes + 255) & ~size_t(255); return at; };
+  const size_t o_status = carve(sizeof(unsigned int)), o_vert = carve(12 * nv), o_face = carve(12 * nf),
+               o_node = carve(sizeof(Node) * nn), o_tri = carve(sizeof(Tri) * nf), o_order = carve(4 * nf),
+               o_parent = carve(4 * nf), o_flag = carve(4 * nn);
+  unsigned char* base = nullptr;
+  const int s = pool_alloc(&base, off, st, "map");
+  if (s != RMG_OK) return s;
+  m->d_arena = base;
+  m->d_status = reinterpret_cast<unsigned int*>(base + o_status);
+  m->d_vertices = reinterpret_cast<float*>(base + o_vert);
+  m->d_faces = reinterpret_cast<uint32_t*>(base + o_face);
+  m->d_nodes = reinterpret_cast<Node*>(base + o_node);
+  m->d_tris = reinterpret_cast<Tri*>(base + o_tri);
+  m->d_leaf_order = reinterpret_cast<uint32_t*>(base + o_order);
+  m->d_leaf_parent = reinterpret_cast<int*>(base + o_parent);
+  m->d_flags = reinterpret_cast<unsigned int*>(base + o_flag);
+  return cuda_status(cudaMemsetAsync(m->d_status, 0, sizeof(unsigned int), st), "memset");
 }
 
 // Packs the triangles and refits all boxes of an existing topology.
@@ -366,15 +406,17 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
     if (n_faces > 0 && (!vertices || !faces))
       return fail(RMG_ERR_INVALID_ARG, "rmg_map_build: vertices/faces are NULL");
     if (n_faces > (1u << 30)) return fail(RMG_ERR_INVALID_ARG, "rmg_map_build: too many faces");
-    for (uint32_t i = 0; i < n_faces; ++i) {
-      if (faces[i].v0 >= n_vertices || faces[i].v1 >= n_vertices || faces[i].v2 >= n_vertices)
-        return fail(RMG_ERR_INVALID_ARG, "rmg_map_build: face index out of range");
-    }
+    // the SAH build checks the face indices as it first reads them (a host loop
+    // over 530,000 faces took 376 us)
+    if (n_faces > 0 && n_vertices == 0) return fail(RMG_ERR_INVALID_ARG, "rmg_map_build: face index out of range");
+    if (builder == RMG_BUILD_LBVH || n_faces == 1)
+      for (uint32_t i = 0; i < n_faces; ++i) {
+        if (faces[i].v0 >= n_vertices || faces[i].v1 >= n_vertices || faces[i].v2 >= n_vertices)
+          return fail(RMG_ERR_INVALID_ARG, "rmg_map_build: face index out of range");
+      }
     cudaStream_t st = as_stream(stream);
-    rmg_map* m = new (std::nothrow) rmg_map;
+    rmg_map* m = new_map();
     if (!m) return fail(RMG_ERR_OOM, "rmg_map_build: host allocation");
-    std::memset(m, 0, sizeof(*m));
-    cudaGetDevice(&m->device);
     m->n_vertices = n_vertices;
     m->n_faces = n_faces;
     m->n_nodes = n_faces >= 2 ? n_faces - 1 : (n_faces == 1 ? 1 : 0);
@@ -382,8 +424,7 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
     int s = RMG_OK;
     auto check = [&](int r) { if (s == RMG_OK) s = r; return s == RMG_OK; };
   
-    check(dev_alloc(&m->d_status, 1, "status"));
-    if (s == RMG_OK) s = cuda_status(cudaMemsetAsync(m->d_status, 0, sizeof(unsigned int), st), "memset");
+    check(alloc_arrays(m, st));
     if (s == RMG_OK && n_faces == 0) {
       s = cuda_status(cudaStreamSynchronize(st), "sync");
       if (s != RMG_OK) { free_map(m); return s; }
@@ -391,13 +432,6 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
       *out = m;
       return RMG_OK;
     }
-    check(dev_alloc(&m->d_vertices, 3 * (size_t)n_vertices, "vertices"));
-    check(dev_alloc(&m->d_faces, 3 * (size_t)n_faces, "faces"));
-    check(dev_alloc(&m->d_nodes, m->n_nodes, "nodes"));
-    check(dev_alloc(&m->d_tris, n_faces, "tris"));
-    check(dev_alloc(&m->d_leaf_order, n_faces, "leaf order"));
-    check(dev_alloc(&m->d_leaf_parent, n_faces, "leaf parent"));
-    check(dev_alloc(&m->d_flags, m->n_nodes, "flags"));
     if (s != RMG_OK) { free_map(m); return s; }
     s = cuda_status(cudaMemcpyAsync(m->d_vertices, vertices, 12 * (size_t)n_vertices,
                                     cudaMemcpyHostToDevice, st), "copy vertices");
@@ -458,20 +492,20 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
     unsigned int* d_depth = nullptr;
     void* d_temp = nullptr;
     size_t temp_bytes = 0;
-    check(dev_alloc(&d_partial, 6 * (size_t)nb, "partial bounds"));
-    check(dev_alloc(&d_bounds, 6, "bounds"));
-    check(dev_alloc(&d_keys, n, "keys"));
-    check(dev_alloc(&d_keys2, n, "keys2"));
-    check(dev_alloc(&d_vals, n, "vals"));
-    check(dev_alloc(&d_vals2, n, "vals2"));
-    check(dev_alloc(&d_depth, 1, "depth"));
+    check(pool_alloc(&d_partial, 6 * (size_t)nb, st, "partial bounds"));
+    check(pool_alloc(&d_bounds, 6, st, "bounds"));
+    check(pool_alloc(&d_keys, n, st, "keys"));
+    check(pool_alloc(&d_keys2, n, st, "keys2"));
+    check(pool_alloc(&d_vals, n, st, "vals"));
+    check(pool_alloc(&d_vals2, n, st, "vals2"));
+    check(pool_alloc(&d_depth, 1, st, "depth"));
     if (s == RMG_OK) {
       s = cuda_status(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, d_keys, d_keys2, d_vals,
                                                        d_vals2, (int)n, 0, 63, st), "sort size");
     }
     if (s == RMG_OK) {
       char* tmp = nullptr;
-      s = dev_alloc(&tmp, temp_bytes, "sort temp");
+      s = pool_alloc(&tmp, temp_bytes, st, "sort temp");
       d_temp = tmp;
     }
     if (s == RMG_OK) {
@@ -499,8 +533,9 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
     unsigned int depth = 0;
     if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&depth, d_depth, 4, cudaMemcpyDeviceToHost, st), "depth copy");
     if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "sync");
-    cudaFree(d_partial); cudaFree(d_bounds); cudaFree(d_keys); cudaFree(d_keys2);
-    cudaFree(d_vals); cudaFree(d_vals2); cudaFree(d_depth); cudaFree(d_temp);
+    for (void* p : {(void*)d_partial, (void*)d_bounds, (void*)d_keys, (void*)d_keys2, (void*)d_vals, (void*)d_vals2,
+                    (void*)d_depth, d_temp})
+      pool_free(p, st);
     if (s != RMG_OK) { free_map(m); return s; }
     m->depth = depth;
     s = wide_build(m, st);
@@ -756,27 +791,17 @@ extern "C" int rmg_map_load(const char* path, void* stream, rmg_map** out) {
     int s = check_tree(h, faces.data(), nodes.data(), tris.data(), order.data(), parents.data(), &depth);
     if (s != RMG_OK) return s;
     cudaStream_t st = as_stream(stream);
-    rmg_map* m = new (std::nothrow) rmg_map;
+    rmg_map* m = new_map();
     if (!m) return fail(RMG_ERR_OOM, "rmg_map_load: host allocation");
-    std::memset(m, 0, sizeof(*m));
-    cudaGetDevice(&m->device);
     m->n_vertices = h.n_vertices;
     m->n_faces = h.n_faces;
     m->n_nodes = h.n_nodes;
     m->depth = depth;
     auto check = [&](int r) { if (s == RMG_OK) s = r; };
-    check(dev_alloc(&m->d_status, 1, "status"));
-    check(dev_alloc(&m->d_vertices, 3 * nv, "vertices"));
-    check(dev_alloc(&m->d_faces, 3 * nf, "faces"));
-    check(dev_alloc(&m->d_nodes, nn, "nodes"));
-    check(dev_alloc(&m->d_tris, nf, "tris"));
-    check(dev_alloc(&m->d_leaf_order, nf, "leaf order"));
-    check(dev_alloc(&m->d_leaf_parent, nf, "leaf parent"));
-    check(dev_alloc(&m->d_flags, nn, "flags"));
+    check(alloc_arrays(m, st));
     auto up = [&](void* dst, const void* src, size_t bytes) {
       if (s == RMG_OK && bytes) s = cuda_status(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st), "upload");
     };
-    if (s == RMG_OK) s = cuda_status(cudaMemsetAsync(m->d_status, 0, 4, st), "memset");
     up(m->d_vertices, pv, 12 * nv);
     up(m->d_faces, faces.data(), 12 * nf);
     up(m->d_nodes, nodes.data(), sizeof(Node) * nn);

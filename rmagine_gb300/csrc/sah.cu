@@ -82,6 +82,7 @@ struct Build {
   uint32_t next_small;   // k_small's work counter
   uint32_t depth;        // deepest leaf (edges)
   uint32_t bad;          // partition disagreed with the bins, or a list was full: never
+  uint32_t bad_face;     // a face names a vertex that is not there
   int root[6];           // bounds of all box centres
 };
 
@@ -252,13 +253,18 @@ __device__ __forceinline__ Choice warp_split(const int* bins, uint32_t count, ui
 // ---- large tasks ---------------------------------------------------------------------
 
 // Boxes and ids of all triangles; bounds of their box centres.
-__global__ void __launch_bounds__(kBlk) k_prep(const float* v, const uint32_t* f, uint32_t n, Rec* rec, Build* B) {
+__global__ void __launch_bounds__(kBlk) k_prep(const float* v, uint32_t n_vertices, const uint32_t* f, uint32_t n, Rec* rec,
+                                               Build* B) {
   __shared__ int sb[6];
   if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? kEmptyLo : kEmptyHi;
   __syncthreads();
   float cl[3] = {INFINITY, INFINITY, INFINITY}, chh[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (uint32_t i = blockIdx.x * kBlk + threadIdx.x; i < n; i += gridDim.x * kBlk) {
-    const float3 a = tri_v(v, f[3 * (size_t)i]), b = tri_v(v, f[3 * (size_t)i + 1]), d = tri_v(v, f[3 * (size_t)i + 2]);
+    uint32_t q[3] = {f[3 * (size_t)i], f[3 * (size_t)i + 1], f[3 * (size_t)i + 2]};
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (q[k] >= n_vertices) { B->bad_face = 1; q[k] = 0; }
+    const float3 a = tri_v(v, q[0]), b = tri_v(v, q[1]), d = tri_v(v, q[2]);
     Rec r;
     r.a = make_float4(fminf(fminf(a.x, b.x), d.x), fminf(fminf(a.y, b.y), d.y), fminf(fminf(a.z, b.z), d.z),
                       __uint_as_float(i));
@@ -769,7 +775,7 @@ inline unsigned blocks(size_t n, unsigned per) { return (unsigned)((n + per - 1)
 
 // A one-triangle-per-leaf SAH tree over the map's n >= 2 faces: links, parents
 // and boxes in m->d_nodes, m->d_leaf_parent, the face of every leaf in d_order,
-// m->depth.  Synchronises.
+// m->depth.  Face indices are checked here.  Synchronises.
 int sah_build(rmg_map* m, cudaStream_t st, uint32_t* d_order) {
   const uint32_t n = m->n_faces;
   if (n < 2) return fail(RMG_ERR_INVALID_ARG, "SAH build needs two or more faces");
@@ -789,7 +795,7 @@ int sah_build(rmg_map* m, cudaStream_t st, uint32_t* d_order) {
   const size_t o_small = carve(sizeof(Task) * max_small);
   const size_t o_build = carve(sizeof(Build));
   unsigned char* base = nullptr;
-  int s = dev_alloc(&base, off, "SAH build");
+  int s = pool_alloc(&base, off, st, "SAH build");
   if (s != RMG_OK) return s;
   Rec* rec[2] = {reinterpret_cast<Rec*>(base + o_rec0), reinterpret_cast<Rec*>(base + o_rec1)};
   Task* big[2] = {reinterpret_cast<Task*>(base + o_big0), reinterpret_cast<Task*>(base + o_big1)};
@@ -804,8 +810,8 @@ int sah_build(rmg_map* m, cudaStream_t st, uint32_t* d_order) {
   auto chk = [&](cudaError_t e, const char* what) { if (s == RMG_OK) s = cuda_status(e, what); };
   chk(cudaMemcpyAsync(B, &h, sizeof h, cudaMemcpyHostToDevice, st), "sah init");
   if (s == RMG_OK) {
-    k_prep<<<std::min(blocks(n, kBlk), 8u * (unsigned)device_sm_count()), kBlk, 0, st>>>(m->d_vertices, m->d_faces, n,
-                                                                                         rec[0], B);
+    k_prep<<<std::min(blocks(n, kBlk), 8u * (unsigned)device_sm_count()), kBlk, 0, st>>>(m->d_vertices, m->n_vertices,
+                                                                                         m->d_faces, n, rec[0], B);
     k_root<<<1, 1024, 0, st>>>(n, B, big[0], chunks[0], bins[0], small);
     chk(cudaGetLastError(), "sah prep");
   }
@@ -831,11 +837,11 @@ int sah_build(rmg_map* m, cudaStream_t st, uint32_t* d_order) {
     chk(cudaGetLastError(), "sah level");
     chk(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "sah counters");
     chk(cudaStreamSynchronize(st), "sah sync");
-    if (s != RMG_OK || h.bad || h.n_big[level & 1u] == 0) break;
+    if (s != RMG_OK || h.bad || h.bad_face || h.n_big[level & 1u] == 0) break;
     if (level > kMaxDepth) { s = fail(RMG_ERR_CUDA, "SAH build: too many levels"); break; }
     upto = level + 3;
   }
-  if (s == RMG_OK && !h.bad) {
+  if (s == RMG_OK && !h.bad && !h.bad_face) {
     const int smem = (int)sizeof(SmallShared);
     chk(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "k_small shared memory");
     int per_sm = 0;
@@ -849,9 +855,10 @@ int sah_build(rmg_map* m, cudaStream_t st, uint32_t* d_order) {
     chk(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "sah counters");
     chk(cudaStreamSynchronize(st), "sah sync");
   }
+  if (s == RMG_OK && h.bad_face) s = fail(RMG_ERR_INVALID_ARG, "rmg_map_build: face index out of range");
   if (s == RMG_OK && h.bad) s = fail(RMG_ERR_CUDA, "SAH build: partition disagrees with the split counts");
   m->depth = h.depth;
-  cudaFree(base);
+  pool_free(base, st);
   return s;
 }
 

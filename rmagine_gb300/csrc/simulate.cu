@@ -104,7 +104,8 @@ int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_tr
 
 int launch_refill(const TraceParams& P, const rmg_sensor* sensor, const rmg_launch_config& cfg, cudaStream_t st) {
   unsigned long long* counter = nullptr;
-  RMG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&counter), sizeof(unsigned long long), st));
+  const int a = pool_alloc(&counter, 1, st, "refill counter");
+  if (a != RMG_OK) return a;
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
   const unsigned block = 32u * cfg.block_warps;
   if (e == cudaSuccess) {
@@ -120,7 +121,7 @@ int launch_refill(const TraceParams& P, const rmg_sensor* sensor, const rmg_laun
     }
   }
   const int s = cuda_status(e, "trace refill launch");
-  cudaFreeAsync(counter, st);
+  pool_free(counter, st);
   return s;
 }
 

@@ -445,11 +445,12 @@ bool vec_ok(const StatsParams& P, bool p2l) {
 
 int launch_stats(StatsParams& P, bool p2l, cudaStream_t st) {
   const unsigned grid = P.n_batches * P.chunks;
-  void* scratch = nullptr;
+  unsigned char* scratch = nullptr;
   if (P.chunks > 1) {
     const size_t bytes = 16 * sizeof(double) * (size_t)grid + 4 * (size_t)P.n_batches;
-    RMG_CUDA_TRY(cudaMallocAsync(&scratch, bytes, st));
-    P.partial = static_cast<double*>(scratch);
+    const int a = pool_alloc(&scratch, bytes, st, "statistics partials");
+    if (a != RMG_OK) return a;
+    P.partial = reinterpret_cast<double*>(scratch);
     P.counters = reinterpret_cast<unsigned int*>(P.partial + 16ull * grid);
     RMG_CUDA_TRY(cudaMemsetAsync(P.counters, 0, 4 * (size_t)P.n_batches, st));
   }
@@ -466,7 +467,7 @@ int launch_stats(StatsParams& P, bool p2l, cudaStream_t st) {
     default: k_stats<true, true, true><<<grid, kStatsThreads, 0, st>>>(P); break;
   }
   const int s = cuda_status(cudaGetLastError(), "k_stats");
-  if (scratch) cudaFreeAsync(scratch, st);
+  pool_free(scratch, st);
   return s;
 }
 
@@ -484,7 +485,8 @@ int stats_entry(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
   P.stats = stats;
   double* dstats = nullptr;
   if (transforms) {
-    RMG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&dstats), 16 * sizeof(double) * (size_t)n_batches, st));
+    s = pool_alloc(&dstats, 16 * (size_t)n_batches, st, "statistics");
+    if (s != RMG_OK) return s;
     P.dstats = dstats;
   }
   s = launch_stats(P, p2l, st);
@@ -492,7 +494,7 @@ int stats_entry(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
     k_umeyama_dstats<<<(n_batches + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, st>>>(dstats, n_batches, transforms);
     s = cuda_status(cudaGetLastError(), "k_umeyama_dstats");
   }
-  if (dstats) cudaFreeAsync(dstats, st);
+  pool_free(dstats, st);
   return s;
 }
 
@@ -605,7 +607,8 @@ extern "C" int rmg_umeyama_backward(const rmg_transform* pre_transforms, uint32_
     if (s != RMG_OK) return s;
     cudaStream_t st = as_stream(stream);
     Coef* coef = nullptr;
-    RMG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&coef), sizeof(Coef) * (size_t)n_batches, st));
+    s = pool_alloc(&coef, n_batches, st, "backward coefficients");
+    if (s != RMG_OK) return s;
     k_umeyama_bwd_coef<<<(n_batches + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, st>>>(stats, grad_R, grad_t, n_batches, coef);
     s = cuda_status(cudaGetLastError(), "k_umeyama_bwd_coef");
     if (s == RMG_OK) {
@@ -615,7 +618,7 @@ extern "C" int rmg_umeyama_backward(const rmg_transform* pre_transforms, uint32_
       k_umeyama_bwd_stream<<<n_batches * B.S.chunks, kStatsThreads, 0, st>>>(B);
       s = cuda_status(cudaGetLastError(), "k_umeyama_bwd_stream");
     }
-    cudaFreeAsync(coef, st);
+    pool_free(coef, st);
     return s;
   });
 }

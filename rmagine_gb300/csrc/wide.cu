@@ -191,8 +191,7 @@ __global__ void k_wide_refit(const Node* __restrict__ bn, const int* __restrict_
 
 void wide_free(rmg_map* m) {
   wide8_free(m);
-  cudaFree(m->d_nodes4);
-  cudaFree(m->d_src4);
+  pool_free(m->d_nodes4, nullptr);  // the caller has waited for the device
   m->d_nodes4 = nullptr;
   m->d_src4 = nullptr;
   m->n_nodes4 = 0;
@@ -207,10 +206,15 @@ int wide_build(rmg_map* m, cudaStream_t st) {
   const uint32_t cap = std::max<uint32_t>(m->n_nodes, 1u);
   int* bin_of = nullptr;
   WideBuild* B = nullptr;
-  int s = dev_alloc(&m->d_nodes4, cap, "wide nodes");
-  if (s == RMG_OK) s = dev_alloc(&m->d_src4, 4 * (size_t)cap, "wide sources");
-  if (s == RMG_OK) s = dev_alloc(&bin_of, cap, "wide roots");
-  if (s == RMG_OK) s = dev_alloc(&B, 1, "wide counters");
+  // all nodes, then the four sources of each
+  unsigned char* base = nullptr;
+  int s = pool_alloc(&base, (sizeof(Node4) + 4 * sizeof(int)) * (size_t)cap, st, "wide nodes");
+  if (s == RMG_OK) {
+    m->d_nodes4 = reinterpret_cast<Node4*>(base);
+    m->d_src4 = reinterpret_cast<int*>(base + sizeof(Node4) * (size_t)cap);
+  }
+  if (s == RMG_OK) s = pool_alloc(&bin_of, cap, st, "wide roots");
+  if (s == RMG_OK) s = pool_alloc(&B, 1, st, "wide counters");
   WideBuild h{};
   h.count = 1;
   h.end[1] = 1;
@@ -227,9 +231,13 @@ int wide_build(rmg_map* m, cudaStream_t st) {
   if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "wide count");
   if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "wide sync");
   if (s == RMG_OK && h.count > cap) s = fail(RMG_ERR_CUDA, "wide build: node count exceeds the binary tree");
-  cudaFree(bin_of);
-  cudaFree(B);
-  if (s != RMG_OK) { wide_free(m); return s; }
+  pool_free(bin_of, st);
+  pool_free(B, st);
+  if (s != RMG_OK) {
+    cudaStreamSynchronize(st);
+    wide_free(m);
+    return s;
+  }
   // a tree deeper than kMaxLevels4 keeps no 4-wide form (its walk takes at most
   // 21 levels anyway, see have_wide4)
   if (h.end[levels + 1] != h.end[levels]) { wide_free(m); return RMG_OK; }
