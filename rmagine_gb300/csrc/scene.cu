@@ -30,11 +30,12 @@
 // after the first of the same geometry are dropped: their hits coincide with
 // the first's in range and face and lose the tie to its smaller index.
 //
-// Traversal (k_trace_scene): the top tree is walked with a full stack; at an
-// instance leaf the ray is taken into the instance's mesh frame,
+// Traversal (k_trace_scene): the top tree is walked with a full stack, the lanes
+// of a warp entering instances together (walk4_gather: 1,275 -> 1,239 us on the
+// terrain under 2,000 boxes); at an instance leaf the ray is taken into the instance's mesh frame,
 //     o_l = s^-1 (.) R^T (o - t),   d_l = s^-1 (.) R^T d   (R^T as conj(q) sandwich),
 // which keeps the ray parameter t, and the geometry's tree is walked by the
-// plain kernel's RayTrav from the leaf's start node with tfar = the best range
+// plain kernel's walk from the leaf's start node with tfar = the best range
 // so far.  A hit replaces the best when its range is smaller, or equal with a
 // smaller instance index, or equal in both with a smaller face index (two
 // pieces of one instance), so the result is the lexicographic minimum
@@ -63,6 +64,7 @@ struct InstDev {
 
 struct GeomDev {
   const Node* nodes;
+  const Node4* nodes4;  // NULL when some geometry's 4-wide tree cannot be walked
   const Tri* tris;
   int root;
   unsigned budget;
@@ -87,77 +89,59 @@ struct Best {
   uint32_t order; // instance index (tie-break)
 };
 
-__device__ __forceinline__ void instance_hit(const SceneParams& S, int k, const V& o, const V& d, Best& best,
-                                             bool& over) {
-  const uint2 leaf = __ldg(&S.leaves[__float_as_uint(__ldg(&S.T.map.tris[k].v0.w))]);
-  const uint32_t slot = leaf.x;
-  const InstDev* ip = S.inst + slot;
-  const float4 qi = __ldg(&ip->qinv), tt = __ldg(&ip->t), is = __ldg(&ip->inv_s);
-  const uint4 ids = __ldg(&ip->ids);
-  const Q qinv{qi.x, qi.y, qi.z, qi.w};
-  const V rl = qrot(qinv, V{sub(o.x, tt.x), sub(o.y, tt.y), sub(o.z, tt.z)});
-  const V ol{mul(rl.x, is.x), mul(rl.y, is.y), mul(rl.z, is.z)};
-  const V rd = qrot(qinv, d);
-  const V dl{mul(rd.x, is.x), mul(rd.y, is.y), mul(rd.z, is.z)};
-  const GeomDev* gp = S.geoms + ids.x;
-  DeviceMap bm;
-  bm.nodes = reinterpret_cast<const Node*>(__ldg(reinterpret_cast<const unsigned long long*>(&gp->nodes)));
-  bm.tris = reinterpret_cast<const Tri*>(__ldg(reinterpret_cast<const unsigned long long*>(&gp->tris)));
-  bm.root = (int)leaf.y;
-  bm.n_nodes = 0;
-  bm.n_tris = 0;
-  bm.status = S.T.map.status;
-  const unsigned budget = __ldg(&gp->budget);
-  RayTrav<kFullStack, 0> r;
-  ShortStack<kFullStack> stack;
-  if (!r.init(bm, ol, dl, best.t)) return;
-  while (!r.step(bm, budget, stack)) {
-  }
-  if (r.over) { over = true; return; }
-  if (r.h.tri < 0) return;
-  // r.h.t <= best.t here (the walk's tfar); at equal range the smaller instance,
-  // then the smaller face (another piece of the same instance) wins
-  if (r.h.t < best.t || best.inst < 0 || ids.w < best.order || (ids.w == best.order && r.h.face < best.face)) {
-    best.t = r.h.t;
-    best.tri = r.h.tri;
-    best.face = r.h.face;
-    best.inst = (int)slot;
-    best.order = ids.w;
-  }
+template <class T>
+__device__ __forceinline__ const T* load_ptr(const T* const* p) {
+  return reinterpret_cast<const T*>(__ldg(reinterpret_cast<const unsigned long long*>(p)));
 }
 
-// The geometry of an identity instance, walked in the map frame (its mesh frame
-// is the map frame); the same tie rule as instance_hit.
-__device__ __forceinline__ void direct_hit(const SceneParams& S, uint2 entry, const V& o, const V& d, Best& best,
-                                           bool& over) {
-  const GeomDev* gp = S.geoms + entry.x;
+// The closest hit of a mesh-frame ray in one geometry's tree from node `start`
+// (a 4-wide node when WIDE), entered as a hit of instance record `slot`.  At equal
+// range the smaller instance, then the smaller face (another piece of the same
+// instance) wins.
+template <bool WIDE>
+__device__ __forceinline__ void geometry_hit(const SceneParams& S, uint32_t geometry, int start, uint32_t slot,
+                                             uint32_t order, const V& o, const V& d, Best& best, bool& over) {
+  const GeomDev* gp = S.geoms + geometry;
   DeviceMap bm;
-  bm.nodes = reinterpret_cast<const Node*>(__ldg(reinterpret_cast<const unsigned long long*>(&gp->nodes)));
-  bm.tris = reinterpret_cast<const Tri*>(__ldg(reinterpret_cast<const unsigned long long*>(&gp->tris)));
-  bm.root = __ldg(&gp->root);
-  bm.n_nodes = 0;
-  bm.n_tris = 0;
+  bm.nodes = WIDE ? nullptr : load_ptr(&gp->nodes);
+  bm.nodes4 = WIDE ? load_ptr(&gp->nodes4) : nullptr;
+  bm.tris = load_ptr(&gp->tris);
+  bm.root = start;
   bm.status = S.T.map.status;
-  const unsigned budget = __ldg(&gp->budget);
-  RayTrav<kFullStack, 0> r;
-  ShortStack<kFullStack> stack;
-  if (!r.init(bm, o, d, best.t)) return;
-  while (!r.step(bm, budget, stack)) {
-  }
-  if (r.over) { over = true; return; }
-  if (r.h.tri < 0) return;
-  const uint32_t order = __ldg(&S.inst[entry.y].ids.w);
-  if (r.h.t < best.t || best.inst < 0 || order < best.order || (order == best.order && r.h.face < best.face)) {
-    best.t = r.h.t;
-    best.tri = r.h.tri;
-    best.face = r.h.face;
-    best.inst = (int)entry.y;
+  Hit h;
+  trace_ray<WIDE ? 0 : kFullStack, WIDE ? kWideTB : 0>(bm, o, d, best.t, __ldg(&gp->budget), h, over);
+  if (over || h.tri < 0) return;
+  // h.t <= best.t here (the walk's tfar)
+  if (h.t < best.t || best.inst < 0 || order < best.order || (order == best.order && h.face < best.face)) {
+    best.t = h.t;
+    best.tri = h.tri;
+    best.face = h.face;
+    best.inst = (int)slot;
     best.order = order;
   }
 }
 
-// Top-level walk with a full stack (depth <= 32 checked at creation; the guard
-// below only fires on a corrupt tree).
+// Leaf k of the top tree: an instance record and a start node in its geometry.
+template <bool WIDE>
+__device__ __forceinline__ void instance_hit(const SceneParams& S, int k, const V& o, const V& d, Best& best,
+                                             bool& over) {
+  const uint2 leaf = __ldg(&S.leaves[__float_as_uint(__ldg(&S.T.map.tris[k].v0.w))]);
+  const InstDev* ip = S.inst + leaf.x;
+  const float4 qi = __ldg(&ip->qinv), tt = __ldg(&ip->t), is = __ldg(&ip->inv_s);
+  const uint4 ids = __ldg(&ip->ids);
+  const Q qinv{qi.x, qi.y, qi.z, qi.w};
+  const V rl = qrot(qinv, V{sub(o.x, tt.x), sub(o.y, tt.y), sub(o.z, tt.z)});
+  const V rd = qrot(qinv, d);
+  geometry_hit<WIDE>(S, ids.x, (int)leaf.y, leaf.x, ids.w, V{mul(rl.x, is.x), mul(rl.y, is.y), mul(rl.z, is.z)},
+                     V{mul(rd.x, is.x), mul(rd.y, is.y), mul(rd.z, is.z)}, best, over);
+}
+
+// The directly walked geometries, then the top-level tree (its depth is checked
+// at creation; the stack guards below only fire on a corrupt tree).  WIDE and
+// TOP: the geometries' and the top tree's 4-wide trees are walked, the rule
+// wherever they can be (the scene's start nodes are then 4-wide ones); the binary
+// walks are left for trees of more than 21 wide levels.
+template <bool WIDE, bool TOP>
 __device__ __forceinline__ void trace_scene(const SceneParams& S, const V& o, const V& d, float tfar, Best& best,
                                             bool& over) {
   best.t = tfar;
@@ -165,61 +149,65 @@ __device__ __forceinline__ void trace_scene(const SceneParams& S, const V& o, co
   best.face = 0xffffffffu;
   best.inst = -1;
   best.order = 0xffffffffu;
-  for (uint32_t i = 0; i < S.n_direct && !over; ++i) direct_hit(S, S.direct[i], o, d, best, over);
+  // an identity instance's mesh frame is the map frame
+  for (uint32_t i = 0; i < S.n_direct && !over; ++i)
+    geometry_hit<WIDE>(S, S.direct[i].x, __ldg(&S.geoms[S.direct[i].x].root), S.direct[i].y,
+                       __ldg(&S.inst[S.direct[i].y].ids.w), o, d, best, over);
   const DeviceMap& tl = S.T.map;
-  if (tl.root < 0 || over) {
-    if (over) {
-      best.tri = -1;
-      best.t = tfar;
-      best.face = 0xffffffffu;
-      best.inst = -1;
+  if (tl.root >= 0 && !over) {
+    if constexpr (TOP) {
+      if (finite_ray(o, d)) {
+        const Ray4 r = make_ray4(make_raybox(o, d, reciprocal(d)));
+        walk4_gather(tl.nodes4, tl.root, r, best.t, S.T.budget, over,
+                     [&](int k) { instance_hit<WIDE>(S, k, o, d, best, over); });
+      }
+    } else {
+      const RayBox rb = make_raybox(o, d, reciprocal(d));
+      int stk_node[kFullStack];
+      float stk_t[kFullStack];
+      int sp = 0;
+      int node = tl.root;
+      unsigned steps = 0;
+      while (true) {
+        if (++steps > S.T.budget) { over = true; break; }
+        const Node* np = tl.nodes + node;
+        const float4 a = __ldg(&np->a), b = __ldg(&np->b), c = __ldg(&np->c);
+        const int4 ln = __ldg(&np->d);
+        float tminL, tmaxL, tminR, tmaxR;
+        slab(rb, a.x, a.y, a.z, a.w, c.x, c.y, tminL, tmaxL);
+        slab(rb, b.x, b.y, b.z, b.w, c.z, c.w, tminR, tmaxR);
+        bool hitL = visit(tminL, tmaxL, best.t);
+        bool hitR = visit(tminR, tmaxR, best.t);
+        const bool leafL = hitL && ln.x < 0, leafR = hitR && ln.y < 0;
+        if (leafL || leafR) {  // only an instance walk can move the closest hit: re-cull on this path
+          if (leafL) instance_hit<WIDE>(S, ~ln.x, o, d, best, over);
+          if (leafR) instance_hit<WIDE>(S, ~ln.y, o, d, best, over);
+          if (over) break;
+          hitL = hitL && !leafL && tminL <= best.t * kWiden;
+          hitR = hitR && !leafR && tminR <= best.t * kWiden;
+        }
+        if (hitL && hitR) {
+          if (sp >= kFullStack) { over = true; break; }
+          const bool lf = tminL <= tminR;
+          stk_node[sp] = lf ? ln.y : ln.x;
+          stk_t[sp] = lf ? tminR : tminL;
+          ++sp;
+          node = lf ? ln.x : ln.y;
+          continue;
+        }
+        if (hitL || hitR) {
+          node = hitL ? ln.x : ln.y;
+          continue;
+        }
+        bool found = false;
+        while (sp > 0) {
+          --sp;
+          node = stk_node[sp];
+          if (stk_t[sp] <= best.t * kWiden) { found = true; break; }
+        }
+        if (!found) break;
+      }
     }
-    return;
-  }
-  const RayBox rb = make_raybox(o, d, reciprocal(d));
-  int stk_node[kFullStack];
-  float stk_t[kFullStack];
-  int sp = 0;
-  int node = tl.root;
-  unsigned steps = 0;
-  while (true) {
-    if (++steps > S.T.budget) { over = true; break; }
-    const Node* np = tl.nodes + node;
-    const float4 a = __ldg(&np->a), b = __ldg(&np->b), c = __ldg(&np->c);
-    const int4 ln = __ldg(&np->d);
-    float tminL, tmaxL, tminR, tmaxR;
-    slab(rb, a.x, a.y, a.z, a.w, c.x, c.y, tminL, tmaxL);
-    slab(rb, b.x, b.y, b.z, b.w, c.z, c.w, tminR, tmaxR);
-    bool hitL = visit(tminL, tmaxL, best.t);
-    bool hitR = visit(tminR, tmaxR, best.t);
-    const bool leafL = hitL && ln.x < 0, leafR = hitR && ln.y < 0;
-    if (leafL || leafR) {  // only an instance walk can move the closest hit: re-cull on this path
-      if (leafL) instance_hit(S, ~ln.x, o, d, best, over);
-      if (leafR) instance_hit(S, ~ln.y, o, d, best, over);
-      if (over) break;
-      hitL = hitL && !leafL && tminL <= best.t * kWiden;
-      hitR = hitR && !leafR && tminR <= best.t * kWiden;
-    }
-    if (hitL && hitR) {
-      if (sp >= kFullStack) { over = true; break; }
-      const bool lf = tminL <= tminR;
-      stk_node[sp] = lf ? ln.y : ln.x;
-      stk_t[sp] = lf ? tminR : tminL;
-      ++sp;
-      node = lf ? ln.x : ln.y;
-      continue;
-    }
-    if (hitL || hitR) {
-      node = hitL ? ln.x : ln.y;
-      continue;
-    }
-    bool found = false;
-    while (sp > 0) {
-      --sp;
-      node = stk_node[sp];
-      if (stk_t[sp] <= best.t * kWiden) { found = true; break; }
-    }
-    if (!found) break;
   }
   if (over) {
     best.tri = -1;
@@ -229,34 +217,43 @@ __device__ __forceinline__ void trace_scene(const SceneParams& S, const V& o, co
   }
 }
 
-#ifndef RMG_SCENE_MIN_BLOCKS
-#define RMG_SCENE_MIN_BLOCKS 4
-#endif
-
-template <int OK>
-__global__ void __launch_bounds__(256, RMG_SCENE_MIN_BLOCKS) k_trace_scene(const SceneParams S) {
+// 64 registers: the instance walk nested in the top-level one keeps both levels'
+// state (1M-triangle terrain under 2,000 boxes: 1,336 / 1,239 / 1,260 us with 56 /
+// 64 / 72, 1,344 with the binary walks on both levels).
+template <int OK, bool WIDE, bool TOP>
+__global__ void __maxnreg__(64) k_trace_scene(const SceneParams S) {
   const TraceParams& P = S.T;
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  __shared__ Tf s_tsm[8];
+  const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint64_t warp0 = (uint64_t)blockIdx.x * nw, warp = warp0 + wib;
+  if (threadIdx.x < nw && warp0 + threadIdx.x < P.n_tiles) {
+    uint32_t r;
+    s_tsm[threadIdx.x] = tmul(load_tf(P.Tbm[tile_pose(P, warp0 + threadIdx.x, r)]), P.Tsb);
+  }
+  __syncthreads();
   if (warp >= P.n_tiles) return;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t pose = (uint32_t)(warp / P.tiles_per_pose);
-  const uint32_t r = (uint32_t)(warp - (uint64_t)pose * P.tiles_per_pose);
-  const uint32_t ty = r / P.tiles_x, tx = r - ty * P.tiles_x;
+  uint32_t r;
+  const uint32_t pose = tile_pose(P, warp, r);
+  const uint32_t ty = P.by_tiles_x(r), tx = r - ty * P.tiles_x;
   const uint32_t tile_w = 1u << P.tile_w_log2;
   const uint32_t vid = ty * P.tile_h + (lane >> P.tile_w_log2);
   const uint32_t hid = tx * tile_w + (lane & (tile_w - 1));
   const uint32_t W = P.sen.width, H = P.sen.height;
   if (vid >= H || hid >= W) return;
   const uint32_t loc = visit_loc(P.sen, vid * W + hid);
-  const uint64_t gid = (uint64_t)pose * W * H + loc;
 
-  const Tf Tsm = tmul(load_tf(P.Tbm[pose]), P.Tsb);
-  V dir_s, orig_s, o, d;
-  setup_ray<OK>(P.sen, Tsm, loc, dir_s, orig_s, o, d);
   Best best;
   bool over = false;
-  trace_scene(S, o, d, P.sen.range_max, best, over);
+  {
+    V dir_s, orig_s, o, d;
+    setup_ray<OK>(P.sen, reread(s_tsm + wib), loc, dir_s, orig_s, o, d);
+    trace_scene<WIDE, TOP>(S, o, d, P.sen.range_max, best, over);
+  }
   if (over) atomicExch(P.map.status, (unsigned)RMG_ERR_TRAVERSAL_BUDGET);
+  const uint64_t gid = (uint64_t)pose * W * H + loc;
+  const Tf Tsm = reread(s_tsm + wib);
+  V dir_s, orig_s;
+  reread_ray<OK>(P.sen, loc, dir_s, orig_s);
 
   const rmg_outputs& out = P.out;
   if (best.tri >= 0) {
@@ -304,9 +301,18 @@ __global__ void __launch_bounds__(256, RMG_SCENE_MIN_BLOCKS) k_trace_scene(const
   }
 }
 
-// Request of k_piece_boxes: the box of one piece, read from its parent node.
+template <int OK>
+void launch_scene(const SceneParams& S, bool wide, bool wide_top, unsigned grid, unsigned block, cudaStream_t st) {
+  if (wide && wide_top) k_trace_scene<OK, true, true><<<grid, block, 0, st>>>(S);
+  else if (wide) k_trace_scene<OK, true, false><<<grid, block, 0, st>>>(S);
+  else k_trace_scene<OK, false, false><<<grid, block, 0, st>>>(S);
+}
+
+// Request of k_piece_boxes: the box of one piece, read from its parent node (a
+// 4-wide one when nodes4 is set).
 struct PieceReq {
   const Node* nodes;
+  const Node4* nodes4;
   int parent, side;
 };
 
@@ -315,9 +321,15 @@ __global__ void k_piece_boxes(const PieceReq* req, uint32_t n, float* out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const PieceReq q = req[i];
+  float* o = out + 6 * (size_t)i;
+  if (q.nodes4) {
+    const Node4* p = q.nodes4 + q.parent;
+    o[0] = (&p->lox.x)[q.side]; o[1] = (&p->loy.x)[q.side]; o[2] = (&p->loz.x)[q.side];
+    o[3] = (&p->hix.x)[q.side]; o[4] = (&p->hiy.x)[q.side]; o[5] = (&p->hiz.x)[q.side];
+    return;
+  }
   const Node* p = q.nodes + q.parent;
   const float4 a = p->a, b = p->b, c = p->c;
-  float* o = out + 6 * (size_t)i;
   if (q.side == 0) {
     o[0] = a.x; o[1] = a.z; o[2] = c.x; o[3] = a.y; o[4] = a.w; o[5] = c.y;
   } else {
@@ -338,7 +350,7 @@ DeviceMap device_view(const rmg_map* m);
 using namespace rmg;
 
 // A piece of an opened geometry tree: subtree root `node`, the box of which
-// sits in child slot `side` of node `parent`.
+// sits in child slot `side` of node `parent` (binary or 4-wide nodes).
 struct ScenePiece {
   int node, parent, side;
 };
@@ -346,6 +358,7 @@ struct ScenePiece {
 struct rmg_scene {
   int device = 0;
   std::vector<const rmg_map*> geoms;
+  bool wide = false;            // every geometry has a 4-wide tree to walk: pieces and start nodes are 4-wide ones
   std::vector<std::vector<ScenePiece>> pieces;  // per geometry; empty = not opened
   std::vector<uint32_t> piece_base;             // per geometry: first request in d_piece_req
   uint32_t n_pieces = 0;
@@ -393,7 +406,7 @@ double box_area(const float lo[3], const float hi[3]) {
 // triangles into about n_faces / RMG_SCENE_PIECE_TRIS pieces (at most
 // kMaxPieces): the piece with the largest box surface is replaced by its two
 // children until there are enough, or until every piece has a leaf child.
-int open_geometry(const rmg_map* g, cudaStream_t st, std::vector<ScenePiece>& out) {
+int open_geometry(const rmg_map* g, bool wide, cudaStream_t st, std::vector<ScenePiece>& out) {
   out.clear();
   const uint32_t per = RMG_SCENE_PIECE_TRIS;
   if (per == 0 || g->n_faces < 2u * per) return RMG_OK;
@@ -412,6 +425,23 @@ int open_geometry(const rmg_map* g, cudaStream_t st, std::vector<ScenePiece>& ou
     for (size_t i = 0; i < c.size(); ++i)
       if (!c[i].closed && box_area(c[i].lo, c[i].hi) > area) { area = box_area(c[i].lo, c[i].hi); pick = (int)i; }
     if (pick < 0) break;
+    if (wide) {
+      Node4 nd;
+      RMG_CUDA_TRY(cudaMemcpyAsync(&nd, g->d_nodes4 + c[pick].p.node, sizeof nd, cudaMemcpyDeviceToHost, st));
+      RMG_CUDA_TRY(cudaStreamSynchronize(st));
+      const int* link = &nd.child.x;
+      bool leaf = false;
+      for (int k = 0; k < 4; ++k) leaf = leaf || (link[k] < 0 && link[k] != kEmpty4);
+      if (leaf) { c[pick].closed = true; continue; }
+      const int parent = c[pick].p.node;
+      c.erase(c.begin() + pick);
+      for (int k = 0; k < 4; ++k)
+        if (link[k] != kEmpty4)
+          c.push_back(Cand{ScenePiece{link[k], parent, k},
+                           {(&nd.lox.x)[k], (&nd.loy.x)[k], (&nd.loz.x)[k]},
+                           {(&nd.hix.x)[k], (&nd.hiy.x)[k], (&nd.hiz.x)[k]}, false});
+      continue;
+    }
     Node nd;
     RMG_CUDA_TRY(cudaMemcpyAsync(&nd, g->d_nodes + c[pick].p.node, sizeof nd, cudaMemcpyDeviceToHost, st));
     RMG_CUDA_TRY(cudaStreamSynchronize(st));
@@ -624,6 +654,8 @@ extern "C" int rmg_scene_create(const rmg_map* const* geometries, uint32_t n_geo
       }
       s->geoms.push_back(geometries[g]);
     }
+    s->wide = true;
+    for (const rmg_map* g : s->geoms) s->wide = s->wide && (g->n_faces == 0 || have_wide4(g));
     int r = check_instances(s, instances, n_instances);
     if (r != RMG_OK) { delete s; return r; }
     cudaStream_t st = as_stream(stream);
@@ -633,7 +665,7 @@ extern "C" int rmg_scene_create(const rmg_map* const* geometries, uint32_t n_geo
       std::vector<GeomDev> g(n_geometries);
       for (uint32_t i = 0; i < n_geometries; ++i) {
         const DeviceMap dm = device_view(geometries[i]);
-        g[i] = GeomDev{dm.nodes, dm.tris, dm.root, 2u * geometries[i]->n_nodes + 64u};
+        g[i] = GeomDev{dm.nodes, dm.nodes4, dm.tris, dm.root, 2u * geometries[i]->n_nodes + 64u};
       }
       r = dev_alloc(&s->d_geoms, n_geometries, "scene geometries");
       if (r == RMG_OK)
@@ -648,9 +680,9 @@ extern "C" int rmg_scene_create(const rmg_map* const* geometries, uint32_t n_geo
     std::vector<PieceReq> req;
     for (uint32_t gi = 0; r == RMG_OK && gi < n_geometries; ++gi) {
       if (!used[gi]) continue;
-      r = open_geometry(geometries[gi], st, s->pieces[gi]);
+      r = open_geometry(geometries[gi], s->wide, st, s->pieces[gi]);
       s->piece_base[gi] = (uint32_t)req.size();
-      for (const ScenePiece& p : s->pieces[gi]) req.push_back(PieceReq{geometries[gi]->d_nodes, p.parent, p.side});
+      for (const ScenePiece& p : s->pieces[gi]) req.push_back(PieceReq{geometries[gi]->d_nodes, s->wide ? geometries[gi]->d_nodes4 : nullptr, p.parent, p.side});
     }
     // Bound the top tree: with more than 2^22 leaves from opened trees, open none.
     uint64_t n_leaves = 0;
@@ -735,11 +767,12 @@ extern "C" int rmg_simulate_scene(const rmg_scene* s, const rmg_sensor* sensor, 
     if (blocks > 0x7fffffffull) return fail(RMG_ERR_INVALID_ARG, "rmg_simulate_scene: too many rays for one launch");
     const unsigned block = 32u * cfg.block_warps;
     cudaStream_t st = as_stream(stream);
+    const bool top4 = !s->tlas || have_wide4(s->tlas);
     switch (sensor->model.kind) {
       case RMG_MODEL_SPHERICAL:
-      case RMG_MODEL_PINHOLE: k_trace_scene<ORIGIN_POSE><<<(unsigned)blocks, block, 0, st>>>(S); break;
-      case RMG_MODEL_O1DN: k_trace_scene<ORIGIN_SINGLE><<<(unsigned)blocks, block, 0, st>>>(S); break;
-      default: k_trace_scene<ORIGIN_TABLE><<<(unsigned)blocks, block, 0, st>>>(S); break;
+      case RMG_MODEL_PINHOLE: launch_scene<ORIGIN_POSE>(S, s->wide, top4, (unsigned)blocks, block, st); break;
+      case RMG_MODEL_O1DN: launch_scene<ORIGIN_SINGLE>(S, s->wide, top4, (unsigned)blocks, block, st); break;
+      default: launch_scene<ORIGIN_TABLE>(S, s->wide, top4, (unsigned)blocks, block, st); break;
     }
     return cuda_status(cudaGetLastError(), "k_trace_scene");
   });

@@ -362,6 +362,189 @@ __device__ __forceinline__ void plane2(unsigned long long p, unsigned long long 
   asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(r));
 }
 
+// The 4-wide walk's view of a ray: 1/d and the near and far planes' addends,
+// each twice for two children at a time, and the byte offsets of the near planes
+// in a node (the far planes are at ^ 16).
+struct Ray4 {
+  unsigned long long pix, piy, piz, cnx, cfx, cny, cfy, cnz, cfz;
+  uint32_t ox, oy, oz;
+};
+
+__device__ __forceinline__ Ray4 make_ray4(const RayBox& rb) {
+  const bool bx = rb.ix < 0.f, by = rb.iy < 0.f, bz = rb.iz < 0.f;
+  const float nxa = bx ? rb.chx : rb.clx, fxa = bx ? rb.clx : rb.chx;
+  const float nya = by ? rb.chy : rb.cly, fya = by ? rb.cly : rb.chy;
+  const float nza = bz ? rb.chz : rb.clz, fza = bz ? rb.clz : rb.chz;
+  return Ray4{pack2(rb.ix, rb.ix), pack2(rb.iy, rb.iy), pack2(rb.iz, rb.iz), pack2(nxa, nxa), pack2(fxa, fxa),
+              pack2(nya, nya),     pack2(fya, fya),     pack2(nza, nza),     pack2(fza, fza),
+              bx ? 16u : 0u,       by ? 48u : 32u,      bz ? 80u : 64u};
+}
+
+// A ray with a NaN or infinite component hits no triangle (its edge functions or
+// its quotient are NaN), but a box test with NaN planes admits everything.
+__device__ __forceinline__ bool finite_ray(const V& o, const V& d) {
+  float z = o.x * 0.0f;
+  z = fmaf(o.y, 0.0f, z); z = fmaf(o.z, 0.0f, z);
+  z = fmaf(d.x, 0.0f, z); z = fmaf(d.y, 0.0f, z); z = fmaf(d.z, 0.0f, z);
+  return z == 0.0f;
+}
+
+// One 4-wide node: entry distances t[] and the slots that the ray enters before
+// `best`, as bits 0-3 (leaves) and 4-7 (internal children, nodes base + slot).
+__device__ __forceinline__ uint32_t visit4(const char* np, const Ray4& r, float best, float t[4], int& base) {
+  const ulonglong2 qnx = __ldg(reinterpret_cast<const ulonglong2*>(np + r.ox));
+  const ulonglong2 qfx = __ldg(reinterpret_cast<const ulonglong2*>(np + (r.ox ^ 16u)));
+  const ulonglong2 qny = __ldg(reinterpret_cast<const ulonglong2*>(np + r.oy));
+  const ulonglong2 qfy = __ldg(reinterpret_cast<const ulonglong2*>(np + (r.oy ^ 16u)));
+  const ulonglong2 qnz = __ldg(reinterpret_cast<const ulonglong2*>(np + r.oz));
+  const ulonglong2 qfz = __ldg(reinterpret_cast<const ulonglong2*>(np + (r.oz ^ 16u)));
+  const int2 meta = __ldg(reinterpret_cast<const int2*>(np + 112));
+  float m[4];
+  float x0, x1, y0, y1, z0, z1;
+  plane2(qnx.x, r.pix, r.cnx, x0, x1); plane2(qny.x, r.piy, r.cny, y0, y1); plane2(qnz.x, r.piz, r.cnz, z0, z1);
+  t[0] = fmax3f(x0, y0, fmaxf(z0, 0.0f));
+  t[1] = fmax3f(x1, y1, fmaxf(z1, 0.0f));
+  plane2(qnx.y, r.pix, r.cnx, x0, x1); plane2(qny.y, r.piy, r.cny, y0, y1); plane2(qnz.y, r.piz, r.cnz, z0, z1);
+  t[2] = fmax3f(x0, y0, fmaxf(z0, 0.0f));
+  t[3] = fmax3f(x1, y1, fmaxf(z1, 0.0f));
+  plane2(qfx.x, r.pix, r.cfx, x0, x1); plane2(qfy.x, r.piy, r.cfy, y0, y1); plane2(qfz.x, r.piz, r.cfz, z0, z1);
+  m[0] = fmin3f(x0, y0, fminf(z0, best));
+  m[1] = fmin3f(x1, y1, fminf(z1, best));
+  plane2(qfx.y, r.pix, r.cfx, x0, x1); plane2(qfy.y, r.piy, r.cfy, y0, y1); plane2(qfz.y, r.piz, r.cfz, z0, z1);
+  m[2] = fmin3f(x0, y0, fminf(z0, best));
+  m[3] = fmin3f(x1, y1, fminf(z1, best));
+  uint32_t hit = 0;
+  if (t[0] <= m[0] * kWiden) hit |= 0x11u;
+  if (t[1] <= m[1] * kWiden) hit |= 0x22u;
+  if (t[2] <= m[2] * kWiden) hit |= 0x44u;
+  if (t[3] <= m[3] * kWiden) hit |= 0x88u;
+  base = meta.x;
+  return hit & (uint32_t)meta.y;
+}
+
+// The pending nodes of a 4-wide walk are (entry distance with the slot in its
+// last two bits, node) pairs.  (The array and its count are apart: in one struct
+// the count went to local memory with the array, 3 to 9% of the walk.)
+//
+// Of the internal children `im` (two or more): the nearest's slot, the others
+// pushed.  Distance and slot in one word are ordered as the distances (>= 0)
+// are, rounded down to 4 ulp, which keeps the later culls conservative.
+__device__ __forceinline__ uint32_t push4(uint2 (&e)[kStack4], int& n, uint32_t im, const float t[4], int base) {
+  const uint32_t k0 = im & 1u ? (__float_as_uint(t[0]) & ~3u) : 0xffffffffu;
+  const uint32_t k1 = im & 2u ? (__float_as_uint(t[1]) & ~3u) | 1u : 0xffffffffu;
+  const uint32_t k2 = im & 4u ? (__float_as_uint(t[2]) & ~3u) | 2u : 0xffffffffu;
+  const uint32_t k3 = im & 8u ? (__float_as_uint(t[3]) & ~3u) | 3u : 0xffffffffu;
+  const uint32_t s = min(min(k0, k1), min(k2, k3)) & 3u;
+  im &= ~(1u << s);
+  if (im & 8u) e[n++] = make_uint2(k3, (uint32_t)base + 3u);
+  if (im & 4u) e[n++] = make_uint2(k2, (uint32_t)base + 2u);
+  if (im & 2u) e[n++] = make_uint2(k1, (uint32_t)base + 1u);
+  if (im & 1u) e[n++] = make_uint2(k0, (uint32_t)base);
+  return s;
+}
+
+// The last pending node nearer than `best`.
+__device__ __forceinline__ bool pop4(const uint2 (&e)[kStack4], int& n, float best, int& node) {
+  const float cull = best * kWiden;
+  while (n > 0) {
+    const uint2 x = e[--n];
+    if (__uint_as_float(x.x & ~3u) <= cull) {
+      node = (int)x.y;
+      return true;
+    }
+  }
+  return false;
+}
+
+// Walks the 4-wide tree `nodes` from `node`; leaf(k) handles leaf k and lowers
+// `best`, the distance beyond which nothing counts.
+template <class Leaf>
+__device__ __forceinline__ void walk4(const Node4* nodes, int node, const Ray4& r, float& best, unsigned budget,
+                                      bool& over_budget, Leaf&& leaf) {
+  uint2 stack[kStack4];
+  int sp = 0;
+  unsigned steps = 0;
+  while (true) {
+    if (++steps > budget) { over_budget = true; break; }
+    const char* np = reinterpret_cast<const char*>(nodes + node);
+    float t[4];
+    int base;
+    const uint32_t hit = visit4(np, r, best, t, base);
+    uint32_t lm = hit & 15u, im = hit >> 4;
+    if (lm) {
+      const int* cp = reinterpret_cast<const int*>(np + 96);
+      do {
+        const int s = __ffs((int)lm) - 1;
+        lm &= lm - 1u;
+        leaf(~__ldg(cp + s));
+      } while (lm);
+      const float cull = best * kWiden;
+      if (!(t[0] <= cull)) im &= ~1u;
+      if (!(t[1] <= cull)) im &= ~2u;
+      if (!(t[2] <= cull)) im &= ~4u;
+      if (!(t[3] <= cull)) im &= ~8u;
+    }
+    if (im) {
+      uint32_t s = (im >> 1) - (im >> 3);  // the slot of a single bit
+      if (im & (im - 1u)) {
+        if (sp + 3 > kStack4) { over_budget = true; break; }  // only a corrupt tree gets this deep
+        s = push4(stack, sp, im, t, base);
+      }
+      node = base + (int)s;
+      continue;
+    }
+    if (!pop4(stack, sp, best, node)) break;
+  }
+}
+
+// The same walk for leaves that are walks of their own (instances): a lane that
+// meets leaves waits until every lane of its warp stands at some or is done, and
+// they enter them together.  The node's internal children are pushed first and
+// wait for the closer hit that the leaves may bring.
+template <class Leaf>
+__device__ __forceinline__ void walk4_gather(const Node4* nodes, int node, const Ray4& r, float& best, unsigned budget,
+                                             bool& over_budget, Leaf&& leaf) {
+  uint2 stack[kStack4];
+  int sp = 0;
+  unsigned steps = 0;
+  bool more = true;
+  while (more) {
+    uint32_t lm = 0;
+    const int* cp = nullptr;
+    while (more) {
+      if (++steps > budget) { over_budget = true; more = false; break; }
+      const char* np = reinterpret_cast<const char*>(nodes + node);
+      float t[4];
+      int base;
+      const uint32_t hit = visit4(np, r, best, t, base);
+      lm = hit & 15u;
+      const uint32_t im = hit >> 4;
+      cp = reinterpret_cast<const int*>(np + 96);
+      if (im) {
+        uint32_t s = (im >> 1) - (im >> 3);
+        if (sp + 4 > kStack4) { over_budget = true; more = false; break; }
+        if (im & (im - 1u)) s = push4(stack, sp, im, t, base);
+        node = base + (int)s;
+        if (lm) {
+          const float ts = s == 0 ? t[0] : (s == 1 ? t[1] : (s == 2 ? t[2] : t[3]));
+          stack[sp++] = make_uint2((__float_as_uint(ts) & ~3u) | s, (uint32_t)node);
+        }
+      } else if (!lm) {
+        more = pop4(stack, sp, best, node);
+      }
+      if (lm) break;
+    }
+    if (over_budget || !lm) break;
+    do {
+      const int s = __ffs((int)lm) - 1;
+      lm &= lm - 1u;
+      leaf(~__ldg(cp + s));
+    } while (lm && !over_budget);
+    if (over_budget) break;
+    more = pop4(stack, sp, best, node);
+  }
+}
+
 // Closest hit through the 4-wide tree, the default walk.  Same boxes, same slab
 // arithmetic and culling rule (tmin <= min(tmax, best) * (1 + 2^-22)) and the
 // same triangle test and tie rule as the binary walk, so the hit (t, face) is
@@ -386,104 +569,11 @@ __device__ __forceinline__ void trace_ray4(const DeviceMap& map, const V& o, con
   h.t = tfar;
   h.tri = -1;
   h.face = 0xffffffffu;
-  if (map.root < 0) return;
-  // A ray with a NaN or infinite component hits no triangle (its edge functions
-  // or its quotient are NaN), but a box test with NaN planes admits everything.
-  float z = o.x * 0.0f;
-  z = fmaf(o.y, 0.0f, z); z = fmaf(o.z, 0.0f, z);
-  z = fmaf(d.x, 0.0f, z); z = fmaf(d.y, 0.0f, z); z = fmaf(d.z, 0.0f, z);
-  if (z != 0.0f) return;
+  if (map.root < 0 || !finite_ray(o, d)) return;
   const V inv = reciprocal(d);
   const RayW rw = make_rayw(o, d, inv);
-  const RayBox rb = make_raybox(o, d, inv);
-  const bool bx = rb.ix < 0.f, by = rb.iy < 0.f, bz = rb.iz < 0.f;
-  const unsigned long long pix = pack2(rb.ix, rb.ix), piy = pack2(rb.iy, rb.iy), piz = pack2(rb.iz, rb.iz);
-  const float nxa = bx ? rb.chx : rb.clx, fxa = bx ? rb.clx : rb.chx;
-  const float nya = by ? rb.chy : rb.cly, fya = by ? rb.cly : rb.chy;
-  const float nza = bz ? rb.chz : rb.clz, fza = bz ? rb.clz : rb.chz;
-  const unsigned long long cnx = pack2(nxa, nxa), cfx = pack2(fxa, fxa), cny = pack2(nya, nya),
-                           cfy = pack2(fya, fya), cnz = pack2(nza, nza), cfz = pack2(fza, fza);
-  // byte offsets of the near planes in a node; the far planes are at ^ 16
-  const uint32_t ox = bx ? 16u : 0u, oy = by ? 48u : 32u, oz = bz ? 80u : 64u;
-  uint2 stack[kStack4];
-  int sp = 0;
-  int node = 0;
-  unsigned steps = 0;
-  while (true) {
-    if (++steps > budget) { over_budget = true; break; }
-    const char* np = reinterpret_cast<const char*>(map.nodes4 + node);
-    const ulonglong2 qnx = __ldg(reinterpret_cast<const ulonglong2*>(np + ox));
-    const ulonglong2 qfx = __ldg(reinterpret_cast<const ulonglong2*>(np + (ox ^ 16u)));
-    const ulonglong2 qny = __ldg(reinterpret_cast<const ulonglong2*>(np + oy));
-    const ulonglong2 qfy = __ldg(reinterpret_cast<const ulonglong2*>(np + (oy ^ 16u)));
-    const ulonglong2 qnz = __ldg(reinterpret_cast<const ulonglong2*>(np + oz));
-    const ulonglong2 qfz = __ldg(reinterpret_cast<const ulonglong2*>(np + (oz ^ 16u)));
-    const int2 meta = __ldg(reinterpret_cast<const int2*>(np + 112));
-    float t[4], m[4];
-    {
-      float x0, x1, y0, y1, z0, z1;
-      plane2(qnx.x, pix, cnx, x0, x1); plane2(qny.x, piy, cny, y0, y1); plane2(qnz.x, piz, cnz, z0, z1);
-      t[0] = fmax3f(x0, y0, fmaxf(z0, 0.0f));
-      t[1] = fmax3f(x1, y1, fmaxf(z1, 0.0f));
-      plane2(qnx.y, pix, cnx, x0, x1); plane2(qny.y, piy, cny, y0, y1); plane2(qnz.y, piz, cnz, z0, z1);
-      t[2] = fmax3f(x0, y0, fmaxf(z0, 0.0f));
-      t[3] = fmax3f(x1, y1, fmaxf(z1, 0.0f));
-      plane2(qfx.x, pix, cfx, x0, x1); plane2(qfy.x, piy, cfy, y0, y1); plane2(qfz.x, piz, cfz, z0, z1);
-      m[0] = fmin3f(x0, y0, fminf(z0, h.t));
-      m[1] = fmin3f(x1, y1, fminf(z1, h.t));
-      plane2(qfx.y, pix, cfx, x0, x1); plane2(qfy.y, piy, cfy, y0, y1); plane2(qfz.y, piz, cfz, z0, z1);
-      m[2] = fmin3f(x0, y0, fminf(z0, h.t));
-      m[3] = fmin3f(x1, y1, fminf(z1, h.t));
-    }
-    uint32_t hit = 0;
-    if (t[0] <= m[0] * kWiden) hit |= 0x11u;
-    if (t[1] <= m[1] * kWiden) hit |= 0x22u;
-    if (t[2] <= m[2] * kWiden) hit |= 0x44u;
-    if (t[3] <= m[3] * kWiden) hit |= 0x88u;
-    hit &= (uint32_t)meta.y;
-    uint32_t lm = hit & 15u, im = hit >> 4;
-    if (lm) {
-      const int* cp = reinterpret_cast<const int*>(np + 96);
-      do {
-        const int s = __ffs((int)lm) - 1;
-        lm &= lm - 1u;
-        test_tri(map, rw, ~__ldg(cp + s), h);
-      } while (lm);
-      const float cull = h.t * kWiden;
-      if (!(t[0] <= cull)) im &= ~1u;
-      if (!(t[1] <= cull)) im &= ~2u;
-      if (!(t[2] <= cull)) im &= ~4u;
-      if (!(t[3] <= cull)) im &= ~8u;
-    }
-    if (im) {
-      uint32_t s = (im >> 1) - (im >> 3);  // the slot of a single bit
-      if (im & (im - 1u)) {
-        // entry distance and slot in one word: ordered as the distances (>= 0)
-        // are, rounded down to 4 ulp, which keeps the later culls conservative
-        const uint32_t k0 = im & 1u ? (__float_as_uint(t[0]) & ~3u) : 0xffffffffu;
-        const uint32_t k1 = im & 2u ? (__float_as_uint(t[1]) & ~3u) | 1u : 0xffffffffu;
-        const uint32_t k2 = im & 4u ? (__float_as_uint(t[2]) & ~3u) | 2u : 0xffffffffu;
-        const uint32_t k3 = im & 8u ? (__float_as_uint(t[3]) & ~3u) | 3u : 0xffffffffu;
-        const uint32_t kn = min(min(k0, k1), min(k2, k3));
-        s = kn & 3u;
-        if (sp + 3 > kStack4) { over_budget = true; break; }  // only a corrupt tree gets this deep
-        im &= ~(1u << s);
-        if (im & 8u) stack[sp++] = make_uint2(k3, (uint32_t)meta.x + 3u);
-        if (im & 4u) stack[sp++] = make_uint2(k2, (uint32_t)meta.x + 2u);
-        if (im & 2u) stack[sp++] = make_uint2(k1, (uint32_t)meta.x + 1u);
-        if (im & 1u) stack[sp++] = make_uint2(k0, (uint32_t)meta.x);
-      }
-      node = meta.x + (int)s;
-      continue;
-    }
-    bool found = false;
-    const float cull = h.t * kWiden;
-    while (sp > 0) {
-      const uint2 e = stack[--sp];
-      if (__uint_as_float(e.x & ~3u) <= cull) { node = (int)e.y; found = true; break; }
-    }
-    if (!found) break;
-  }
+  const Ray4 r = make_ray4(make_raybox(o, d, inv));
+  walk4(map.nodes4, map.root, r, h.t, budget, over_budget, [&](int k) { test_tri(map, rw, k, h); });
   if (over_budget) {
     h.tri = -1;
     h.t = tfar;
