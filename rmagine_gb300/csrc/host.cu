@@ -29,6 +29,11 @@ constexpr int kSlots = 4;        // staging chunks in flight; more than the comp
 constexpr int kMaxDevices = 64;
 constexpr size_t kDefaultChunkBytes = size_t(128) << 20;
 constexpr int kDefaultCompute = 2;
+// A launch lasts as long as its slowest rays (60 to 100 us) however few poses it
+// has, while 8 MiB cross the link in 45 us.  64 poses of 10,000 directions with
+// 17 bytes a ray: 427 / 331 / 284 / 281 / 287 us with least chunks of 1 / 4 / 8 /
+// 16 / 32 MiB; 200 poses 558 / 520 / 511 / 515 / 596.
+constexpr size_t kLeastChunkBytes = size_t(8) << 20;
 std::atomic<size_t> g_chunk_bytes{kDefaultChunkBytes};
 std::atomic<int> g_compute{kDefaultCompute};
 
@@ -92,17 +97,18 @@ rmg_outputs outputs_at(const AttrList& a) {
 using Launch = std::function<int(const rmg_transform* Tbm, uint32_t n, const rmg_outputs* out, cudaStream_t st)>;
 
 // Pose chunks of the simulate host forms: full chunks of `chunk` poses, then
-// the last two chunks' worth split in halving sizes (at least chunk / 8 poses),
-// so that the work left after the final launch -- its copy, and forming its
-// points -- is a small chunk's.  Returns the first pose of every chunk and n.
-std::vector<uint32_t> chunk_schedule(uint32_t n, size_t chunk) {
+// the last two chunks' worth split in halving sizes (at least chunk / 8 and
+// `least` poses), so that the work left after the final launch -- its copy, and
+// forming its points -- is a small chunk's.  Returns the first pose of every
+// chunk and n.
+std::vector<uint32_t> chunk_schedule(uint32_t n, size_t chunk, size_t least) {
   std::vector<uint32_t> first{0};
   uint64_t p = 0;
   while (n - p > 2 * chunk) {
     p += chunk;
     first.push_back((uint32_t)p);
   }
-  const uint64_t min_tail = std::max<uint64_t>(1, chunk / 8);
+  const uint64_t min_tail = std::max<uint64_t>(std::max<uint64_t>(1, least), chunk / 8);
   while (p < n) {
     const uint64_t rem = n - p;
     const uint64_t take = rem <= min_tail ? rem : std::max<uint64_t>(min_tail, std::min<uint64_t>(chunk, (rem + 1) / 2));
@@ -293,10 +299,13 @@ int host_pipeline(const char* what, const rmg_sensor* sensor, const rmg_transfor
     if (host.ptr[a]) bytes_per_ray += host.size[a];
   if (bytes_per_ray == 0 || rays_per_pose == 0) return RMG_OK;
   const size_t bytes_per_pose = bytes_per_ray * rays_per_pose;
-  // at least one pose, at most ceil(n/2) so that two chunks overlap
-  size_t chunk = std::max<size_t>(1, g_chunk_bytes.load() / bytes_per_pose);
-  chunk = std::min<size_t>(chunk, std::max<uint32_t>(1u, (n_poses + 1) / 2));
-  const std::vector<uint32_t> first = chunk_schedule(n_poses, chunk);  // chunk k: poses [first[k], first[k+1])
+  // at least one pose, at most ceil(n/2) so that two chunks overlap, but no chunk
+  // below kLeastChunkBytes, unless the caller asks for smaller ones
+  const size_t want = g_chunk_bytes.load();
+  const size_t least = std::min(want, kLeastChunkBytes) / bytes_per_pose;
+  size_t chunk = std::max<size_t>(1, want / bytes_per_pose);
+  chunk = std::min<size_t>(chunk, std::max<size_t>(std::max<size_t>(1, (n_poses + 1) / 2), least));
+  const std::vector<uint32_t> first = chunk_schedule(n_poses, chunk, least);  // chunk k: poses [first[k], first[k+1])
   const uint32_t n_chunks = (uint32_t)first.size() - 1;
   const int slots = (int)std::min<uint32_t>(kSlots, n_chunks);
 
