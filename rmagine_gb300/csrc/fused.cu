@@ -238,7 +238,7 @@ cudaError_t launch_fused(const FusedParams& F, int kind, unsigned grid, unsigned
 int default_config(const rmg_sensor* s, rmg_launch_config* cfg);
 int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_transform* Tsb,
                       const rmg_transform* Tbm, uint32_t n_poses, const rmg_outputs* out,
-                      const rmg_launch_config& cfg, TraceParams& P);
+                      const rmg_launch_config& cfg, TraceParams& P, bool any_tile);
 
 }  // namespace rmg
 
@@ -259,7 +259,7 @@ extern "C" int rmg_simulate_statistics(const rmg_map* map, const rmg_sensor* sen
     default_config(sensor, &cfg);
     rmg_outputs out{};
     FusedParams F;
-    make_trace_params(map, sensor, Tsb, Tbm, n_poses, &out, cfg, F.T);
+    make_trace_params(map, sensor, Tsb, Tbm, n_poses, &out, cfg, F.T, false);
     F.dp = reinterpret_cast<const float*>(dataset->points);
     F.dmask = dataset->mask;
     F.dids = dataset->ids;

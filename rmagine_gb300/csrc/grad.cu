@@ -174,7 +174,7 @@ int default_config(const rmg_sensor* s, rmg_launch_config* cfg);
 int check_config(const rmg_launch_config& c);
 int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_transform* Tsb,
                       const rmg_transform* Tbm, uint32_t n_poses, const rmg_outputs* out,
-                      const rmg_launch_config& cfg, TraceParams& P);
+                      const rmg_launch_config& cfg, TraceParams& P, bool any_tile);
 
 }  // namespace rmg
 
@@ -197,7 +197,7 @@ extern "C" int rmg_range_pose_grad(const rmg_map* map, const rmg_sensor* sensor,
     out.ranges = ranges_sim;
     out.face_ids = face_ids;
     GradParams G;
-    make_trace_params(map, sensor, Tsb, Tbm, n_poses, &out, cfg, G.T);
+    make_trace_params(map, sensor, Tsb, Tbm, n_poses, &out, cfg, G.T, false);
     G.r_obs = ranges_obs;
     G.delta = huber_delta;
     const uint32_t ctas_per_pose = (G.T.tiles_per_pose + cfg.block_warps - 1) / cfg.block_warps;

@@ -239,7 +239,7 @@ __global__ void __maxnreg__(64) k_trace_scene(const SceneParams S) {
   const uint32_t vid = ty * P.tile_h + (lane >> P.tile_w_log2);
   const uint32_t hid = tx * tile_w + (lane & (tile_w - 1));
   const uint32_t W = P.sen.width, H = P.sen.height;
-  if (vid >= H || hid >= W) return;
+  if (lane >= P.tile_lanes || vid >= H || hid >= W) return;
   const uint32_t loc = visit_loc(P.sen, vid * W + hid);
 
   Best best;
@@ -342,7 +342,7 @@ __global__ void k_piece_boxes(const PieceReq* req, uint32_t n, float* out) {
 int default_config(const rmg_sensor* s, rmg_launch_config* cfg);
 int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_transform* Tsb,
                       const rmg_transform* Tbm, uint32_t n_poses, const rmg_outputs* out,
-                      const rmg_launch_config& cfg, TraceParams& P);
+                      const rmg_launch_config& cfg, TraceParams& P, bool any_tile);
 DeviceMap device_view(const rmg_map* m);
 
 }  // namespace rmg
@@ -756,7 +756,7 @@ extern "C" int rmg_simulate_scene(const rmg_scene* s, const rmg_sensor* sensor, 
     rmg_map empty;
     std::memset(&empty, 0, sizeof(empty));
     const rmg_map* top = s->tlas ? s->tlas : &empty;
-    make_trace_params(top, sensor, Tsb, Tbm, n_poses, out, cfg, S.T);
+    make_trace_params(top, sensor, Tsb, Tbm, n_poses, out, cfg, S.T, true);
     S.T.map.status = s->d_status;
     S.inst = s->d_inst;
     S.geoms = s->d_geoms;

@@ -62,10 +62,29 @@ void fit_tile(uint32_t W, uint32_t H, uint32_t& tw, uint32_t& th) {
   while (tw > 1 && tw / 2 >= W) { tw /= 2; th *= 2; }
 }
 
-// Fills the parameter block of one sensor's launch; returns the tile count.
+// Rays per warp of a launch of n rays: 32, halved (down to 4) while the warps
+// still find room on the GPU, 36 per SM at the 4-wide walk's 56 registers and a
+// few more.  A launch of few warps is a latency chain as long as the longest path
+// of a warp's rays, and fewer rays share fewer detours: one 16 x 900 scan of the
+// box room 28.6 -> 20.7 us (4 rays a warp), of the 1M-triangle terrain 59.6 ->
+// 42.5, 3 x 32 x 513 there 84.8 -> 62.4 (8), 4 x 10,000 scattered directions 73.5
+// -> 57.6.  Larger launches fill the SMs with whole warps: with room for 120 per
+// SM eight room scans take 48 us instead of 37.
+constexpr uint32_t kWarpRoom = 42;
+uint32_t lanes_for(uint64_t n_rays) {
+  const uint64_t room = (uint64_t)kWarpRoom * (uint64_t)device_sm_count();
+  uint32_t lanes = 32;
+  while (lanes > 4 && n_rays * 2 <= room * lanes) lanes /= 2;
+  return lanes;
+}
+
+// Fills the parameter block of one sensor's launch.  any_tile: its tiles may hold
+// fewer than 32 rays -- where the caller left the launch to the library and every
+// ray stands for itself; sums over a warp's rays keep whole warps, so that a
+// pose's result does not depend on the launch it is part of.
 int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_transform* Tsb,
                       const rmg_transform* Tbm, uint32_t n_poses, const rmg_outputs* out,
-                      const rmg_launch_config& cfg, TraceParams& P) {
+                      const rmg_launch_config& cfg, TraceParams& P, bool any_tile) {
   P.map = device_view(map);
   P.sen = device_view(sensor);
   const rmg_transform Tsb_ = *Tsb;
@@ -75,6 +94,11 @@ int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_tr
   P.out = *out;
   uint32_t tw = cfg.tile_w, th = cfg.tile_h;
   fit_tile(sensor->width, sensor->height, tw, th);
+  if (any_tile)
+    for (uint32_t lanes = lanes_for((uint64_t)sensor->width * sensor->height * n_poses); tw * th > lanes;) {
+      if (tw > th) tw /= 2; else th /= 2;
+    }
+  P.tile_lanes = tw * th;
   P.tile_w_log2 = (uint32_t)log2u(tw);
   P.tile_h = th;
   P.tiles_x = (sensor->width + tw - 1) / tw;
@@ -170,7 +194,7 @@ extern "C" int rmg_simulate_ex(const rmg_map* map, const rmg_sensor* sensor, con
         !out->geom_ids && !out->object_ids)
       return RMG_OK;  // nothing requested: the reference writes nothing either
     TraceParams P;
-    make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, cfg, P);
+    make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, cfg, P, cfg_in == nullptr);
     return launch_plain(P, sensor, cfg, as_stream(stream));
   });
 }
@@ -221,7 +245,7 @@ extern "C" int rmg_autotune_launch_config(const rmg_map* map, const rmg_sensor* 
           if (c.tile_w > sensor->width && c.tile_w != base.tile_w) continue;
           if (check_config(c) != RMG_OK) continue;
           TraceParams P;
-          make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, c, P);
+          make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, c, P, false);
           if ((w.bvh_width == 4 && !P.wide) || (w.bvh_width == 8 && !P.wide8) || (w.packet == 1 && !P.packet))
             continue;  // not available here
           s = launch_plain(P, sensor, c, st);

@@ -884,6 +884,7 @@ struct TraceParams {
   rmg_outputs out;
   uint32_t tile_w_log2;
   uint32_t tile_h;
+  uint32_t tile_lanes;     // tile_w * tile_h: 32, or fewer where a launch is too small to fill the GPU
   uint32_t tiles_x;
   uint32_t tiles_per_pose;
   uint64_t n_tiles;
@@ -1057,7 +1058,7 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_trace(const TraceParams P) {
   const uint32_t vid = ty * P.tile_h + (lane >> P.tile_w_log2);
   const uint32_t hid = tx * tile_w + (lane & (tile_w - 1));
   const uint32_t W = P.sen.width, H = P.sen.height;
-  const bool inside = vid < H && hid < W;
+  const bool inside = lane < P.tile_lanes && vid < H && hid < W;
   if (TB != kPacketTB && !inside) return;  // the packet walk needs every lane
   const uint32_t loc = inside ? visit_loc(P.sen, vid * W + hid) : 0;
 
