@@ -173,18 +173,18 @@ __global__ void __launch_bounds__(kBlock4) k_collapse(const Node* __restrict__ b
   }
 }
 
-// Boxes of every slot from the (refitted) binary records.
+// Boxes of every slot from the (refitted) binary records, one thread per slot.
 __global__ void k_wide_refit(const Node* __restrict__ bn, const int* __restrict__ src4, uint32_t n4, Node4* w4) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n4) return;
-  Node4 w = w4[j];
-  for (int k = 0; k < 4; ++k) {
-    const int s = src4[4 * j + k];
-    if (s < 0) continue;
-    const Cand c = cand_of(bn[s >> 1], s >> 1, s & 1);
-    set_slot(w, k, c.lo, c.hi);
-  }
-  w4[j] = w;
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 4ull * n4) return;
+  const int s = src4[i];
+  if (s < 0) return;
+  const Node* b = bn + (s >> 1);
+  const int side = s & 1;
+  const float4 xy = __ldg(side ? &b->b : &b->a);
+  const float2 z = __ldg(reinterpret_cast<const float2*>(&b->c) + side);
+  float* w = reinterpret_cast<float*>(w4 + (i >> 2)) + (i & 3);
+  w[0] = xy.x; w[4] = xy.y; w[8] = xy.z; w[12] = xy.w; w[16] = z.x; w[20] = z.y;
 }
 
 }  // namespace
@@ -296,8 +296,8 @@ int wide_set_child(rmg_map* m, uint32_t node, uint32_t slot, int child) {
 // Refreshes the wide boxes after the binary tree was refitted (asynchronous).
 int wide_refit(rmg_map* m, cudaStream_t st) {
   if (!m->d_nodes4 || m->n_nodes4 == 0) return RMG_OK;
-  k_wide_refit<<<(m->n_nodes4 + kBlock4 - 1) / kBlock4, kBlock4, 0, st>>>(m->d_nodes, m->d_src4, m->n_nodes4,
-                                                                        m->d_nodes4);
+  k_wide_refit<<<(unsigned)((4ull * m->n_nodes4 + kBlock4 - 1) / kBlock4), kBlock4, 0, st>>>(m->d_nodes, m->d_src4,
+                                                                                          m->n_nodes4, m->d_nodes4);
   const int s = cuda_status(cudaGetLastError(), "k_wide_refit");
   return s == RMG_OK ? wide8_refit(m, st) : s;
 }
