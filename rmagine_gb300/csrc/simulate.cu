@@ -78,6 +78,13 @@ uint32_t lanes_for(uint64_t n_rays) {
   return lanes;
 }
 
+// A tile of at most `lanes` rays: the longer side halved as often as it takes.
+void shrink_tile(uint32_t lanes, uint32_t& tw, uint32_t& th) {
+  while (tw * th > lanes) {
+    if (tw > th) tw /= 2; else th /= 2;
+  }
+}
+
 // Fills the parameter block of one sensor's launch.  any_tile: its tiles may hold
 // fewer than 32 rays -- where the caller left the launch to the library and every
 // ray stands for itself; sums over a warp's rays keep whole warps, so that a
@@ -94,10 +101,7 @@ int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_tr
   P.out = *out;
   uint32_t tw = cfg.tile_w, th = cfg.tile_h;
   fit_tile(sensor->width, sensor->height, tw, th);
-  if (any_tile)
-    for (uint32_t lanes = lanes_for((uint64_t)sensor->width * sensor->height * n_poses); tw * th > lanes;) {
-      if (tw > th) tw /= 2; else th /= 2;
-    }
+  if (any_tile) shrink_tile(lanes_for((uint64_t)sensor->width * sensor->height * n_poses), tw, th);
   P.tile_lanes = tw * th;
   P.tile_w_log2 = (uint32_t)log2u(tw);
   P.tile_h = th;

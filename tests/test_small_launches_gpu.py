@@ -8,6 +8,7 @@ import torch
 
 import rmagine_gb300 as rm
 from rmagine_gb300 import scenes, sensors
+from rmagine_gb300.batched import BatchPlan
 from rmagine_gb300.grad import range_pose_grad
 
 pytestmark = pytest.mark.gpu
@@ -44,6 +45,26 @@ def test_few_rays_equal_the_same_rays_among_many(world, name, kind):
         part = sim.simulate(poses[:n].contiguous()).tensors()
         for a, t in part.items():
             assert torch.equal(t.contiguous().view(torch.uint8), whole[a][:n * per].contiguous().view(torch.uint8)), (n, a)
+
+
+@pytest.mark.parametrize("poses", [1, 9, 60])
+def test_batch_of_few_rays_equals_plain_launches(world, poses):
+    s, m, _ = world
+    jobs, want = [], []
+    for i, (name, model) in enumerate(models().items()):
+        n = poses + i
+        T = torch.from_numpy(scenes.terrain_poses(s, n, seed=7 + i, size=60.0)).cuda()
+        b = rm.resize_memory_bundle(rm.Bundle("hits", "ranges", "normals"), model.getWidth(), model.getHeight(), n)
+        sim = rm.make_simulator(model, m)
+        sim.launch_config = rm.launch_config(bvh_width=2, packet=0)  # whole warps, the binary walk
+        jobs.append((sim, T, b))
+        want.append(sim.simulate(T, attrs=("hits", "ranges", "normals")).tensors())
+    plan = BatchPlan(m, jobs)
+    for _ in range(2):
+        plan.launch()
+        for (_, _, b), w in zip(jobs, want):
+            for a, t in b.tensors().items():
+                assert torch.equal(t.contiguous().view(torch.uint8), w[a].contiguous().view(torch.uint8)), a
 
 
 @pytest.mark.parametrize("name", ["1x1", "3x5", "40x1", "33x65", "table"])
