@@ -435,9 +435,12 @@ int fill_params(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
   return RMG_OK;
 }
 
-// The 4-correspondence loads need aligned arrays (16 bytes; 4 for byte masks),
-// nothing of the batch size.
+// The 4-correspondence loads need aligned arrays (16 bytes; 4 for byte masks).  A
+// batch that is no multiple of four takes them from 2,048 correspondences per CTA
+// on: below, one correspondence per thread spreads over more warps, whose
+// binary32 sums are shorter.
 bool vec_ok(const StatsParams& P, bool p2l) {
+  if (P.n_per % 4 != 0 && std::min(P.n_per, P.chunk_len) < 2048) return false;
   auto al = [](const void* p, uintptr_t a) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) % a) == 0; };
   return al(P.dp, 16) && al(P.mp, 16) && (!p2l || al(P.mn, 16)) && al(P.dmask, 4) && al(P.mmask, 4) &&
          al(P.dids, 16) && al(P.mids, 16);
