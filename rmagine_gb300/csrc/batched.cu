@@ -215,8 +215,8 @@ int build_jobs(rmg_batch* b) {
   uint64_t begin = 0, rays = 0;
   for (const rmg_batch_entry& e : b->entries) rays += (uint64_t)e.sensor->width * e.sensor->height * e.n_poses;
   // few rays: tiles of 4 to 16 (see lanes_for).  24,600 rays of 64 scattered and
-  // camera sensors on a 30,000-triangle terrain: 125 us with whole warps, 76 so;
-  // 590,000 rays keep whole warps (266 us, 322 with 16).
+  // camera sensors on a 30,000-triangle terrain: 79 us with whole warps, 56 so;
+  // 590,000 rays keep whole warps (231 us, 272 with 16).
   const uint32_t lanes = lanes_for(rays);
   for (const rmg_batch_entry& e : b->entries) {
     JobDev J;
@@ -260,14 +260,18 @@ int persistent_grid(const rmg_batch_config& c, int trail_bits, unsigned& grid) {
   return RMG_OK;
 }
 
-BatchParams params(const rmg_batch* b) {
+BatchParams params(const rmg_batch* b, uint64_t warps) {
   BatchParams B;
   B.map = device_view(b->map);
   B.jobs = b->jobs;
   B.n_jobs = (uint32_t)b->jobs_h.size();
   B.total_tiles = b->total_tiles;
   B.counter = b->counter;
-  B.grab = b->cfg.grab;
+  // A warp takes `grab` tiles at a time only where there are many times as many:
+  // a tile of scattered rays lasts 60 us, and 3.4 tiles for each warp in twos make
+  // four (590,000 rays of 512 sensors: 266 -> 231 us; 161,000
+  // rays 165 -> 103).
+  B.grab = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(b->cfg.grab, b->total_tiles / (16 * warps)));
   B.budget = 2u * b->map->n_nodes + 64u;
   B.trail_bits = trail_bits_for_depth(b->map->depth);
   B.full_stack = b->map->depth <= (unsigned)kFullStack ? 1 : 0;
@@ -285,7 +289,7 @@ int launch_direct(rmg_batch* b, cudaStream_t st) {
                                   : full ? 0 : trail_bits_for_depth(b->map->depth), grid);
   if (s != RMG_OK) return s;
   RMG_CUDA_TRY(cudaMemsetAsync(b->counter, 0, sizeof(unsigned long long), st));
-  return cuda_status(launch_batched(params(b), (int)b->cfg.stack_depth, grid, 32u * b->cfg.block_warps, st),
+  return cuda_status(launch_batched(params(b, (uint64_t)grid * b->cfg.block_warps), (int)b->cfg.stack_depth, grid, 32u * b->cfg.block_warps, st),
                      "k_trace_batched");
 }
 
