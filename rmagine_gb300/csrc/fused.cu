@@ -33,10 +33,14 @@
 namespace rmg {
 namespace {
 
-// tiles (32 rays) each warp reduces before its CTA writes one partial record
-#ifndef RMG_FUSED_TILES_PER_WARP
-#define RMG_FUSED_TILES_PER_WARP 8
-#endif
+// Tiles (32 rays) that a warp reduces before its CTA writes one partial record.
+// Fewer make more CTAs, of which the last, partly idle wave is a smaller part;
+// more make fewer records and less final work.  8 / 4 / 2 / 1 tiles, us: 256 poses
+// x 180 tiles 279 / 259 / 246 / 238, 1 pose 123 / 101 / 79 / 67, 48 x 656 500 / 347 /
+// 334 / 328, 4,000 x 180 2,668 / 2,687 / 2,747 / 2,877, 300 x 4,096 4,201 / 4,203 /
+// 4,254 / 4,512.  The number depends on the sensor alone, so that a pose's sums
+// do not depend on how many poses a launch holds.
+constexpr uint32_t tiles_per_warp(uint32_t tiles_per_pose) { return tiles_per_pose >= 1024 ? 4 : 2; }
 
 struct FusedParams {
   TraceParams T;
@@ -268,7 +272,7 @@ extern "C" int rmg_simulate_statistics(const rmg_map* map, const rmg_sensor* sen
     F.pre_stride = pre_transform_stride ? 1u : 0u;
     F.max_dist = params->max_dist;
     F.dataset_id = params->dataset_id;
-    F.tiles_per_cta = cfg.block_warps * RMG_FUSED_TILES_PER_WARP;
+    F.tiles_per_cta = cfg.block_warps * tiles_per_warp(F.T.tiles_per_pose);
     F.ctas_per_pose = (F.T.tiles_per_pose + F.tiles_per_cta - 1) / F.tiles_per_cta;
     const uint64_t grid = (uint64_t)F.ctas_per_pose * n_poses;
     if (grid > 0x7fffffffull) return fail(RMG_ERR_INVALID_ARG, "rmg_simulate_statistics: too many rays for one launch");
