@@ -133,6 +133,27 @@ __device__ __forceinline__ V qrot(const Q& q, const V& p) {
   return V{r.x, r.y, r.z};
 }
 
+// Sums of N values over a warp, N a power of two up to 32: lane l gets the sum of
+// v[l / (32 / N)].  Each exchange halves the values a lane keeps (N - 1 shuffles
+// and one per level left, where every lane summing every value takes 5 N), and
+// each sum's tree is that of the butterfly over 16, 8, 4, 2 and 1 lanes.
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+  const uint32_t lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int n = N / 2; n > 0; n >>= 1, o >>= 1) {
+    const bool up = (lane & (uint32_t)o) != 0;
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      const float give = up ? v[k] : v[k + n];
+      v[k] = (up ? v[k + n] : v[k]) + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
 // Three-input float min/max (PTX ISA 8.8, sm_100 and later); same NaN rules as
 // the two-input forms.
 __device__ __forceinline__ float fmin3f(float a, float b, float c) {

@@ -17,10 +17,9 @@
 // masked out (mask == 0 or id != dataset_id) are not cast at all.
 //
 // Reduction: a warp casts one 32-ray tile at a time; the tile's correspondences
-// are summed around the tile's first valid correspondence in binary32 (a
-// 5-level butterfly), then lanes 0..15 turn the 16 sums into raw moments about
-// the sensor origin in binary64 (one moment per lane) and accumulate them over
-// the warp's tiles.  A CTA adds its warps in a fixed order into one partial
+// are summed around the tile's first valid correspondence in binary32, then 16
+// lanes turn the 16 sums into raw moments about the sensor origin in binary64
+// (one moment per lane) and accumulate them over the warp's tiles.  A CTA adds its warps in a fixed order into one partial
 // record; k_fused_final adds a pose's partials in a fixed order, forms the
 // means and the covariance E[m d^T] - E[m] E[d]^T and runs Umeyama in binary64.
 // Deterministic; the result differs from simulate + statistics only by the
@@ -57,30 +56,26 @@ struct FusedParams {
   double* partial;        // [n_poses * ctas_per_pose][16]
 };
 
-// v[0..15] = (n, sum d', sum m', sum m' d'^T row-major) around the shift
-// (sd, sm); returns, for lane k < 16, moment k about the origin in binary64:
+// Adds a tile's sums to the moments about the origin in binary64.  Lane 2 k (and
+// its neighbour) holds moment k and x, the tile's (n, sum d', sum m', sum m' d'^T
+// row-major) around the shift (sd, sm):
 //   n, sum d = sum d' + n sd, sum m = sum m' + n sm,
-//   sum m d^T = sum m' d'^T + sm (sum d')^T + (sum m') sd^T + n sm sd^T.
-__device__ __forceinline__ double raw_moment(const float v[16], uint32_t k, const V& sd, const V& sm) {
-  float x = v[0];
-#pragma unroll
-  for (int j = 1; j < 16; ++j) x = k == (uint32_t)j ? v[j] : x;
-  const double n = (double)v[0];
-  if (k == 0) return n;
-  if (k < 4) {
-    const float s = k == 1 ? sd.x : (k == 2 ? sd.y : sd.z);
-    return (double)x + n * (double)s;
-  }
-  if (k < 7) {
-    const float s = k == 4 ? sm.x : (k == 5 ? sm.y : sm.z);
-    return (double)x + n * (double)s;
-  }
-  const uint32_t i = (k - 7) / 3, j = (k - 7) - 3 * ((k - 7) / 3);
+//   sum m d^T = sum m' d'^T + (sum m') sd^T + sm (sum d)^T.
+// A binary64 instruction takes 64 cycles for a warp, however many of its lanes
+// are on, so every lane does the same three, on its own operands.  With branches
+// on k there were some 15, and the 16 sums took 80 shuffles: 256 poses of 16 x 360
+// rays 240 us a call, now 235.
+__device__ __forceinline__ double add_moment(double acc, float x, float n, const V& sd, const V& sm) {
+  const uint32_t k = (threadIdx.x & 31) >> 1;
+  const uint32_t e = k < 7 ? 0 : k - 7, i = e / 3, j = e - 3 * i;
+  const float sum_mi = __shfl_sync(0xffffffffu, x, 2 * (4 + i));
   const float smi = i == 0 ? sm.x : (i == 1 ? sm.y : sm.z);
-  const float sdj = j == 0 ? sd.x : (j == 1 ? sd.y : sd.z);
-  const float sum_dj = j == 0 ? v[1] : (j == 1 ? v[2] : v[3]);
-  const float sum_mi = i == 0 ? v[4] : (i == 1 ? v[5] : v[6]);
-  return (double)x + (double)smi * (double)sum_dj + (double)sum_mi * (double)sdj + n * (double)smi * (double)sdj;
+  const uint32_t c = k < 4 ? k - 1 : k < 7 ? k - 4 : j;
+  const float b0 = k < 4 || k >= 7 ? sd.x : sm.x, b1 = k < 4 || k >= 7 ? sd.y : sm.y, b2 = k < 4 || k >= 7 ? sd.z : sm.z;
+  const float b = k == 0 ? 0.f : c == 0 ? b0 : (c == 1 ? b1 : b2);
+  const double y = fma((double)(k < 7 ? n : sum_mi), (double)b, (double)x);
+  const double sum_dj = __shfl_sync(0xffffffffu, y, 2 * (1 + j));
+  return acc + fma(k < 7 ? 0.0 : (double)smi, k < 7 ? 0.0 : sum_dj, y);
 }
 
 template <bool P2L, int OK, int SS, int TB>
@@ -147,13 +142,11 @@ __global__ void __maxnreg__((trace_regs<TB>())) k_trace_stats(const FusedParams 
       v[10] = my * dx; v[11] = my * dy; v[12] = my * dz;
       v[13] = mz * dx; v[14] = mz * dy; v[15] = mz * dz;
     }
-#pragma unroll
-    for (int k = 0; k < 16; ++k)
-      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    if (lane < 16) acc += raw_moment(v, lane, sd, sm);
+    const float x = warp_sums(v);
+    acc = add_moment(acc, x, (float)__popc(bal), sd, sm);
   }
   __shared__ double red[16][8];
-  if (lane < 16) red[lane][wib] = acc;
+  if (!(lane & 1)) red[lane >> 1][wib] = acc;
   __syncthreads();
   if (threadIdx.x < 16) {
     double s = 0.0;

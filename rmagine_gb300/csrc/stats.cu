@@ -101,23 +101,17 @@ struct FAcc {
 };
 
 // Folding a binary32 run into binary64: the 32 lanes' runs are first summed
-// pairwise across the warp in binary32 (a 5-level butterfly), then ONE lane
-// adds the 16 warp sums to the warp's binary64 accumulators in shared memory.
-// The GB300's binary64 pipe is narrow; this keeps it at 16 operations per 1024
-// correspondences instead of 16 per 32.  All lanes must call fold together.
+// pairwise across the warp in binary32, then a lane for each of the 16 sums adds
+// it to the warp's binary64 accumulators in shared memory.  A binary64
+// instruction takes the GB300 64 cycles for a warp, however many of its lanes
+// are on; this keeps it at one per 1024 correspondences.  All lanes must call
+// fold together.
 __device__ __forceinline__ void fold(double (*acc)[kStatsThreads / 32], FAcc& f) {
   float v[16] = {f.n, f.d[0], f.d[1], f.d[2], f.m[0], f.m[1], f.m[2], f.md[0], f.md[1], f.md[2],
                  f.md[3], f.md[4], f.md[5], f.md[6], f.md[7], f.md[8]};
-#pragma unroll
-  for (int k = 0; k < 16; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  const float x = warp_sums(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane < 16) {
-    float x = v[0];
-#pragma unroll
-    for (int k = 1; k < 16; ++k) x = lane == k ? v[k] : x;
-    acc[lane][warp] += (double)x;
-  }
+  if (!(lane & 1)) acc[lane >> 1][warp] += (double)x;
   f.zero();
 }
 
@@ -125,28 +119,35 @@ __device__ __forceinline__ V ldv(const float* p, uint64_t i) {
   return V{__ldg(p + 3 * i), __ldg(p + 3 * i + 1), __ldg(p + 3 * i + 2)};
 }
 
-__device__ void finalize(const StatsParams& P, uint32_t b, const double* acc, const V& sd, const V& sm) {
-  const double n = acc[0];
-  double dm[3] = {0, 0, 0}, mm[3] = {0, 0, 0}, C[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (n > 0.0) {
-    const double ds[3] = {acc[1] / n, acc[2] / n, acc[3] / n};
-    const double ms[3] = {acc[4] / n, acc[5] / n, acc[6] / n};
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) C[3 * i + j] = acc[7 + 3 * i + j] / n - ms[i] * ds[j];
-    dm[0] = (double)sd.x + ds[0]; dm[1] = (double)sd.y + ds[1]; dm[2] = (double)sd.z + ds[2];
-    mm[0] = (double)sm.x + ms[0]; mm[1] = (double)sm.y + ms[1]; mm[2] = (double)sm.z + ms[2];
+// Lanes 0-15 hold a batch's 16 sums v: its mean, covariance and count, a lane
+// each (one division deep; by one lane the 15 divisions took 1.2 us of the
+// narrow binary64 pipe).
+__device__ __forceinline__ void finalize(const StatsParams& P, uint32_t b, double v, const V& sd, const V& sm,
+                                         double* tot) {
+  const int k = threadIdx.x;
+  const double n = __shfl_sync(0xffffu, v, 0);
+  const bool some = n > 0.0;
+  const double x = some ? v / n : 0.0;
+  const int e = k < 7 ? 0 : k - 7;  // covariance element of this lane
+  const double md = __shfl_sync(0xffffu, x, 4 + e / 3), dd = __shfl_sync(0xffffu, x, 1 + e % 3);
+  double o = n;
+  if (k > 0) {
+    const float s = k == 1 ? sd.x : k == 2 ? sd.y : k == 3 ? sd.z : k == 4 ? sm.x : k == 5 ? sm.y : sm.z;
+    o = !some ? 0.0 : k < 7 ? (double)s + x : x - md * dd;
   }
-  if (P.stats) store_cross_stats(n, dm, mm, C, P.stats + b);
-  if (P.dstats) {
-    double* o = P.dstats + 16ull * b;
-    for (int k = 0; k < 3; ++k) { o[k] = dm[k]; o[3 + k] = mm[k]; }
-    for (int k = 0; k < 9; ++k) o[6 + k] = C[k];
-    o[15] = n;
+  if (P.dstats) P.dstats[16ull * b + (k == 0 ? 15 : k - 1)] = o;
+  if (P.stats) {
+    tot[k == 0 ? 15 : k - 1] = o;
+    __syncwarp(0xffffu);
+    if (k == 0) store_cross_stats(n, tot, tot + 3, tot + 6, P.stats + b);
   }
 }
 
+// Bound by latency: a CTA loads three or four times, sums and retires.  Four CTAs
+// (64 registers) hide more of it than three; five spill.  400 batches of 10,007
+// with masks, statistics, transform and backward, us a call: 140 / 136 / 150.
 template <bool P2L, bool VEC, bool PRE>
-__global__ void __launch_bounds__(kStatsThreads, 3) k_stats(const StatsParams P) {
+__global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P) {
   const uint32_t b = blockIdx.x / P.chunks;
   const uint32_t c = blockIdx.x - b * P.chunks;
   const uint64_t base = (uint64_t)b * P.n_per;
@@ -169,8 +170,7 @@ __global__ void __launch_bounds__(kStatsThreads, 3) k_stats(const StatsParams P)
     // per array, one word of masks -- counted over the whole array, so that they
     // are aligned whatever n_per is; a batch's first and last group may hold
     // neighbours of other batches, which are skipped, and the array's last group
-    // is read one by one if it is cut short.  400 batches of 10,007 with masks and
-    // pre-transforms: 46 us, one correspondence at a time 51.
+    // is read one by one if it is cut short.
     const uint64_t e0 = base + lo, e1 = base + hi, total = (uint64_t)P.n_batches * P.n_per;
     const uint64_t g0 = e0 / 4, g1 = lo < hi ? (e1 + 3) / 4 : g0;
     int run = 0;
@@ -256,10 +256,8 @@ __global__ void __launch_bounds__(kStatsThreads, 3) k_stats(const StatsParams P)
   for (int w = 0; w < kStatsThreads / 32; ++w) v += acc[threadIdx.x][w];
   __shared__ double tot[16];
   __shared__ bool last;
-  tot[threadIdx.x] = v;
   if (P.chunks == 1) {
-    __syncwarp(0xffffu);
-    if (threadIdx.x == 0) finalize(P, b, tot, sd, sm);
+    finalize(P, b, v, sd, sm, tot);
     return;
   }
   P.partial[16ull * blockIdx.x + threadIdx.x] = v;
@@ -271,9 +269,7 @@ __global__ void __launch_bounds__(kStatsThreads, 3) k_stats(const StatsParams P)
   __threadfence();
   double s = 0.0;
   for (uint32_t k = 0; k < P.chunks; ++k) s += __ldcg(&P.partial[16ull * (b * P.chunks + k) + threadIdx.x]);
-  tot[threadIdx.x] = s;
-  __syncwarp(0xffffu);
-  if (threadIdx.x == 0) finalize(P, b, tot, sd, sm);
+  finalize(P, b, s, sd, sm, tot);
 }
 
 __global__ void k_umeyama_dstats(const double* dstats, uint32_t n, rmg_transform* out) {
@@ -335,16 +331,16 @@ __global__ void k_umeyama_bwd_coef(const rmg_cross_stats* stats, const float* gr
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) gR.a[i][j] = (grad_R ? (double)grad_R[9ull * b + 3 * i + j] : 0.0) - gt[i] * d[j];
     const M3d GC = rotation_backward(U, sv, V, gR);
-    const double n = (double)s.n_meas;
+    const double rn = 1.0 / (double)s.n_meas;
     double A[3][3], B[3][3];
     for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) { A[i][j] = GC.a[i][j] / n; B[i][j] = GC.a[j][i] / n; }
+      for (int j = 0; j < 3; ++j) { A[i][j] = GC.a[i][j] * rn; B[i][j] = GC.a[j][i] * rn; }
     double gd[3];
     for (int i = 0; i < 3; ++i) gd[i] = -(R.a[0][i] * gt[0] + R.a[1][i] * gt[1] + R.a[2][i] * gt[2]);
     bool finite = true;
     for (int i = 0; i < 3; ++i) {
-      c.cm[i] = (float)(gt[i] / n - (A[i][0] * d[0] + A[i][1] * d[1] + A[i][2] * d[2]));
-      c.cd[i] = (float)(gd[i] / n - (B[i][0] * m[0] + B[i][1] * m[1] + B[i][2] * m[2]));
+      c.cm[i] = (float)(gt[i] * rn - (A[i][0] * d[0] + A[i][1] * d[1] + A[i][2] * d[2]));
+      c.cd[i] = (float)(gd[i] * rn - (B[i][0] * m[0] + B[i][1] * m[1] + B[i][2] * m[2]));
       for (int j = 0; j < 3; ++j) {
         c.A[3 * i + j] = (float)A[i][j];
         c.B[3 * i + j] = (float)B[i][j];
