@@ -1,6 +1,5 @@
-// Binary64 3x3 linear algebra for the Umeyama step: singular value
-// decomposition with right-handed factors, the Kabsch/Umeyama rotation, the
-// rotation-matrix -> quaternion conversion, and the rotation's derivative.
+// Binary64 3x3 singular value decomposition with right-handed factors by one
+// thread (linalg4.cuh solves the Umeyama step with four lanes per problem).
 //
 // Replaces rmagine's Numerical-Recipes svdcmp (src/rmagine_core/src/math/
 // linalg.cpp:101, device src/rmagine_cuda/src/math/linalg.cu:61) and
@@ -45,13 +44,6 @@ __host__ __device__ inline M3d m3_mul_tn(const M3d& x, const M3d& y) {  // x^T y
   M3d r;
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) r.a[i][j] = x.a[0][i] * y.a[0][j] + x.a[1][i] * y.a[1][j] + x.a[2][i] * y.a[2][j];
-  return r;
-}
-
-__host__ __device__ inline M3d m3_mul_nt(const M3d& x, const M3d& y) {  // x y^T
-  M3d r;
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) r.a[i][j] = x.a[i][0] * y.a[j][0] + x.a[i][1] * y.a[j][1] + x.a[i][2] * y.a[j][2];
   return r;
 }
 
@@ -102,7 +94,7 @@ __host__ __device__ inline void swap_columns(double& lx, double& ly, double x[3]
 
 // C = U diag(s) V^T with U, V proper rotations; s[0] >= s[1] >= |s[2]|, s[2] signed.
 //
-// One thread solves one matrix, so what counts is the latency of its binary64
+// One thread solves one matrix, so what counts is the length of its binary64
 // chain.  400 matrices: 41 us with indexed arrays in local memory, five
 // divisions and square roots per rotation and four warps to an SM's narrow
 // binary64 pipe; 26 us in registers, with three, one warp to a CTA.
@@ -157,78 +149,10 @@ __host__ __device__ inline void svd3_rot(const M3d& C, M3d& U, double s[3], M3d&
   s[2] = u3[0] * B.a[0][2] + u3[1] * B.a[1][2] + u3[2] * B.a[2][2];
 }
 
-// Rotation matrix -> unit quaternion (x, y, z, w).  Branch choice as in
-// rmagine's Matrix -> Quaternion cast (math/types/MatrixOps.tcc:1492-1529),
-// so both pick the same of the two signs q / -q.
-__host__ __device__ inline void rot_to_quat(const M3d& R, double q[4]) {
-  const double tr = R.a[0][0] + R.a[1][1] + R.a[2][2];
-  // S^2 / 4 and which component it is; the others are sums over S
-  const int big = tr > 0.0 ? 3 : (R.a[0][0] > R.a[1][1] && R.a[0][0] > R.a[2][2]) ? 0 : (R.a[1][1] > R.a[2][2] ? 1 : 2);
-  const double x = R.a[2][1] - R.a[1][2], y = R.a[0][2] - R.a[2][0], z = R.a[1][0] - R.a[0][1];
-  const double xy = R.a[0][1] + R.a[1][0], xz = R.a[0][2] + R.a[2][0], yz = R.a[1][2] + R.a[2][1];
-  const double arg = big == 3 ? tr + 1.0
-                              : big == 0 ? 1.0 + R.a[0][0] - R.a[1][1] - R.a[2][2]
-                                         : big == 1 ? 1.0 + R.a[1][1] - R.a[0][0] - R.a[2][2]
-                                                    : 1.0 + R.a[2][2] - R.a[0][0] - R.a[1][1];
-  const double S = sqrt(arg) * 2.0, rS = 1.0 / S;
-  if (big == 3) { q[3] = 0.25 * S; q[0] = x * rS; q[1] = y * rS; q[2] = z * rS; }
-  else if (big == 0) { q[3] = x * rS; q[0] = 0.25 * S; q[1] = xy * rS; q[2] = xz * rS; }
-  else if (big == 1) { q[3] = y * rS; q[0] = xy * rS; q[1] = 0.25 * S; q[2] = yz * rS; }
-  else { q[3] = z * rS; q[0] = xz * rS; q[1] = yz * rS; q[2] = 0.25 * S; }
-  const double n = 1.0 / sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
-  for (int k = 0; k < 4; ++k) q[k] *= n;
-}
-
-// Umeyama / Kabsch: R = U V^T, t = m - R d.  n == 0 or a non-finite result
-// gives the identity rotation (optimization.cpp:19-46).
-__host__ __device__ inline void umeyama_d(const M3d& C, const double d[3], const double m[3], unsigned int n,
-                                          M3d& R, double q[4], double t[3]) {
-  if (n == 0) {
-    R = m3_eye();
-    q[0] = q[1] = q[2] = 0.0; q[3] = 1.0;
-    t[0] = t[1] = t[2] = 0.0;
-    return;
-  }
-  M3d U, V;
-  double s[3];
-  svd3_rot(C, U, s, V);
-  R = m3_mul_nt(U, V);
-  rot_to_quat(R, q);
-  bool finite = true;
-  for (int k = 0; k < 4; ++k) finite = finite && isfinite(q[k]);
-  if (!finite) {
-    R = m3_eye();
-    q[0] = q[1] = q[2] = 0.0; q[3] = 1.0;
-  }
-  for (int i = 0; i < 3; ++i) t[i] = m[i] - (R.a[i][0] * d[0] + R.a[i][1] * d[1] + R.a[i][2] * d[2]);
-}
-
-// Relative size below which s_i + s_j counts as zero in rotation_backward.
+// Relative size below which s_i + s_j counts as zero in the rotation's gradient.
 // The covariance reaches the backward in binary32 (rmagine's CrossStatistics),
 // so singular values carry an absolute error of about 1e-7 s0: a smaller sum
 // is rounding noise, and dividing by it would only amplify that noise.
 constexpr double kRotGradGap = 1e-6;
-
-// Gradient of L through R = U V^T (C = U diag(s) V^T, rotations U, V):
-// dL/dC = U K V^T with K_ij = (G_ij - G_ji) / (s_i + s_j) for i != j, K_ii = 0,
-// G = U^T (dL/dR) V.  Where s_i + s_j <= kRotGradGap * s0 the optimal rotation
-// about the axis u_i x u_j is not unique (collinear correspondences: s2 = s3 = 0;
-// a reflection with two equal singular values: s2 = -s3) and R is not
-// differentiable there: that pair contributes no gradient (K_ij = K_ji = 0).
-// The rest of the gradient is exact; close to the boundary it grows like
-// 1 / (s_i + s_j), as the rotation's true derivative does.
-__host__ __device__ inline M3d rotation_backward(const M3d& U, const double s[3], const M3d& V, const M3d& gR) {
-  const M3d G = m3_mul(m3_mul_tn(U, gR), V);
-  M3d K = m3_zero();
-  const double gap = kRotGradGap * fabs(s[0]);
-  for (int i = 0; i < 3; ++i) {
-    for (int j = 0; j < 3; ++j) {
-      if (i == j) continue;
-      const double den = s[i] + s[j];
-      K.a[i][j] = den > gap ? (G.a[i][j] - G.a[j][i]) / den : 0.0;
-    }
-  }
-  return m3_mul_nt(m3_mul(U, K), V);
-}
 
 }  // namespace rmg

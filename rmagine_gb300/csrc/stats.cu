@@ -16,7 +16,7 @@
 // batches split over several CTAs are combined in a fixed order by the last
 // CTA to finish, so results are deterministic.  The mean and covariance are
 // formed in binary64 (cov = E[m' d'^T] - E[m'] E[d']^T), then rounded to the
-// binary32 CrossStatistics record.  Umeyama runs in binary64 (linalg.cuh).
+// binary32 CrossStatistics record.  Umeyama runs in binary64 (linalg4.cuh).
 //
 // Filters follow the reference GPU kernels: mask > 0, ids equal to the
 // constraint ids, and ||M - D||^2 < max_dist^2 (p2p) or
@@ -24,17 +24,18 @@
 #include <algorithm>
 
 #include "internal.h"
-#include "linalg.cuh"
+#include "linalg4.cuh"
 #include "stats.cuh"
 
 namespace rmg {
 namespace {
 
 constexpr int kStatsThreads = 256;
-// Threads of the CTAs that solve one 3x3 problem per thread: one warp, so that
-// a few hundred problems reach as many SMs as there are and no two warps share
-// an SM's narrow binary64 pipe.
+// Threads of the CTAs that solve 3x3 problems (svd3 one per thread, the others with
+// four lanes each): one warp, so that a few hundred problems reach as many SMs as
+// there are.
 constexpr int kSolveThreads = 32;
+unsigned solve_grid(uint32_t n) { return (unsigned)((4ull * n + kSolveThreads - 1) / kSolveThreads); }
 constexpr int kFold = 8;  // vector groups (4 correspondences) per binary32 run
 
 struct StatsParams {
@@ -272,17 +273,17 @@ __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P)
   finalize(P, b, s, sd, sm, tot);
 }
 
-__global__ void k_umeyama_dstats(const double* dstats, uint32_t n, rmg_transform* out) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
+__global__ void __launch_bounds__(kSolveThreads) k_umeyama_dstats(const double* dstats, uint32_t n,
+                                                                  rmg_transform* out) {
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, b = min(i, n - 1);
   const double* s = dstats + 16ull * b;
   M3d C;
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) C.a[i][j] = s[6 + 3 * i + j];
-  M3d R;
+  const double d[3] = {s[0], s[1], s[2]}, m[3] = {s[3], s[4], s[5]};
   double q[4], t[3];
-  umeyama_d(C, s, s + 3, (unsigned int)s[15], R, q, t);
-  store_tf(out + b, q, t);
+  umeyama_lanes(C, d, m, (unsigned int)s[15], q, t);
+  if (i < n && (threadIdx.x & 3) == 0) store_tf(out + b, q, t);
 }
 
 __device__ __forceinline__ void load_stats(const rmg_cross_stats& s, M3d& C, double d[3], double m[3]) {
@@ -292,67 +293,60 @@ __device__ __forceinline__ void load_stats(const rmg_cross_stats& s, M3d& C, dou
     for (int c = 0; c < 3; ++c) C.a[r][c] = s.covariance.data[3 * c + r];
 }
 
-__global__ void k_umeyama_stats(const rmg_cross_stats* stats, uint32_t n, rmg_transform* out) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
+__global__ void __launch_bounds__(kSolveThreads) k_umeyama_stats(const rmg_cross_stats* stats, uint32_t n,
+                                                                 rmg_transform* out) {
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, b = min(i, n - 1);
   const rmg_cross_stats s = stats[b];
-  M3d C, R;
+  M3d C;
   double d[3], m[3], q[4], t[3];
   load_stats(s, C, d, m);
-  umeyama_d(C, d, m, s.n_meas, R, q, t);
-  store_tf(out + b, q, t);
+  umeyama_lanes(C, d, m, s.n_meas, q, t);
+  if (i < n && (threadIdx.x & 3) == 0) store_tf(out + b, q, t);
 }
 
 // ---- backward --------------------------------------------------------------------
 // Per batch: coefficients of the affine per-correspondence gradients
 //   dL/dM_i = A D_i + cm,   dL/dD_i = B M_i + cd
 // with A = G_C / n, B = G_C^T / n, cm = g_t/n - A d_mean,
-// cd = -R^T g_t / n - B m_mean, G_C = rotation_backward(dL/dR - g_t d_mean^T).
+// cd = -R^T g_t / n - B m_mean, G_C = rotation_backward_lanes(dL/dR - g_t d_mean^T).
 struct Coef { float A[9], cm[3], B[9], cd[3]; };
 
-__global__ void k_umeyama_bwd_coef(const rmg_cross_stats* stats, const float* grad_R, const float* grad_t,
-                                   uint32_t n_batches, Coef* coef) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_batches) return;
+__global__ void __launch_bounds__(kSolveThreads) k_umeyama_bwd_coef(const rmg_cross_stats* stats, const float* grad_R,
+                                                                    const float* grad_t, uint32_t n_batches,
+                                                                    Coef* coef) {
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, b = min(i, n_batches - 1);
+  const int j = column4();
   const rmg_cross_stats s = stats[b];
-  Coef c;
-  for (int k = 0; k < 9; ++k) { c.A[k] = 0.f; c.B[k] = 0.f; }
-  for (int k = 0; k < 3; ++k) { c.cm[k] = 0.f; c.cd[k] = 0.f; }
-  if (s.n_meas > 0) {
-    M3d C, U, V;
-    double d[3], m[3], sv[3];
-    load_stats(s, C, d, m);
-    svd3_rot(C, U, sv, V);
-    const M3d R = m3_mul_nt(U, V);
-    double gt[3] = {0, 0, 0};
-    if (grad_t)
-      for (int k = 0; k < 3; ++k) gt[k] = grad_t[3ull * b + k];
-    M3d gR;
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) gR.a[i][j] = (grad_R ? (double)grad_R[9ull * b + 3 * i + j] : 0.0) - gt[i] * d[j];
-    const M3d GC = rotation_backward(U, sv, V, gR);
-    const double rn = 1.0 / (double)s.n_meas;
-    double A[3][3], B[3][3];
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) { A[i][j] = GC.a[i][j] * rn; B[i][j] = GC.a[j][i] * rn; }
-    double gd[3];
-    for (int i = 0; i < 3; ++i) gd[i] = -(R.a[0][i] * gt[0] + R.a[1][i] * gt[1] + R.a[2][i] * gt[2]);
-    bool finite = true;
-    for (int i = 0; i < 3; ++i) {
-      c.cm[i] = (float)(gt[i] * rn - (A[i][0] * d[0] + A[i][1] * d[1] + A[i][2] * d[2]));
-      c.cd[i] = (float)(gd[i] * rn - (B[i][0] * m[0] + B[i][1] * m[1] + B[i][2] * m[2]));
-      for (int j = 0; j < 3; ++j) {
-        c.A[3 * i + j] = (float)A[i][j];
-        c.B[3 * i + j] = (float)B[i][j];
-        finite = finite && isfinite(A[i][j]);
-      }
-    }
-    if (!finite) {  // the forward fell back to the identity: no gradient flows
-      for (int k = 0; k < 9; ++k) { c.A[k] = 0.f; c.B[k] = 0.f; }
-      for (int k = 0; k < 3; ++k) { c.cm[k] = 0.f; c.cd[k] = 0.f; }
-    }
+  M3d C, U, V;
+  double d[3], m[3], sv[3];
+  load_stats(s, C, d, m);
+  svd3_lanes(C, U, sv, V);
+  double gt[3] = {0, 0, 0}, gR[3], vr[3], R[3], GC[3];
+  if (grad_t)
+    for (int k = 0; k < 3; ++k) gt[k] = grad_t[3ull * b + k];
+  for (int k = 0; k < 3; ++k)
+    gR[k] = (grad_R ? (double)grad_R[9ull * b + 3 * k + j] : 0.0) - gt[k] * pick(j, d[0], d[1], d[2]);
+  rotation_backward_lanes(U, sv, V, gR, GC);
+  row_of(V, j, vr);
+  mul_col(U, vr, R);  // column j of R = U V^T
+  const double rn = 1.0 / (double)s.n_meas;
+  for (int k = 0; k < 3; ++k) GC[k] *= rn;
+  const M3d A = gather4(GC);
+  double row[3];
+  row_of(A, j, row);
+  const float cm = (float)(pick(j, gt[0], gt[1], gt[2]) * rn - dot(row, d));
+  const float cd = (float)(-dot(R, gt) * rn - dot(GC, m));
+  bool finite = s.n_meas > 0;  // not finite: the forward fell back to the identity, no gradient flows
+  for (int k = 0; k < 3; ++k)
+    for (int c = 0; c < 3; ++c) finite = finite && isfinite(A.a[k][c]);
+  if (i >= n_batches || (threadIdx.x & 3) == 3) return;
+  Coef* o = coef + b;  // lane j: column j of A, row j of B = A^T, element j of the others
+  for (int k = 0; k < 3; ++k) {
+    o->A[3 * k + j] = finite ? (float)GC[k] : 0.f;
+    o->B[3 * j + k] = finite ? (float)GC[k] : 0.f;
   }
-  coef[b] = c;
+  o->cm[j] = finite ? cm : 0.f;
+  o->cd[j] = finite ? cd : 0.f;
 }
 
 struct BwdParams {
@@ -490,7 +484,7 @@ int stats_entry(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
   }
   s = launch_stats(P, p2l, st);
   if (s == RMG_OK && transforms) {
-    k_umeyama_dstats<<<(n_batches + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, st>>>(dstats, n_batches, transforms);
+    k_umeyama_dstats<<<solve_grid(n_batches), kSolveThreads, 0, st>>>(dstats, n_batches, transforms);
     s = cuda_status(cudaGetLastError(), "k_umeyama_dstats");
   }
   pool_free(dstats, st);
@@ -584,7 +578,7 @@ extern "C" int rmg_umeyama_transform(const rmg_cross_stats* stats, uint32_t n, r
   return guarded("rmg_umeyama_transform", [&]() -> int {
     if (n == 0) return RMG_OK;
     if (!stats || !out) return fail(RMG_ERR_INVALID_ARG, "rmg_umeyama_transform: NULL argument");
-    k_umeyama_stats<<<(n + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, as_stream(stream)>>>(stats, n, out);
+    k_umeyama_stats<<<solve_grid(n), kSolveThreads, 0, as_stream(stream)>>>(stats, n, out);
     return cuda_status(cudaGetLastError(), "k_umeyama_stats");
   });
 }
@@ -608,7 +602,7 @@ extern "C" int rmg_umeyama_backward(const rmg_transform* pre_transforms, uint32_
     Coef* coef = nullptr;
     s = pool_alloc(&coef, n_batches, st, "backward coefficients");
     if (s != RMG_OK) return s;
-    k_umeyama_bwd_coef<<<(n_batches + kSolveThreads - 1) / kSolveThreads, kSolveThreads, 0, st>>>(stats, grad_R, grad_t, n_batches, coef);
+    k_umeyama_bwd_coef<<<solve_grid(n_batches), kSolveThreads, 0, st>>>(stats, grad_R, grad_t, n_batches, coef);
     s = cuda_status(cudaGetLastError(), "k_umeyama_bwd_coef");
     if (s == RMG_OK) {
       B.coef = coef;
