@@ -125,7 +125,9 @@ typedef struct rmg_launch_config {
   uint32_t chunk;         /* refill mode: tiles a warp takes from the work counter at a time (>= 1) */
   uint32_t bvh_width;     /* 2: walk the binary tree; 4: the 4-wide tree collapsed from it; 8: the 8-wide
                              tree with quantized boxes collapsed from it (4 and 8 when the map has the tree
-                             and refill == 0); 0: the default.  Results are identical. */
+                             and refill == 0); 0: the default, the 4-wide tree where it can be walked, unless
+                             refill, packet == 1 or a stack_depth other than 16 asks for the binary one.
+                             Results are identical. */
   uint32_t packet;        /* 1: the warp walks the binary tree together (a node is visited when any of
                              its 32 rays needs it; refill == 0, bvh_width != 4); 0: each ray walks alone;
                              2: the default.  Results are identical. */
@@ -193,7 +195,7 @@ int rmg_map_refit(rmg_map* map, const rmg_vec3* vertices, uint32_t n_vertices, v
  * Karras and Laine, HPG 2017) collapsed from the map's binary tree, for
  * rmg_launch_config.bvh_width = 8; refits refresh it.  Opt-in, as Embree's
  * scene build options choose its BVH (EmbreeScene.hpp:61-83): on the
- * workloads measured here the binary walk is faster, so maps do not build it
+ * workloads measured here the other walks are faster, so maps do not build it
  * by default.  Not concurrent with simulate calls on the same map; synchronises
  * with `stream`.  A map whose boxes cannot be quantized (extents beyond
  * 255 * 2^60) keeps no 8-wide tree. */
@@ -210,9 +212,11 @@ int rmg_map_status(rmg_map* map, int clear);
 /* Test hook: overwrite one child link of one BVH node (synchronous).  Used
  * to check that a corrupt tree ends in RMG_ERR_TRAVERSAL_BUDGET, not a
  * fault; values are range-checked so every link stays inside the arrays.
- * which 0 / 1: left / right link of binary node `node` (the map then drops
- * its 4-wide tree, so the damaged binary tree is the one walked);
- * which 2..5: slot which-2 of 4-wide node `node`. */
+ * which 0 / 1: left / right link of binary node `node` (the map's 4-wide tree
+ * is walked no longer, so the damaged binary tree is the one walked);
+ * which 2..5: slot which-2 of 4-wide node `node` (the node's slots are put in
+ * order again, internal children first, and those children are copied behind
+ * the last node). */
 int rmg_map_debug_set_child(rmg_map* map, uint32_t node, uint32_t which, int32_t child);
 
 /* ---------------------------------------------------------------------------
@@ -293,7 +297,8 @@ int rmg_host_set_pipeline(uint64_t chunk_bytes, uint32_t compute_streams);
  * other attributes and keeps the host threads free.  The results are the same
  * bytes under both. */
 int rmg_host_set_points_policy(uint32_t policy);
-/* Returns the host forms' cached staging memory to the driver. */
+/* Returns the host forms' cached staging memory to the driver, and what the
+ * library's memory pool (maps, scratch, workspaces) keeps unused. */
 int rmg_host_staging_trim(void);
 
 /* Times a fixed set of launch configurations (per-ray binary walk, warp

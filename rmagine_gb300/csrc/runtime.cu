@@ -165,7 +165,7 @@ std::vector<uint32_t> visiting_order(const float* dirs, size_t n) {
 
 // ---- the library's device memory pool ---------------------------------------
 // cudaMalloc / cudaFree of a map's arrays and a build's scratch took 1.0 of the
-// 2.6 ms of building and scanning a 530,000-triangle map; workspaces taken from
+// 2.6 ms of building and scanning a 537,000-triangle map; workspaces taken from
 // the device's default pool cost 250 us again after every synchronisation, when
 // that pool returns what is unused.  One pool of the library's own per device
 // keeps up to kPoolKeepBytes between calls; it gives everything back when the

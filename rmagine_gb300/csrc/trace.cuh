@@ -559,9 +559,10 @@ __device__ __forceinline__ void walk4_gather(const Node4* nodes, int node, const
 // nearest first and the others as they come (a third hit is rare).  Internal
 // children are consecutive nodes, so no link is read for them.  12.7 visits per
 // ray against 24.9 binary ones there.  Both walks, us a pass: that terrain with
-// a 128 x 1024 lidar 3,221 (binary) / 3,126, a 2.1M-triangle terrain with a
-// 640 x 480 camera 1,558 / 1,466, the box room with a 16 x 360 lidar 318 / 299,
-// one 16 x 900 scan there 32.5 / 29.3, scattered directions 204 / 184.  Sorting
+// a 128 x 1024 lidar 3,140 (binary) / 3,030, a 2.1M-triangle terrain with a
+// 640 x 480 camera 1,513 / 1,414, the box room with a 16 x 360 lidar 312 / 292,
+// one 16 x 900 scan there 32.1 / 27.8 (tiles of 32), scattered directions 202 /
+// 178.  Sorting
 // all four distances, postponing the leaf tests until every lane has one,
 // 32-bit node offsets and a pointer per plane all measured slower.
 __device__ __forceinline__ void trace_ray4(const DeviceMap& map, const V& o, const V& d, float tfar,

@@ -70,7 +70,7 @@ __device__ __forceinline__ void swap_cand(Cand& x, Cand& y, bool yes) {
 // Level `level` of the collapse: its wide nodes, whose binary roots are
 // bin_of[j], get their children; internal children receive new wide indices, a
 // CTA's with one addition to the counter.  The last CTA to finish closes the
-// next level, so the launches follow one another without the host.  530,000
+// next level, so the launches follow one another without the host.  537,000
 // triangles, 13 levels: 188 us with all allocations made, where a host
 // synchronisation per level and an atomic per node took 330.
 __global__ void __launch_bounds__(kBlock4) k_collapse(const Node* __restrict__ bn, int* bin_of, WideBuild* B, int level,
