@@ -646,13 +646,17 @@ __device__ void build_tiny(Rec* slot, const uint16_t* perm, const Rec* rec, cons
 }
 
 // One CTA builds the subtree of one small task at a time.
-__global__ void __launch_bounds__(kSmallBlk) k_small(Build* B, const Task* small, const Rec* rec0, const Rec* rec1,
-                                                     SmallOut out) {
+__global__ void __launch_bounds__(kSmallBlk) k_small(Build* B, uint32_t p, const Task* small, const Rec* rec0,
+                                                     const Rec* rec1, SmallOut out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmallShared& S = *reinterpret_cast<SmallShared*>(smem_raw);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t n_small = B->n_small;
   uint32_t max_depth = 0;
+  // large tasks are left (of level parity p), or the build has failed
+  if (threadIdx.x == 0) S.task = B->n_big[p] | B->bad | B->bad_face;
+  __syncthreads();
+  if (S.task != 0) return;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) S.task = atomicAdd(&B->next_small, 1u);
@@ -815,14 +819,21 @@ int sah_build(rmg_map* m, cudaStream_t st, uint32_t* d_order) {
     k_root<<<1, 1024, 0, st>>>(n, B, big[0], chunks[0], bins[0], small);
     chk(cudaGetLastError(), "sah prep");
   }
-  // Levels of large tasks: as many as a balanced tree has and a few more, then
-  // as many more as the counters ask for.
+  // Levels of large tasks: as many as a balanced tree has and one more, then the
+  // small tasks; where large ones are left after all, k_small does nothing and the
+  // host, which looks once at the end, adds levels.  (A look before k_small as well
+  // was 15 us of an idle GPU.)
+  const int smem = (int)sizeof(SmallShared);
+  int per_sm = 0;
+  chk(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "k_small shared memory");
+  chk(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small, kSmallBlk, smem), "k_small occupancy");
+  const unsigned most = (unsigned)(std::max(per_sm, 1) * device_sm_count());
   uint32_t level = 0, upto = 0;
   if (n > kSmall) {
     while ((uint64_t)kSmall << upto < n) ++upto;
-    upto += 2;
+    upto += 1;
   }
-  while (s == RMG_OK && upto > 0) {
+  while (s == RMG_OK) {
     for (; level < upto; ++level) {
       const uint32_t p = level & 1u;
       // a level's chunks: at most one per kChunk positions and one more per task
@@ -834,26 +845,14 @@ int sah_build(rmg_map* m, cudaStream_t st, uint32_t* d_order) {
       k_partition<<<grid, kBlk, 0, st>>>(B, p, big[p], chunks[p], splits, hist, rec[p], rec[p ^ 1], big[p ^ 1],
                                          m->d_nodes, d_order);
     }
-    chk(cudaGetLastError(), "sah level");
+    k_small<<<std::min(most, max_small), kSmallBlk, smem, st>>>(B, level & 1u, small, rec[0], rec[1],
+                                                                SmallOut{m->d_nodes, m->d_leaf_parent, d_order});
+    chk(cudaGetLastError(), "sah levels");
     chk(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "sah counters");
     chk(cudaStreamSynchronize(st), "sah sync");
     if (s != RMG_OK || h.bad || h.bad_face || h.n_big[level & 1u] == 0) break;
     if (level > kMaxDepth) { s = fail(RMG_ERR_CUDA, "SAH build: too many levels"); break; }
     upto = level + 3;
-  }
-  if (s == RMG_OK && !h.bad && !h.bad_face) {
-    const int smem = (int)sizeof(SmallShared);
-    chk(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "k_small shared memory");
-    int per_sm = 0;
-    chk(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small, kSmallBlk, smem), "k_small occupancy");
-    if (s == RMG_OK) {
-      const unsigned most = (unsigned)(std::max(per_sm, 1) * device_sm_count());
-      k_small<<<std::min(most, max_small), kSmallBlk, smem, st>>>(B, small, rec[0], rec[1],
-                                                                  SmallOut{m->d_nodes, m->d_leaf_parent, d_order});
-      chk(cudaGetLastError(), "k_small");
-    }
-    chk(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "sah counters");
-    chk(cudaStreamSynchronize(st), "sah sync");
   }
   if (s == RMG_OK && h.bad_face) s = fail(RMG_ERR_INVALID_ARG, "rmg_map_build: face index out of range");
   if (s == RMG_OK && h.bad) s = fail(RMG_ERR_CUDA, "SAH build: partition disagrees with the split counts");

@@ -199,7 +199,8 @@ void wide_free(rmg_map* m) {
 }
 
 // Builds the 4-wide tree of a map whose binary tree is complete (its depth
-// known).  Synchronises once.
+// known).  Synchronises once, or twice for a tree whose wide levels descend less
+// than two binary ones each.
 int wide_build(rmg_map* m, cudaStream_t st) {
   wide_free(m);
   if (m->n_faces == 0) return RMG_OK;
@@ -220,16 +221,21 @@ int wide_build(rmg_map* m, cudaStream_t st) {
   h.end[1] = 1;
   if (s == RMG_OK) s = cuda_status(cudaMemsetAsync(bin_of, 0, 4, st), "wide init");
   if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(B, &h, sizeof h, cudaMemcpyHostToDevice, st), "wide init");
-  // every wide level descends at least one binary level
+  // Every wide level descends at least one binary level, most descend two: half the
+  // depth and two more are launched before the host looks whether nodes are left
+  // (a launch that finds none takes 2 us, an early look 10).
   const int levels = (int)std::min<unsigned>(std::max(m->depth, 1u), (unsigned)kMaxLevels4);
-  for (int l = 0; s == RMG_OK && l < levels; ++l) {
-    const uint64_t most = std::min<uint64_t>(cap, 1ull << std::min(2 * l, 62));
-    const unsigned grid = (unsigned)std::min<uint64_t>((most + kBlock4 - 1) / kBlock4, 4ull * device_sm_count());
-    k_collapse<<<grid, kBlock4, 0, st>>>(m->d_nodes, bin_of, B, l, cap, m->d_nodes4, m->d_src4);
-    s = cuda_status(cudaGetLastError(), "k_collapse");
+  for (int l = 0, upto = std::min(levels, levels / 2 + 2); s == RMG_OK && l < levels; upto = levels) {
+    for (; s == RMG_OK && l < upto; ++l) {
+      const uint64_t most = std::min<uint64_t>(cap, 1ull << std::min(2 * l, 62));
+      const unsigned grid = (unsigned)std::min<uint64_t>((most + kBlock4 - 1) / kBlock4, 4ull * device_sm_count());
+      k_collapse<<<grid, kBlock4, 0, st>>>(m->d_nodes, bin_of, B, l, cap, m->d_nodes4, m->d_src4);
+      s = cuda_status(cudaGetLastError(), "k_collapse");
+    }
+    if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "wide count");
+    if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "wide sync");
+    if (h.end[l + 1] == h.end[l]) break;
   }
-  if (s == RMG_OK) s = cuda_status(cudaMemcpyAsync(&h, B, sizeof h, cudaMemcpyDeviceToHost, st), "wide count");
-  if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "wide sync");
   if (s == RMG_OK && h.count > cap) s = fail(RMG_ERR_CUDA, "wide build: node count exceeds the binary tree");
   pool_free(bin_of, st);
   pool_free(B, st);
@@ -240,7 +246,7 @@ int wide_build(rmg_map* m, cudaStream_t st) {
   }
   // a tree deeper than kMaxLevels4 keeps no 4-wide form (its walk takes at most
   // 21 levels anyway, see have_wide4)
-  if (h.end[levels + 1] != h.end[levels]) { wide_free(m); return RMG_OK; }
+  if (h.end[h.levels + 1] != h.end[h.levels]) { wide_free(m); return RMG_OK; }
   m->n_nodes4 = h.count;
   m->depth4 = h.levels;
   return RMG_OK;

@@ -55,3 +55,29 @@ def test_vertices_that_are_not_finite(n):
         assert m.status() == 0
     for a, t in got[0].items():
         assert torch.equal(t.view(torch.uint8), got[1][a].view(torch.uint8)), a
+
+
+@pytest.mark.parametrize("n", [600, 1500, 6000])
+@pytest.mark.parametrize("builder", ["sah", "lbvh"])
+def test_trees_with_more_levels_than_a_balanced_one(n, builder):
+    """A dense cluster and 80 triangles at growing distances from it: splits take off a few distant
+    triangles each, so the cluster stays large, and nodes stay to be collapsed, for many levels."""
+    rng = np.random.default_rng(n)
+    c = rng.standard_normal((n, 1, 3)) * 0.1
+    c[:80, 0, 0] = 1.3 ** np.arange(80)
+    c[40:80, 0, 1] = 1.2 ** np.arange(40)
+    v = (c + 0.05 * rng.standard_normal((n, 3, 3))).reshape(-1, 3).astype(np.float32)
+    f = np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+    m = rm.Map(v, f, builder=builder)
+    if builder == "sah":
+        _check_tree(m, v, f)
+    sim = rm.SphereSimulator(m)
+    sim.setModel(sensors.vlp16_360())
+    poses = torch.from_numpy(scenes.room_poses(4, seed=1)).cuda()
+    got = []
+    for width in (0, 2):
+        sim.launch_config = rm.launch_config(bvh_width=width, packet=0)
+        got.append(sim.simulate(poses, attrs=("hits", "ranges", "face_ids")).tensors())
+    assert m.status() == 0
+    for a, t in got[0].items():
+        assert torch.equal(t.view(torch.uint8), got[1][a].view(torch.uint8)), a
