@@ -126,7 +126,8 @@ typedef struct rmg_launch_config {
   uint32_t bvh_width;     /* 2: walk the binary tree; 4: the 4-wide tree collapsed from it; 8: the 8-wide
                              tree with quantized boxes collapsed from it (4 and 8 when the map has the tree
                              and refill == 0); 0: the default, the 4-wide tree where it can be walked, unless
-                             refill, packet == 1 or a stack_depth other than 16 asks for the binary one.
+                             refill, packet == 1 or a stack_depth other than 16 asks for the binary one
+                             (and with no configuration at all, the faster of the two for the launch).
                              Results are identical. */
   uint32_t packet;        /* 1: the warp walks the binary tree together (a node is visited when any of
                              its 32 rays needs it; refill == 0, bvh_width != 4); 0: each ray walks alone;

@@ -86,3 +86,19 @@ def test_gradient_and_correction_of_few_rays(world, name):
         assert torch.equal(g, g0[:n]) and torch.equal(l, l0[:n])
         st, _ = sim.simulate_statistics(poses[:n].contiguous(), scan[:n].contiguous(), dataset_mask=mask[:n].contiguous())
         assert torch.equal(st.view(torch.int32), st0[:n].view(torch.int32))
+
+
+@pytest.mark.parametrize("poses", [14, 40, 41])
+def test_walk_by_launch_size_gives_the_same_bytes(poses):
+    """On a small map, launches of 16 rays a warp, just inside and just outside of 48 warps per SM
+    (152 SMs, 180 tiles a pose): the walk that the library picks, the binary and the 4-wide one."""
+    sc = scenes.box_room(seed=6, n_boxes=60)
+    sim = rm.make_simulator(sensors.vlp16_360(), rm.Map(sc.vertices, sc.faces))
+    T = torch.from_numpy(scenes.room_poses(poses, seed=3)).cuda()
+    got = []
+    for cfg in (None, rm.launch_config(bvh_width=2, packet=0), rm.launch_config(bvh_width=4)):
+        sim.launch_config = cfg
+        got.append(sim.simulate(T, attrs=("hits", "ranges", "points", "normals", "face_ids")).tensors())
+    for other in got[1:]:
+        for a, t in got[0].items():
+            assert torch.equal(t.view(torch.uint8), other[a].view(torch.uint8)), a
