@@ -128,12 +128,22 @@ __device__ __forceinline__ bool too_deep(uint32_t depth, uint32_t l, uint32_t r)
   return depth + 1 + ceil_log2(l) > kMaxDepth || depth + 1 + ceil_log2(r) > kMaxDepth;
 }
 
-// A child's box in its parent's record.
+// A child's box in its parent's record.  A coordinate that is NaN in every
+// vertex below the child has an empty interval here (see k_prep) and is NaN in
+// the record, as a refit leaves it.
 __device__ __forceinline__ void write_box(Node* nodes, int parent, uint32_t side, const float lo[3], const float hi[3]) {
   Node* p = nodes + parent;
-  const float4 xy = make_float4(lo[0], hi[0], lo[1], hi[1]);
+  const float nan = __int_as_float(0x7fffffff);
+  float l[3], h[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const bool empty = lo[k] > hi[k];
+    l[k] = empty ? nan : lo[k];
+    h[k] = empty ? nan : hi[k];
+  }
+  const float4 xy = make_float4(l[0], h[0], l[1], h[1]);
   if (side == 0) p->a = xy; else p->b = xy;
-  reinterpret_cast<float2*>(&p->c)[side] = make_float2(lo[2], hi[2]);
+  reinterpret_cast<float2*>(&p->c)[side] = make_float2(l[2], h[2]);
 }
 
 // Links of one node whose task covers `count` triangles from position `first`,
@@ -252,7 +262,11 @@ __device__ __forceinline__ Choice warp_split(const int* bins, uint32_t count, ui
 
 // ---- large tasks ---------------------------------------------------------------------
 
-// Boxes and ids of all triangles; bounds of their box centres.
+// Boxes and ids of all triangles; bounds of their box centres.  A coordinate that
+// is NaN in all three vertices gets the empty interval (+inf, -inf): the bins'
+// order-preserving integers would take a NaN for the largest of numbers, while
+// every minimum and maximum passes over an empty interval, as fminf and fmaxf
+// pass over a NaN.  (Its centre is NaN still, and falls into bin 0.)
 __global__ void __launch_bounds__(kBlk) k_prep(const float* v, uint32_t n_vertices, const uint32_t* f, uint32_t n, Rec* rec,
                                                Build* B) {
   __shared__ int sb[6];
@@ -269,6 +283,9 @@ __global__ void __launch_bounds__(kBlk) k_prep(const float* v, uint32_t n_vertic
     r.a = make_float4(fminf(fminf(a.x, b.x), d.x), fminf(fminf(a.y, b.y), d.y), fminf(fminf(a.z, b.z), d.z),
                       __uint_as_float(i));
     r.b = make_float4(fmaxf(fmaxf(a.x, b.x), d.x), fmaxf(fmaxf(a.y, b.y), d.y), fmaxf(fmaxf(a.z, b.z), d.z), 0.f);
+    if (isnan(r.a.x)) { r.a.x = INFINITY; r.b.x = -INFINITY; }
+    if (isnan(r.a.y)) { r.a.y = INFINITY; r.b.y = -INFINITY; }
+    if (isnan(r.a.z)) { r.a.z = INFINITY; r.b.z = -INFINITY; }
     rec[i] = r;
     const float3 c = centre(r.a, r.b);
     cl[0] = fminf(cl[0], c.x); cl[1] = fminf(cl[1], c.y); cl[2] = fminf(cl[2], c.z);
