@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P)
   const uint32_t c = blockIdx.x - b * P.chunks;
   const uint64_t base = (uint64_t)b * P.n_per;
   const uint32_t lo = c * P.chunk_len;
-  const uint32_t hi = min(P.n_per, lo + P.chunk_len);
+  const uint32_t hi = lo + min(P.n_per - lo, P.chunk_len);  // lo < n_per, see fill_params
   const Tf pre = batch_pre(P, b);
   // per-batch shift: first correspondence of the batch (any value works; it only
   // keeps the binary32 partial sums small)
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P)
     // neighbours of other batches, which are skipped, and the array's last group
     // is read one by one if it is cut short.
     const uint64_t e0 = base + lo, e1 = base + hi, total = (uint64_t)P.n_batches * P.n_per;
-    const uint64_t g0 = e0 / 4, g1 = lo < hi ? (e1 + 3) / 4 : g0;
+    const uint64_t g0 = e0 / 4, g1 = lo < hi ? (e1 + 3) / 4 : g0;  // (none in a batch of nothing)
     int run = 0;
     // warp-uniform trip count (lanes past the end skip the loads)
     const uint32_t iters = (uint32_t)((g1 - g0 + blockDim.x - 1) / blockDim.x);
@@ -236,10 +236,10 @@ __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P)
     }
   } else {
     int run = 0;
-    const uint32_t iters = (hi - lo + blockDim.x - 1) / blockDim.x;
+    const uint32_t len = hi - lo, iters = (uint32_t)(((uint64_t)len + blockDim.x - 1) / blockDim.x);
     for (uint32_t it = 0; it < iters; ++it) {
-      const uint32_t j = lo + threadIdx.x + it * blockDim.x;
-      if (j < hi) {
+      const uint32_t k = threadIdx.x + it * blockDim.x, j = lo + k;
+      if (k < len) {
         V D, M;
         const V np = P2L ? ldv(P.mn, base + j) : zero;
         if (correspondence<P2L, PRE>(P, pre, base + j, ldv(P.dp, base + j), ldv(P.mp, base + j), np, D, M))
@@ -362,15 +362,15 @@ __global__ void __launch_bounds__(kStatsThreads) k_umeyama_bwd_stream(const BwdP
   const uint32_t c = blockIdx.x - b * P.chunks;
   const uint64_t base = (uint64_t)b * P.n_per;
   const uint32_t lo = c * P.chunk_len;
-  const uint32_t hi = min(P.n_per, lo + P.chunk_len);
+  const uint32_t hi = lo + min(P.n_per - lo, P.chunk_len);  // lo < n_per, see fill_params
   const Tf pre = batch_pre(P, b);
   const Q preinv = qconj(pre.R);
   __shared__ Coef cf;
   if (threadIdx.x == 0) cf = B.coef[b];
   __syncthreads();
   const V zero{0.f, 0.f, 0.f};
-  for (uint32_t j = lo + threadIdx.x; j < hi; j += blockDim.x) {
-    const uint64_t i = base + j;
+  for (uint32_t j = threadIdx.x; j < hi - lo; j += blockDim.x) {
+    const uint64_t i = base + lo + j;
     V D, M;
     const bool ok = correspondence<false>(P, pre, i, ldv(P.dp, i), ldv(P.mp, i), zero, D, M);
     float gm[3] = {0.f, 0.f, 0.f}, gdv[3] = {0.f, 0.f, 0.f};
@@ -415,13 +415,14 @@ int fill_params(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
     chunks = std::min<uint32_t>((target + n_batches - 1) / n_batches, (n_per + 4095) / 4096);
     chunks = std::max<uint32_t>(chunks, 1);
   }
-  P.chunks = chunks;
-  P.chunk_len = ((n_per + chunks - 1) / chunks + 3) & ~3u;
+  // a multiple of four each, so fewer may do: none starts past the batch
+  P.chunk_len = (uint32_t)((((uint64_t)n_per + chunks - 1) / chunks + 3) & ~3ull);
+  P.chunks = n_per ? (uint32_t)(((uint64_t)n_per + P.chunk_len - 1) / P.chunk_len) : 1;
   P.partial = nullptr;
   P.counters = nullptr;
   P.dstats = nullptr;
   P.stats = nullptr;
-  if ((uint64_t)n_batches * chunks > 0x7fffffffull) return fail(RMG_ERR_INVALID_ARG, "statistics: too many batches");
+  if ((uint64_t)n_batches * P.chunks > 0x7fffffffull) return fail(RMG_ERR_INVALID_ARG, "statistics: too many batches");
   return RMG_OK;
 }
 
