@@ -36,6 +36,12 @@ constexpr int kStatsThreads = 256;
 // there are.
 constexpr int kSolveThreads = 32;
 unsigned solve_grid(uint32_t n) { return (unsigned)((4ull * n + kSolveThreads - 1) / kSolveThreads); }
+
+// The problem of this thread's group of four (a thread's index times the grid may
+// not fit 32 bits; the problems' number does, but for the last CTA's excess).
+__host__ __device__ __forceinline__ uint64_t solve_index(uint32_t cta, uint32_t thread) {
+  return (uint64_t)cta * (kSolveThreads / 4) + (thread >> 2);
+}
 constexpr int kFold = 8;  // vector groups (4 correspondences) per binary32 run
 
 struct StatsParams {
@@ -275,7 +281,8 @@ __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P)
 
 __global__ void __launch_bounds__(kSolveThreads) k_umeyama_dstats(const double* dstats, uint32_t n,
                                                                   rmg_transform* out) {
-  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, b = min(i, n - 1);
+  const uint64_t i = solve_index(blockIdx.x, threadIdx.x);
+  const uint32_t b = (uint32_t)min(i, (uint64_t)n - 1);
   const double* s = dstats + 16ull * b;
   M3d C;
   for (int i = 0; i < 3; ++i)
@@ -295,7 +302,8 @@ __device__ __forceinline__ void load_stats(const rmg_cross_stats& s, M3d& C, dou
 
 __global__ void __launch_bounds__(kSolveThreads) k_umeyama_stats(const rmg_cross_stats* stats, uint32_t n,
                                                                  rmg_transform* out) {
-  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, b = min(i, n - 1);
+  const uint64_t i = solve_index(blockIdx.x, threadIdx.x);
+  const uint32_t b = (uint32_t)min(i, (uint64_t)n - 1);
   const rmg_cross_stats s = stats[b];
   M3d C;
   double d[3], m[3], q[4], t[3];
@@ -314,7 +322,8 @@ struct Coef { float A[9], cm[3], B[9], cd[3]; };
 __global__ void __launch_bounds__(kSolveThreads) k_umeyama_bwd_coef(const rmg_cross_stats* stats, const float* grad_R,
                                                                     const float* grad_t, uint32_t n_batches,
                                                                     Coef* coef) {
-  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, b = min(i, n_batches - 1);
+  const uint64_t i = solve_index(blockIdx.x, threadIdx.x);
+  const uint32_t b = (uint32_t)min(i, (uint64_t)n_batches - 1);
   const int j = column4();
   const rmg_cross_stats s = stats[b];
   M3d C, U, V;
