@@ -285,7 +285,10 @@ __device__ __forceinline__ void umeyama_lanes(const M3d& C, const double d[3], c
   row_of(R, j, r);
   const double x = pick(j, m[0], m[1], m[2]) - dot(r, d);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) t[k] = n == 0 ? 0.0 : of4(x, k);
+  for (int k = 0; k < 3; ++k) {
+    const double tk = of4(x, k);  // every lane of the warp takes part, whatever its own n
+    t[k] = n == 0 ? 0.0 : tk;
+  }
 }
 
 // Gradient of L through R = U V^T (C = U diag(s) V^T, rotations U, V):
