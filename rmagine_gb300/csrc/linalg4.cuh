@@ -121,9 +121,12 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   double v[3], y[3], z[3];  // this lane's column of V, the columns n1 and n2
   double d, off, g;         // elements (j, j) and (j, n1) of A in V's frame, and the gap of their eigenvalues
   float X, fg;
-  // One pass, and up to two more for the warps with small eigenvalues closer than a
+  // One pass, and up to two more for the groups with small eigenvalues closer than a
   // first binary32 frame tells apart: A in that frame is graded, and the next
-  // frame's binary32 angles are good relative to those eigenvalues.
+  // frame's binary32 angles are good relative to those eigenvalues.  The warp's
+  // other groups keep their frame meanwhile and form the same numbers from it again,
+  // so that a problem's result does not depend on its neighbours.
+  bool again = true;
 #pragma unroll 1
   for (int pass = 0;; ++pass) {
     float w0[3] = {1.f, 0.f, 0.f}, w1[3] = {0.f, 1.f, 0.f}, w2[3] = {0.f, 0.f, 1.f};
@@ -147,7 +150,10 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
       for (int k = 0; k < 3; ++k) v[k] = r[k];
     } else {
       const M3d old = gather4(v);
-      mul_col(old, r, v);
+      double turned[3];
+      mul_col(old, r, turned);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = again ? turned[k] : v[k];
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) { y[k] = of4(v[k], n1); z[k] = of4(v[k], n2); }
@@ -160,17 +166,23 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
     const float fo = (float)off;
     X = fo == 0.0f ? 0.0f : fo / fg;  // X_(j, n1)
     bool far = !(fabsf(X) < 4e-6f);   // third-order terms up to here are below binary64's rounding
-    if (far && fabsf(fo) <= 4e-16f) {  // equal eigenvalues, diagonal to binary64's rounding of A
+    // Equal eigenvalues, diagonal to binary64's rounding of A.  Leaving `off` turns the
+    // rotation sought by off / (2 d); small eigenvalues get their frames first (singular
+    // values 1, 1e-7, 1e-7 left at once: mean error 8.7e-4, so 2.7e-4, by one thread 3.4e-4).
+    if (far && fabsf(fo) <= 4e-16f && (d > 1e-2 || pass == 2)) {
       far = false;
       X = 0.0f;
     }
-    if (pass == 2 || !__any_sync(0xffffffffu, far && !bad)) {
+    const int away = far && !bad ? 1 : 0;
+    again = (of4(away, 0) | of4(away, 1) | of4(away, 2)) != 0;
+    if (pass == 2 || !__any_sync(0xffffffffu, again)) {
       bad = bad || far;
       break;
     }
     const float fd = (float)d;
     f00 = of4(fd, 0); f11 = of4(fd, 1); f22 = of4(fd, 2);
     f01 = of4(fo, 0); f12 = of4(fo, 1); f02 = of4(fo, 2);
+    if (!again) f01 = f12 = f02 = 0.0f;
   }
   {
     const float Xa = of4(X, n1), Xb = of4(X, n2), ga = of4(fg, n1), gb = of4(fg, n2);
