@@ -97,8 +97,22 @@ __device__ __forceinline__ void quat_f(const float w0[3], const float w1[3], con
   for (int k = 0; k < 4; ++k) q[k] *= r;
 }
 
+// Whether any lane of a group says so, in its lanes.
+__device__ __forceinline__ bool any4(bool x) {
+  return (__ballot_sync(0xffffffffu, x) >> (threadIdx.x & 28) & 15u) != 0;
+}
+
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+
 // svd3_rot of the same C in the four lanes of a group; U, s and V in all of them.
-__device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3d& V) {
+// True if the whole warp's are zero (U and V the identity then).
+// Where A = C^T C is diagonal (no correspondences, one, a line along an axis) its
+// frame is the identity and needs no pass, which a warp of such problems leaves
+// out, and svd3_rot's choices for a rank of one and zero are made here: svd3_rot
+// itself takes eight problems to a warp here, where one thread each has 32.
+// 40,000 zero matrices (transform alone) 91 -> 19 us, one thread each 37; of rank
+// one along an axis 111 -> 51, one thread each 51 (of 400,000 989 -> 444 and 332).
+__device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3d& V) {
   const int j = column4(), n1 = j == 2 ? 0 : j + 1, n2 = 3 - j - n1;
   // column j of A, times the power of two that brings its largest diagonal element to [1, 2)
   double a[3];
@@ -110,8 +124,17 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   }
   int e = __double2hiint(pick(j, a[0], a[1], a[2])) & 0x7ff00000;
   e = max(max(of4(e, 0), of4(e, 1)), of4(e, 2));
-  bool bad = e < (64 << 20) || e > (1983 << 20);  // (NaN and infinity have the largest exponent)
-  const double scale = __hiloint2double(bad ? 0x3ff00000 : (2046 << 20) - e, 0);
+  // (no exchange inside a choice: every lane of the warp takes part in all of them)
+  const bool mixed = any4(!is_zero(pick(j, a[1], a[2], a[0])) || !is_zero(pick(j, a[2], a[0], a[1])));
+  const bool some = any4(!is_zero(pick(j, a[0], a[1], a[2])));
+  const bool diagonal = !mixed, zero = !mixed && !some;
+  if (__all_sync(0xffffffffu, zero)) {
+    U = V = m3_eye();
+    s[0] = s[1] = s[2] = 0.0;
+    return true;
+  }
+  bool bad = !zero && (e < (64 << 20) || e > (1983 << 20));  // (NaN and infinity have the largest exponent)
+  const double scale = __hiloint2double(bad || zero ? 0x3ff00000 : (2046 << 20) - e, 0);
 #pragma unroll
   for (int i = 0; i < 3; ++i) a[i] *= scale;
 
@@ -127,8 +150,9 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   // other groups keep their frame meanwhile and form the same numbers from it again,
   // so that a problem's result does not depend on its neighbours.
   bool again = true;
+  const bool passes = !__all_sync(0xffffffffu, diagonal || bad);
 #pragma unroll 1
-  for (int pass = 0;; ++pass) {
+  for (int pass = 0; passes; ++pass) {
     float w0[3] = {1.f, 0.f, 0.f}, w1[3] = {0.f, 1.f, 0.f}, w2[3] = {0.f, 0.f, 1.f};
     const float tol = pass == 0 ? 1e-13f : 1e-34f;
 #pragma unroll 1
@@ -169,14 +193,13 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
     // Equal eigenvalues, diagonal to binary64's rounding of A.  Leaving `off` turns the
     // rotation sought by off / (2 d); small eigenvalues get their frames first (singular
     // values 1, 1e-7, 1e-7 left at once: mean error 8.7e-4, so 2.7e-4, by one thread 3.4e-4).
-    if (far && fabsf(fo) <= 4e-16f && (d > 1e-2 || pass == 2)) {
+    if (far && fabsf(fo) <= 4e-16f && (__double2hiint(d) >= 0x3f800000 || pass == 2)) {  // d >= 2^-7
       far = false;
       X = 0.0f;
     }
-    const int away = far && !bad ? 1 : 0;
-    again = (of4(away, 0) | of4(away, 1) | of4(away, 2)) != 0;
+    again = any4(far && !bad && !diagonal);
     if (pass == 2 || !__any_sync(0xffffffffu, again)) {
-      bad = bad || far;
+      bad = bad || (far && !diagonal);
       break;
     }
     const float fd = (float)d;
@@ -184,16 +207,20 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
     f01 = of4(fo, 0); f12 = of4(fo, 1); f02 = of4(fo, 2);
     if (!again) f01 = f12 = f02 = 0.0f;
   }
-  {
+  if (passes) {
     const float Xa = of4(X, n1), Xb = of4(X, n2), ga = of4(fg, n1), gb = of4(fg, n2);
     const float rest = (float)(off - g * (double)X) + 0.5f * Xa * Xb * (ga - gb);
     const float Xc = fabsf(rest) <= 4e-16f && !(fabsf(rest) < 1e-8f * fabsf(fg)) ? 0.0f : rest / fg;
-    bad = bad || !(fabsf(Xc) < 1e-8f);
+    bad = bad || (!(fabsf(Xc) < 1e-8f) && !diagonal);
     const float Xcb = of4(Xc, n2);
     const double p0 = -0.5f * (X * X + Xb * Xb), p1 = (double)(0.5f * Xa * Xb - Xc) - (double)X,
                  p2 = (double)(0.5f * Xa * X + Xcb) + (double)Xb;
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] += p0 * v[k] + p1 * y[k] + p2 * z[k];
+  }
+  if (diagonal || !passes) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = k == j ? 1.0 : 0.0;
   }
   // B = C V: columns s_i u_i; the columns in the order of their lengths, V right-handed
   double B[3];
@@ -224,8 +251,18 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   const double d01 = dot(u0, u1);
 #pragma unroll
   for (int k = 0; k < 3; ++k) u1[k] -= d01 * u0[k];
-  const double q1 = dot(u1, u1);
-  bad = bad || !(q1 > 1e-24 * q0);
+  double q1 = dot(u1, u1);
+  if (!(q1 > 1e-24 * q0)) {
+    if (!diagonal) {
+      bad = true;
+    } else {  // rank one: any unit vector orthogonal to u0
+      const int k = (fabs(u0[0]) <= fabs(u0[1]) && fabs(u0[0]) <= fabs(u0[2])) ? 0 : (fabs(u0[1]) <= fabs(u0[2]) ? 1 : 2);
+      const double u0k = pick(k, u0[0], u0[1], u0[2]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) u1[i] = (i == k ? 1.0 : 0.0) - u0k * u0[i];
+      q1 = dot(u1, u1);
+    }
+  }
   const double i1 = rsqrt(q1);
 #pragma unroll
   for (int k = 0; k < 3; ++k) u1[k] *= i1;
@@ -240,8 +277,12 @@ __device__ __forceinline__ void svd3_lanes(const M3d& C, M3d& U, double s[3], M3
     U.a[k][0] = u0[k]; U.a[k][1] = u1[k]; U.a[k][2] = u2[k];
     s[k] = of4(sj, k);
   }
-  const int any = bad ? 1 : 0;
-  if (of4(any, 0) | of4(any, 1) | of4(any, 2)) svd3_rot(C, U, s, V);
+  if (any4(bad)) svd3_rot(C, U, s, V);
+  if (zero) {
+    U = V;
+    s[0] = s[1] = s[2] = 0.0;
+  }
+  return false;
 }
 
 // R = U V^T in all lanes.
@@ -284,11 +325,14 @@ __device__ __forceinline__ void umeyama_lanes(const M3d& C, const double d[3], c
                                               double q[4], double t[3]) {
   M3d U, V;
   double s[3];
-  svd3_lanes(C, U, s, V);
-  M3d R = rotation_lanes(U, V);
-  rot_to_quat_lanes(R, q);
-  const bool finite = isfinite(q[0]) && isfinite(q[1]) && isfinite(q[2]) && isfinite(q[3]);
-  if (n == 0 || !finite) {
+  M3d R = m3_eye();
+  bool identity = svd3_lanes(C, U, s, V);
+  if (!identity) {  // the whole warp's
+    R = rotation_lanes(U, V);
+    rot_to_quat_lanes(R, q);
+    identity = n == 0 || !(isfinite(q[0]) && isfinite(q[1]) && isfinite(q[2]) && isfinite(q[3]));
+  }
+  if (identity) {
     R = m3_eye();
     q[0] = q[1] = q[2] = 0.0; q[3] = 1.0;
   }
