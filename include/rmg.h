@@ -328,9 +328,14 @@ typedef struct rmg_batch_entry {
 } rmg_batch_entry;
 
 typedef struct rmg_batch_config {
-  uint32_t stack_depth;  /* 0, 8 or 16 */
+  uint32_t stack_depth;  /* 8, the default: the 4-wide tree where it can be walked; 16: the binary tree with a
+                            full stack; 0: the binary tree with restarts.  (8 and 16 are the short stack of a
+                            tree too deep for these.)  Results are identical. */
   uint32_t block_warps;  /* 1..8 */
-  uint32_t tile_w;       /* tile of a 2-D sensor, tile_w * tile_h == 32; 1-row sensors use 32 x 1 */
+  uint32_t tile_w;       /* tile of a 2-D sensor, tile_w * tile_h == 32; 1-row sensors use 32 x 1.  While tile_w,
+                            tile_h and grab all have their defaults (8, 4, 2) they are left to the library: plans
+                            of few rays take tiles of 4 to 16 rays, and warps take one tile at a time unless
+                            there are many; a configuration that sets any of them is taken literally. */
   uint32_t tile_h;
   uint32_t grab;         /* tiles a warp takes from the work counter at a time, 1..64 */
   uint32_t ctas_per_sm;  /* 0 = as many as fit */

@@ -209,6 +209,34 @@ int check_batch_config(const rmg_batch_config& c) {
   return RMG_OK;
 }
 
+rmg_batch_config default_batch_config() {
+  rmg_batch_config c;
+  c.stack_depth = 8;
+  c.block_warps = 4;
+  c.tile_w = 8;
+  c.tile_h = 4;
+  c.grab = 2;
+  c.ctas_per_sm = 0;
+  c.use_graph = 1;
+  return c;
+}
+
+// Whether the tiles and the tiles per fetch are left to the library: a
+// configuration that sets any of the three is taken literally.
+bool own_tiles(const rmg_batch_config& c) {
+  const rmg_batch_config d = default_batch_config();
+  return c.tile_w == d.tile_w && c.tile_h == d.tile_h && c.grab == d.grab;
+}
+
+// The walk of a plan, as kernel_ptr takes it: the default's stack depth is the
+// 4-wide tree, 16 the binary one with a full stack, 0 (and trees too deep for
+// either) the short-stack walk.  512 sensors, 590,000 rays: 193, 208 and 345 us.
+int batch_walk(const rmg_batch* b) {
+  if (b->cfg.stack_depth == default_batch_config().stack_depth && have_wide4(b->map)) return kWideTB;
+  if (b->cfg.stack_depth > 0 && b->map->depth <= (unsigned)kFullStack) return 0;
+  return trail_bits_for_depth(b->map->depth);
+}
+
 // (Re)builds the device job table for the plan's tile shape.
 int build_jobs(rmg_batch* b) {
   b->jobs_h.clear();
@@ -217,7 +245,7 @@ int build_jobs(rmg_batch* b) {
   // few rays: tiles of 4 to 16 (see lanes_for).  24,600 rays of 64 scattered and
   // camera sensors on a 30,000-triangle terrain: 79 us with whole warps, 56 so;
   // 590,000 rays keep whole warps (231 us, 272 with 16).
-  const uint32_t lanes = lanes_for(rays);
+  const uint32_t lanes = own_tiles(b->cfg) ? lanes_for(rays) : 32;
   for (const rmg_batch_entry& e : b->entries) {
     JobDev J;
     std::memset(&J, 0, sizeof(J));
@@ -267,15 +295,16 @@ BatchParams params(const rmg_batch* b, uint64_t warps) {
   B.n_jobs = (uint32_t)b->jobs_h.size();
   B.total_tiles = b->total_tiles;
   B.counter = b->counter;
-  // A warp takes `grab` tiles at a time only where there are many times as many:
-  // a tile of scattered rays lasts 60 us, and 3.4 tiles for each warp in twos make
-  // four (590,000 rays of 512 sensors: 266 -> 231 us; 161,000
+  // Left to the library, a warp takes `grab` tiles at a time only where there are
+  // many times as many: a tile of scattered rays lasts 60 us, and 3.4 tiles for each
+  // warp in twos make four (590,000 rays of 512 sensors: 266 -> 231 us; 161,000
   // rays 165 -> 103).
-  B.grab = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(b->cfg.grab, b->total_tiles / (16 * warps)));
+  B.grab = b->cfg.grab;
+  if (own_tiles(b->cfg)) B.grab = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(B.grab, b->total_tiles / (16 * warps)));
   B.budget = 2u * b->map->n_nodes + 64u;
   B.trail_bits = trail_bits_for_depth(b->map->depth);
   B.full_stack = b->map->depth <= (unsigned)kFullStack ? 1 : 0;
-  B.wide = have_wide4(b->map) ? 1 : 0;
+  B.wide = batch_walk(b) == kWideTB ? 1 : 0;
   return B;
 }
 
@@ -283,10 +312,7 @@ BatchParams params(const rmg_batch* b, uint64_t warps) {
 int launch_direct(rmg_batch* b, cudaStream_t st) {
   if (b->total_tiles == 0) return RMG_OK;
   unsigned grid = 0;
-  const bool stack = b->cfg.stack_depth > 0;
-  const bool full = stack && b->map->depth <= (unsigned)kFullStack;
-  int s = persistent_grid(b->cfg, stack && have_wide4(b->map) ? kWideTB
-                                  : full ? 0 : trail_bits_for_depth(b->map->depth), grid);
+  int s = persistent_grid(b->cfg, batch_walk(b), grid);
   if (s != RMG_OK) return s;
   RMG_CUDA_TRY(cudaMemsetAsync(b->counter, 0, sizeof(unsigned long long), st));
   return cuda_status(launch_batched(params(b, (uint64_t)grid * b->cfg.block_warps), (int)b->cfg.stack_depth, grid, 32u * b->cfg.block_warps, st),
@@ -315,13 +341,7 @@ using namespace rmg;
 extern "C" int rmg_batch_default_config(rmg_batch_config* cfg) {
   return guarded("rmg_batch_default_config", [&]() -> int {
     if (!cfg) return fail(RMG_ERR_INVALID_ARG, "rmg_batch_default_config: NULL");
-    cfg->stack_depth = 8;
-    cfg->block_warps = 4;
-    cfg->tile_w = 8;
-    cfg->tile_h = 4;
-    cfg->grab = 2;
-    cfg->ctas_per_sm = 0;
-    cfg->use_graph = 1;
+    *cfg = default_batch_config();
     return RMG_OK;
   });
 }
