@@ -114,7 +114,10 @@ typedef struct rmg_outputs {
   uint32_t* object_ids;
 } rmg_outputs;
 
-/* Traversal launch options (the knobs the autotuner searches). */
+/* Traversal launch options (the knobs the autotuner searches).  A configuration
+ * that is rmg_default_launch_config's in every field leaves the launch to the
+ * library, as none does: small launches then take fewer rays per warp, and the
+ * binary walk where it is the faster one. */
 typedef struct rmg_launch_config {
   uint32_t stack_depth;   /* short-stack entries per ray: 0 (stackless, parent pointers), 8 or 16 */
   uint32_t block_warps;   /* warps per CTA */
@@ -122,12 +125,13 @@ typedef struct rmg_launch_config {
   uint32_t tile_h;        /* tile_w * tile_h must be 32 */
   uint32_t refill;        /* 0: one tile per warp.  1..32: persistent warps that hand new rays to
                              idle lanes whenever fewer than `refill` lanes are busy (stack_depth 8 or 16) */
-  uint32_t chunk;         /* refill mode: tiles a warp takes from the work counter at a time (>= 1) */
+  uint32_t chunk;         /* refill mode: tiles a warp takes from the work counter at a time (>= 1);
+                             otherwise 0 leaves the rays per warp to the library (packet != 1): small
+                             launches take 4 to 16, in tiles of the given shape cut down */
   uint32_t bvh_width;     /* 2: walk the binary tree; 4: the 4-wide tree collapsed from it; 8: the 8-wide
                              tree with quantized boxes collapsed from it (4 and 8 when the map has the tree
                              and refill == 0); 0: the default, the 4-wide tree where it can be walked, unless
-                             refill, packet == 1 or a stack_depth other than 16 asks for the binary one
-                             (and with no configuration at all, the faster of the two for the launch).
+                             refill, packet == 1 or a stack_depth other than 16 asks for the binary one.
                              Results are identical. */
   uint32_t packet;        /* 1: the warp walks the binary tree together (a node is visited when any of
                              its 32 rays needs it; refill == 0, bvh_width != 4); 0: each ray walks alone;
@@ -302,7 +306,7 @@ int rmg_host_set_points_policy(uint32_t policy);
  * library's memory pool (maps, scratch, workspaces) keeps unused. */
 int rmg_host_staging_trim(void);
 
-/* Times a fixed set of launch configurations (per-ray binary walk, warp
+/* Times the default launch and a fixed set of configurations (per-ray binary walk, warp
  * packet walk, 4-wide walk; tiles 8x4, 16x2, 4x8; 4 or 2 warps per CTA) on
  * the caller's poses and output buffers -- all write the same results -- and
  * returns the fastest (median of `reps` runs after a warm-up).  Same pointer

@@ -29,6 +29,18 @@ int default_config(const rmg_sensor* s, rmg_launch_config* cfg) {
   return RMG_OK;
 }
 
+// Whether a configuration leaves the rays per warp to the library: the sensor's
+// default in every field (as no configuration at all), or chunk == 0 outside of
+// the refill mode.
+bool own_tiles(const rmg_launch_config& c, const rmg_sensor* s) {
+  rmg_launch_config d;
+  default_config(s, &d);
+  if (c.refill == 0 && c.chunk == 0 && c.packet != 1) return true;
+  return c.stack_depth == d.stack_depth && c.block_warps == d.block_warps && c.tile_w == d.tile_w &&
+         c.tile_h == d.tile_h && c.refill == d.refill && c.chunk == d.chunk && c.bvh_width == d.bvh_width &&
+         c.packet == d.packet;
+}
+
 int check_config(const rmg_launch_config& c) {
   if (!valid_stack_depth(c.stack_depth))
     return fail(RMG_ERR_UNSUPPORTED, "launch config: stack_depth must be 0, 8 or 16");
@@ -214,7 +226,7 @@ extern "C" int rmg_simulate_ex(const rmg_map* map, const rmg_sensor* sensor, con
         !out->geom_ids && !out->object_ids)
       return RMG_OK;  // nothing requested: the reference writes nothing either
     TraceParams P;
-    make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, cfg, P, cfg_in == nullptr);
+    make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, cfg, P, own_tiles(cfg, sensor));
     return launch_plain(P, sensor, cfg, as_stream(stream));
   });
 }
@@ -228,11 +240,13 @@ extern "C" int rmg_simulate(const rmg_map* map, const rmg_sensor* sensor, const 
 }
 
 // Launch autotuner for one (map, sensor, pose set): times a fixed list of
-// candidate configurations -- per-ray binary walk, warp packet walk and 4-wide
-// walk, each with three tile shapes and two CTA sizes -- on the caller's own
-// poses and output buffers (every candidate writes the same results) and
-// returns the fastest by median of `reps` timed runs after one warm-up run.
-// Synchronises.  No counterpart in the reference.
+// candidate configurations -- the per-ray binary and 4-wide walks with the rays
+// per warp left to the library (one of them is the default launch), and the
+// per-ray binary walk, warp packet walk and 4-wide and 8-wide walks, each with
+// three tile shapes and two CTA sizes -- on the caller's own poses and output
+// buffers (every candidate writes the same results) and returns the fastest by
+// median of `reps` timed runs after one warm-up run.  Synchronises.  No
+// counterpart in the reference.
 extern "C" int rmg_autotune_launch_config(const rmg_map* map, const rmg_sensor* sensor, const rmg_transform* Tsb,
                                           const rmg_transform* Tbm, uint32_t n_poses, const rmg_outputs* out,
                                           uint32_t reps, rmg_launch_config* best, void* stream) {
@@ -243,18 +257,20 @@ extern "C" int rmg_autotune_launch_config(const rmg_map* map, const rmg_sensor* 
     cudaStream_t st = as_stream(stream);
     rmg_launch_config base;
     default_config(sensor, &base);
+    std::vector<rmg_launch_config> candidates;
+    for (uint32_t width : {4u, 2u}) {
+      rmg_launch_config c = base;
+      c.bvh_width = width;
+      c.packet = 0;
+      c.chunk = 0;
+      candidates.push_back(c);
+    }
     struct Walk { uint32_t bvh_width, packet; };
     const Walk walks[4] = {{2, 0}, {2, 1}, {4, 0}, {8, 0}};
     const uint32_t tiles[3][2] = {{8, 4}, {16, 2}, {4, 8}};
     const uint32_t warps[2] = {4, 2};
-    cudaEvent_t e0, e1;
-    RMG_CUDA_TRY(cudaEventCreate(&e0));
-    RMG_CUDA_TRY(cudaEventCreate(&e1));
-    float best_ms = 1e30f;
-    int s = RMG_OK;
-    bool any = false;
-    for (const Walk& w : walks) {
-      for (const auto& t : tiles) {
+    for (const Walk& w : walks)
+      for (const auto& t : tiles)
         for (uint32_t bw : warps) {
           rmg_launch_config c = base;
           c.bvh_width = w.bvh_width;
@@ -263,31 +279,35 @@ extern "C" int rmg_autotune_launch_config(const rmg_map* map, const rmg_sensor* 
           c.tile_h = t[1];
           c.block_warps = bw;
           if (c.tile_w > sensor->width && c.tile_w != base.tile_w) continue;
-          if (check_config(c) != RMG_OK) continue;
-          TraceParams P;
-          make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, c, P, false);
-          if ((w.bvh_width == 4 && !P.wide) || (w.bvh_width == 8 && !P.wide8) || (w.packet == 1 && !P.packet))
-            continue;  // not available here
-          s = launch_plain(P, sensor, c, st);
-          if (s != RMG_OK) break;
-          std::vector<float> ms;
-          for (uint32_t r = 0; r < reps && s == RMG_OK; ++r) {
-            s = cuda_status(cudaEventRecord(e0, st), "event");
-            if (s == RMG_OK) s = launch_plain(P, sensor, c, st);
-            if (s == RMG_OK) s = cuda_status(cudaEventRecord(e1, st), "event");
-            if (s == RMG_OK) s = cuda_status(cudaEventSynchronize(e1), "event sync");
-            float x = 0.f;
-            if (s == RMG_OK) s = cuda_status(cudaEventElapsedTime(&x, e0, e1), "event time");
-            ms.push_back(x);
-          }
-          if (s != RMG_OK) break;
-          std::sort(ms.begin(), ms.end());
-          const float med = ms[ms.size() / 2];
-          if (med < best_ms) { best_ms = med; *best = c; any = true; }
+          candidates.push_back(c);
         }
-        if (s != RMG_OK) break;
+    cudaEvent_t e0, e1;
+    RMG_CUDA_TRY(cudaEventCreate(&e0));
+    RMG_CUDA_TRY(cudaEventCreate(&e1));
+    float best_ms = 1e30f;
+    int s = RMG_OK;
+    bool any = false;
+    for (const rmg_launch_config& c : candidates) {
+      if (check_config(c) != RMG_OK) continue;
+      TraceParams P;
+      make_trace_params(map, sensor, Tsb, Tbm, n_poses, out, c, P, own_tiles(c, sensor));
+      if ((c.bvh_width == 4 && !P.wide) || (c.bvh_width == 8 && !P.wide8) || (c.packet == 1 && !P.packet))
+        continue;  // not available here
+      s = launch_plain(P, sensor, c, st);
+      std::vector<float> ms;
+      for (uint32_t r = 0; r < reps && s == RMG_OK; ++r) {
+        s = cuda_status(cudaEventRecord(e0, st), "event");
+        if (s == RMG_OK) s = launch_plain(P, sensor, c, st);
+        if (s == RMG_OK) s = cuda_status(cudaEventRecord(e1, st), "event");
+        if (s == RMG_OK) s = cuda_status(cudaEventSynchronize(e1), "event sync");
+        float x = 0.f;
+        if (s == RMG_OK) s = cuda_status(cudaEventElapsedTime(&x, e0, e1), "event time");
+        ms.push_back(x);
       }
       if (s != RMG_OK) break;
+      std::sort(ms.begin(), ms.end());
+      const float med = ms[ms.size() / 2];
+      if (med < best_ms) { best_ms = med; *best = c; any = true; }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
