@@ -19,6 +19,7 @@
 #include <thread>
 #include <vector>
 
+#include "chunks.h"
 #include "internal.h"
 
 namespace rmg {
@@ -95,28 +96,6 @@ rmg_outputs outputs_at(const AttrList& a) {
 }
 
 using Launch = std::function<int(const rmg_transform* Tbm, uint32_t n, const rmg_outputs* out, cudaStream_t st)>;
-
-// Pose chunks of the simulate host forms: full chunks of `chunk` poses, then
-// the last two chunks' worth split in halving sizes (at least chunk / 8 and
-// `least` poses), so that the work left after the final launch -- its copy, and
-// forming its points -- is a small chunk's.  Returns the first pose of every
-// chunk and n.
-std::vector<uint32_t> chunk_schedule(uint32_t n, size_t chunk, size_t least) {
-  std::vector<uint32_t> first{0};
-  uint64_t p = 0;
-  while (n - p > 2 * chunk) {
-    p += chunk;
-    first.push_back((uint32_t)p);
-  }
-  const uint64_t min_tail = std::max<uint64_t>(std::max<uint64_t>(1, least), chunk / 8);
-  while (p < n) {
-    const uint64_t rem = n - p;
-    const uint64_t take = rem <= min_tail ? rem : std::max<uint64_t>(min_tail, std::min<uint64_t>(chunk, (rem + 1) / 2));
-    p += take;
-    first.push_back((uint32_t)p);
-  }
-  return first;
-}
 
 // Points follow from the range of a ray (the attribute rules of
 // SphereSimulatorEmbree.tcc:104-249, as the traversal kernels write them): a
@@ -299,12 +278,10 @@ int host_pipeline(const char* what, const rmg_sensor* sensor, const rmg_transfor
     if (host.ptr[a]) bytes_per_ray += host.size[a];
   if (bytes_per_ray == 0 || rays_per_pose == 0) return RMG_OK;
   const size_t bytes_per_pose = bytes_per_ray * rays_per_pose;
-  // at least one pose, at most ceil(n/2) so that two chunks overlap, but no chunk
-  // below kLeastChunkBytes, unless the caller asks for smaller ones
+  // no chunk below kLeastChunkBytes but the last (see least_rest), unless the caller asks for smaller ones
   const size_t want = g_chunk_bytes.load();
   const size_t least = std::min(want, kLeastChunkBytes) / bytes_per_pose;
-  size_t chunk = std::max<size_t>(1, want / bytes_per_pose);
-  chunk = std::min<size_t>(chunk, std::max<size_t>(std::max<size_t>(1, (n_poses + 1) / 2), least));
+  const size_t chunk = chunk_poses(n_poses, want / bytes_per_pose, least);
   const std::vector<uint32_t> first = chunk_schedule(n_poses, chunk, least);  // chunk k: poses [first[k], first[k+1])
   const uint32_t n_chunks = (uint32_t)first.size() - 1;
   const int slots = (int)std::min<uint32_t>(kSlots, n_chunks);
