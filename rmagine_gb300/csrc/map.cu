@@ -354,7 +354,7 @@ int repack_and_refit(rmg_map* m, cudaStream_t st, const uint32_t* d_order) {
 }
 
 // The map's bounds from its root; waits for the stream.
-int update_info(rmg_map* m, cudaStream_t st) {
+[[nodiscard]] int update_info(rmg_map* m, cudaStream_t st) {
   for (int k = 0; k < 3; ++k) { m->lo[k] = INFINITY; m->hi[k] = -INFINITY; }
   if (m->n_faces == 0) return RMG_OK;
   Node root;
@@ -438,8 +438,8 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
     check(alloc_arrays(m, st));
     if (s == RMG_OK && n_faces == 0) {
       s = cuda_status(cudaStreamSynchronize(st), "sync");
+      if (s == RMG_OK) s = update_info(m, st);
       if (s != RMG_OK) { free_map(m); return s; }
-      update_info(m, st);
       *out = m;
       return RMG_OK;
     }
@@ -473,8 +473,8 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
       if (s != RMG_OK) { free_map(m); return s; }
       m->depth = 1;
       s = wide_build(m, st);
+      if (s == RMG_OK) s = update_info(m, st);
       if (s != RMG_OK) { free_map(m); return s; }
-      update_info(m, st);
       *out = m;
       return RMG_OK;
     }
@@ -488,8 +488,8 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
       }
       if (s != RMG_OK) { free_map(m); return s; }
       s = wide_build(m, st);
+      if (s == RMG_OK) s = update_info(m, st);
       if (s != RMG_OK) { free_map(m); return s; }
-      update_info(m, st);
       *out = m;
       return RMG_OK;
     }
@@ -550,8 +550,8 @@ extern "C" int rmg_map_build_ex(const rmg_vec3* vertices, uint32_t n_vertices, c
     if (s != RMG_OK) { free_map(m); return s; }
     m->depth = depth;
     s = wide_build(m, st);
+    if (s == RMG_OK) s = update_info(m, st);
     if (s != RMG_OK) { free_map(m); return s; }
-    update_info(m, st);
     *out = m;
     return RMG_OK;
   });
@@ -819,8 +819,8 @@ extern "C" int rmg_map_load(const char* path, void* stream, rmg_map** out) {
     up(m->d_leaf_parent, parents.data(), 4 * nf);
     if (s == RMG_OK) s = cuda_status(cudaStreamSynchronize(st), "sync");
     if (s == RMG_OK) s = wide_build(m, st);
+    if (s == RMG_OK) s = update_info(m, st);
     if (s != RMG_OK) { free_map(m); return s; }
-    update_info(m, st);
     *out = m;
     return RMG_OK;
   });
