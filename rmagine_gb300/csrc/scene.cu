@@ -404,7 +404,7 @@ double box_area(const float lo[3], const float hi[3]) {
 
 // Opens the tree of a geometry with at least 2 x RMG_SCENE_PIECE_TRIS
 // triangles into about n_faces / RMG_SCENE_PIECE_TRIS pieces (at most
-// kMaxPieces): the piece with the largest box surface is replaced by its two
+// kMaxPieces): the piece with the largest box surface is replaced by its
 // children until there are enough, or until every piece has a leaf child.
 int open_geometry(const rmg_map* g, bool wide, cudaStream_t st, std::vector<ScenePiece>& out) {
   out.clear();
@@ -414,7 +414,7 @@ int open_geometry(const rmg_map* g, bool wide, cudaStream_t st, std::vector<Scen
   struct Cand {
     ScenePiece p;
     float lo[3], hi[3];
-    bool closed;  // has a leaf child: stays whole
+    bool closed;  // has a leaf child, or more children than there is room for: stays whole
   };
   std::vector<Cand> c;
   c.push_back(Cand{ScenePiece{0, -1, 0}, {g->lo[0], g->lo[1], g->lo[2]}, {g->hi[0], g->hi[1], g->hi[2]}, false});
@@ -431,8 +431,12 @@ int open_geometry(const rmg_map* g, bool wide, cudaStream_t st, std::vector<Scen
       RMG_CUDA_TRY(cudaStreamSynchronize(st));
       const int* link = &nd.child.x;
       bool leaf = false;
-      for (int k = 0; k < 4; ++k) leaf = leaf || (link[k] < 0 && link[k] != kEmpty4);
-      if (leaf) { c[pick].closed = true; continue; }
+      size_t n = 0;
+      for (int k = 0; k < 4; ++k) {
+        leaf = leaf || (link[k] < 0 && link[k] != kEmpty4);
+        n += link[k] != kEmpty4 ? 1 : 0;
+      }
+      if (leaf || c.size() - 1 + n > kMaxPieces) { c[pick].closed = true; continue; }
       const int parent = c[pick].p.node;
       c.erase(c.begin() + pick);
       for (int k = 0; k < 4; ++k)
