@@ -455,7 +455,11 @@ int launch_stats(StatsParams& P, bool p2l, cudaStream_t st) {
     if (a != RMG_OK) return a;
     P.partial = reinterpret_cast<double*>(scratch);
     P.counters = reinterpret_cast<unsigned int*>(P.partial + 16ull * grid);
-    RMG_CUDA_TRY(cudaMemsetAsync(P.counters, 0, 4 * (size_t)P.n_batches, st));
+    const cudaError_t e = cudaMemsetAsync(P.counters, 0, 4 * (size_t)P.n_batches, st);
+    if (e != cudaSuccess) {
+      pool_free(scratch, st);
+      return cuda_status(e, "statistics counters");
+    }
   }
   const bool vec = vec_ok(P, p2l);
   const int variant = (p2l ? 4 : 0) | (vec ? 2 : 0) | (P.pre ? 1 : 0);
