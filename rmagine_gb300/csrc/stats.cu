@@ -153,7 +153,10 @@ __device__ __forceinline__ void finalize(const StatsParams& P, uint32_t b, doubl
 // Bound by latency: a CTA loads three or four times, sums and retires.  Four CTAs
 // (64 registers) hide more of it than three; five spill.  400 batches of 10,007
 // with masks, statistics, transform and backward, us a call: 140 / 136 / 150.
-template <bool P2L, bool VEC, bool PRE>
+//
+// VEC: 0 a correspondence at a time, 1 four at a time, 2 the same with masks and
+// ids one by one.
+template <bool P2L, int VEC, bool PRE>
 __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P) {
   const uint32_t b = blockIdx.x / P.chunks;
   const uint32_t c = blockIdx.x - b * P.chunks;
@@ -172,7 +175,7 @@ __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P)
   FAcc f;
   f.zero();
   const V zero{0.f, 0.f, 0.f};
-  if (VEC) {
+  if (VEC != 0) {
     // Thread t takes groups of 4 consecutive correspondences -- 3 x 16-byte loads
     // per array, one word of masks -- counted over the whole array, so that they
     // are aligned whatever n_per is; a batch's first and last group may hold
@@ -204,18 +207,24 @@ __global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P)
             *reinterpret_cast<float4*>(nn + 4) = __ldg(nv + 1);
             *reinterpret_cast<float4*>(nn + 8) = __ldg(nv + 2);
           }
-          const uint32_t dm = P.dmask ? __ldg(reinterpret_cast<const uint32_t*>(P.dmask + e)) : 0x01010101u;
-          const uint32_t mm = P.mmask ? __ldg(reinterpret_cast<const uint32_t*>(P.mmask + e)) : 0x01010101u;
-          const uint4 di = P.dids ? __ldg(reinterpret_cast<const uint4*>(P.dids + e))
-                                  : make_uint4(P.dataset_id, P.dataset_id, P.dataset_id, P.dataset_id);
-          const uint4 mi = P.mids ? __ldg(reinterpret_cast<const uint4*>(P.mids + e))
-                                  : make_uint4(P.model_id, P.model_id, P.model_id, P.model_id);
-          const bool id[4] = {di.x == P.dataset_id && mi.x == P.model_id, di.y == P.dataset_id && mi.y == P.model_id,
-                              di.z == P.dataset_id && mi.z == P.model_id, di.w == P.dataset_id && mi.w == P.model_id};
+          if (VEC == 1) {
+            const uint32_t dm = P.dmask ? __ldg(reinterpret_cast<const uint32_t*>(P.dmask + e)) : 0x01010101u;
+            const uint32_t mm = P.mmask ? __ldg(reinterpret_cast<const uint32_t*>(P.mmask + e)) : 0x01010101u;
+            const uint4 di = P.dids ? __ldg(reinterpret_cast<const uint4*>(P.dids + e))
+                                    : make_uint4(P.dataset_id, P.dataset_id, P.dataset_id, P.dataset_id);
+            const uint4 mi = P.mids ? __ldg(reinterpret_cast<const uint4*>(P.mids + e))
+                                    : make_uint4(P.model_id, P.model_id, P.model_id, P.model_id);
+            const bool id[4] = {di.x == P.dataset_id && mi.x == P.model_id, di.y == P.dataset_id && mi.y == P.model_id,
+                                di.z == P.dataset_id && mi.z == P.model_id, di.w == P.dataset_id && mi.w == P.model_id};
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (id[k] && (dm & (0xffu << (8 * k))) != 0 && (mm & (0xffu << (8 * k))) != 0 && e + k >= e0 && e + k < e1)
-              keep |= 1u << k;
+            for (int k = 0; k < 4; ++k)
+              if (id[k] && (dm & (0xffu << (8 * k))) != 0 && (mm & (0xffu << (8 * k))) != 0 && e + k >= e0 && e + k < e1)
+                keep |= 1u << k;
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (e + k >= e0 && e + k < e1 && passes(P, e + k)) keep |= 1u << k;
+          }
         } else {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -435,15 +444,22 @@ int fill_params(const rmg_transform* pre, uint32_t pre_stride, const rmg_vec3* d
   return RMG_OK;
 }
 
-// The 4-correspondence loads need aligned arrays (16 bytes; 4 for byte masks).  A
-// batch that is no multiple of four takes them from 2,048 correspondences per CTA
-// on: below, one correspondence per thread spreads over more warps, whose
-// binary32 sums are shorter.
-bool vec_ok(const StatsParams& P, bool p2l) {
-  if (P.n_per % 4 != 0 && std::min(P.n_per, P.chunk_len) < 2048) return false;
+// How k_stats reads (its VEC).  Four correspondences at a time need points that start
+// on 16 bytes; masks on 4 and ids on 16, or they are read one by one.  A batch that
+// is no multiple of four is read so from 2,048 correspondences per CTA on: below,
+// one correspondence per thread spreads over more warps, whose binary32 sums are
+// shorter.
+int vec_of(const StatsParams& P, bool p2l) {
   auto al = [](const void* p, uintptr_t a) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) % a) == 0; };
-  return al(P.dp, 16) && al(P.mp, 16) && (!p2l || al(P.mn, 16)) && al(P.dmask, 4) && al(P.mmask, 4) &&
-         al(P.dids, 16) && al(P.mids, 16);
+  if (P.n_per % 4 != 0 && std::min(P.n_per, P.chunk_len) < 2048) return 0;
+  if (!al(P.dp, 16) || !al(P.mp, 16) || (p2l && !al(P.mn, 16))) return 0;
+  return al(P.dmask, 4) && al(P.mmask, 4) && al(P.dids, 16) && al(P.mids, 16) ? 1 : 2;
+}
+
+template <bool P2L, int VEC>
+void launch_stats_as(const StatsParams& P, unsigned grid, cudaStream_t st) {
+  if (P.pre) k_stats<P2L, VEC, true><<<grid, kStatsThreads, 0, st>>>(P);
+  else k_stats<P2L, VEC, false><<<grid, kStatsThreads, 0, st>>>(P);
 }
 
 int launch_stats(StatsParams& P, bool p2l, cudaStream_t st) {
@@ -461,17 +477,13 @@ int launch_stats(StatsParams& P, bool p2l, cudaStream_t st) {
       return cuda_status(e, "statistics counters");
     }
   }
-  const bool vec = vec_ok(P, p2l);
-  const int variant = (p2l ? 4 : 0) | (vec ? 2 : 0) | (P.pre ? 1 : 0);
-  switch (variant) {
-    case 0: k_stats<false, false, false><<<grid, kStatsThreads, 0, st>>>(P); break;
-    case 1: k_stats<false, false, true><<<grid, kStatsThreads, 0, st>>>(P); break;
-    case 2: k_stats<false, true, false><<<grid, kStatsThreads, 0, st>>>(P); break;
-    case 3: k_stats<false, true, true><<<grid, kStatsThreads, 0, st>>>(P); break;
-    case 4: k_stats<true, false, false><<<grid, kStatsThreads, 0, st>>>(P); break;
-    case 5: k_stats<true, false, true><<<grid, kStatsThreads, 0, st>>>(P); break;
-    case 6: k_stats<true, true, false><<<grid, kStatsThreads, 0, st>>>(P); break;
-    default: k_stats<true, true, true><<<grid, kStatsThreads, 0, st>>>(P); break;
+  switch ((p2l ? 3 : 0) + vec_of(P, p2l)) {
+    case 0: launch_stats_as<false, 0>(P, grid, st); break;
+    case 1: launch_stats_as<false, 1>(P, grid, st); break;
+    case 2: launch_stats_as<false, 2>(P, grid, st); break;
+    case 3: launch_stats_as<true, 0>(P, grid, st); break;
+    case 4: launch_stats_as<true, 1>(P, grid, st); break;
+    default: launch_stats_as<true, 2>(P, grid, st); break;
   }
   const int s = cuda_status(cudaGetLastError(), "k_stats");
   pool_free(scratch, st);
