@@ -152,12 +152,14 @@ __device__ __forceinline__ void finalize(const StatsParams& P, uint32_t b, doubl
 
 // Bound by latency: a CTA loads three or four times, sums and retires.  Four CTAs
 // (64 registers) hide more of it than three; five spill.  400 batches of 10,007
-// with masks, statistics, transform and backward, us a call: 140 / 136 / 150.
+// with masks, statistics, transform and backward, us a call: 140 / 136 / 150.  Point
+// to plane holds a group's normals too and takes three CTAs (80 registers): at four
+// it spilled, 4,096 batches of 32,768 1,024 us, so 669 (4.8 GB).
 //
 // VEC: 0 a correspondence at a time, 1 four at a time, 2 the same with masks and
 // ids one by one.
 template <bool P2L, int VEC, bool PRE>
-__global__ void __launch_bounds__(kStatsThreads, 4) k_stats(const StatsParams P) {
+__global__ void __launch_bounds__(kStatsThreads, P2L && VEC != 0 ? 3 : 4) k_stats(const StatsParams P) {
   const uint32_t b = blockIdx.x / P.chunks;
   const uint32_t c = blockIdx.x - b * P.chunks;
   const uint64_t base = (uint64_t)b * P.n_per;
