@@ -116,8 +116,7 @@ typedef struct rmg_outputs {
 
 /* Traversal launch options (the knobs the autotuner searches).  A configuration
  * that is rmg_default_launch_config's in every field leaves the launch to the
- * library, as none does: small launches then take fewer rays per warp, and the
- * binary walk where it is the faster one. */
+ * library, as none does: small launches then take fewer rays per warp. */
 typedef struct rmg_launch_config {
   uint32_t stack_depth;   /* short-stack entries per ray: 0 (stackless, parent pointers), 8 or 16 */
   uint32_t block_warps;   /* warps per CTA */

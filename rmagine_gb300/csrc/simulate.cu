@@ -84,18 +84,6 @@ void fit_tile(uint32_t W, uint32_t H, uint32_t& tw, uint32_t& th) {
 // SM eight room scans take 48 us instead of 37.
 constexpr uint32_t kWarpRoom = 42;
 
-// A launch left to the library takes the binary walk where its warps are (nearly)
-// all on the GPU at once, of 16 rays or more, and the tree stays in the caches:
-// such a launch lasts as long as its slowest warp, and with few misses to wait for
-// that warp gets through many cheap visits sooner than through fewer dear ones.
-// 20 / 30 / 36 poses of 16 x 360 rays (24 / 36 / 43 warps per SM), us, 4-wide and
-// binary: 2,400 triangles 53.3 / 57.3 / 62.7 and 45.7 / 47.8 / 52.8, 1,000
-// 36.1 / 39.6 / 42.1 and 35.5 / 37.5 / 41.8, 20,000 79.0 / 84.6 / 90.9 and 68.8 /
-// 74.6 / 77.1; 180,000 85.2 / 98.6 / 105.6 and 81.1 / 96.1 / 101.7; 1,000,000 91 /
-// 114 / 131 and 110 / 141 / 150.  Fewer rays a warp (8 poses): 43.6 and 34.7 on
-// 2,400 triangles, but 52.4 and 56.0 on 20,000; one pose on 20,000 31 and 36.
-constexpr uint32_t kBinaryWarps = 48;        // per SM
-constexpr uint32_t kBinaryFaces = 1u << 17;
 uint32_t lanes_for(uint64_t n_rays) {
   const uint64_t room = (uint64_t)kWarpRoom * (uint64_t)device_sm_count();
   uint32_t lanes = 32;
@@ -140,12 +128,14 @@ int make_trace_params(const rmg_map* map, const rmg_sensor* sensor, const rmg_tr
   P.trail_bits = trail_bits_for_depth(map->depth);
   P.full_stack = map->depth <= (unsigned)kFullStack ? 1 : 0;
   // 4-wide walk unless another walk is asked for (a width, the packet walk, or a
-  // short stack other than the default's)
+  // short stack other than the default's).  It is the faster one from 252 to
+  // 1,000,000 triangles and from 2,000 to 10 million rays a launch: 0.77 of the
+  // binary walk's time on average over 13 meshes, 5 sensors and 10 sizes (0.36 to
+  // 1.06), 0.79 in the pose gradient, 0.74 in the fused correction.  (With the
+  // waiting children in no order, launches of few warps on small meshes took up to
+  // 1.4 times as long.)
   P.wide = (have_wide4(map) && cfg.refill == 0 &&
             (cfg.bvh_width == 4 || (cfg.bvh_width == 0 && cfg.packet != 1 && cfg.stack_depth == 16))) ? 1 : 0;
-  if (P.wide && any_tile && cfg.bvh_width == 0 && P.full_stack && P.tile_lanes >= 16 && map->n_faces <= kBinaryFaces &&
-      P.n_tiles <= (uint64_t)kBinaryWarps * (uint64_t)device_sm_count())
-    P.wide = 0;
   // 8-wide quantized walk: a pending-children stack of kStack8 entries holds trees of kStack8 + 1 levels
   const bool have8 = map->d_nodes8 && map->depth8 <= (unsigned)kStack8 + 1u;
   P.wide8 = (have8 && cfg.refill == 0 && (cfg.bvh_width == 8 || (cfg.bvh_width == 0 && RMG_DEFAULT_WIDE8))) ? 1 : 0;
