@@ -187,14 +187,19 @@ int work_pool(cudaMemPool_t* out) {
     p.handleTypes = cudaMemHandleTypeNone;
     p.location.type = cudaMemLocationTypeDevice;
     p.location.id = dev;
+    // the first call may be one that is being captured, here or in another thread:
+    // making the pool is no part of what is captured
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RMG_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
     cudaMemPool_t pool;
-    RMG_CUDA_TRY(cudaMemPoolCreate(&pool, &p));
-    uint64_t keep = kPoolKeepBytes;
-    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-      cudaMemPoolDestroy(pool);
-      return cuda_status(e, "cudaMemPoolSetAttribute");
+    cudaError_t e = cudaMemPoolCreate(&pool, &p);
+    if (e == cudaSuccess) {
+      uint64_t keep = kPoolKeepBytes;
+      e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) cudaMemPoolDestroy(pool);
     }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    RMG_CUDA_TRY(e);
     g_work_pool[dev] = pool;
   }
   *out = g_work_pool[dev];
