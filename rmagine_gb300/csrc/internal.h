@@ -17,7 +17,7 @@ struct rmg_map {
   uint32_t n_nodes;
   uint32_t depth;
   float lo[3], hi[3];
-  // device arrays, all in one allocation from the pool
+  // device arrays, all but the status word in one allocation from the pool
   void* d_arena;
   float* d_vertices;          // 3*n_vertices
   uint32_t* d_faces;          // 3*n_faces
@@ -80,10 +80,12 @@ int dev_alloc(T** p, size_t count, const char* what) {
 
 // Device memory from the library's stream-ordered pool of the current device
 // (runtime.cu): what a call or a map gives back is kept for the next one, up to
-// kPoolKeepBytes, instead of going through the driver.  pool_free takes NULL.
+// kPoolKeepBytes, instead of going through the driver.  pool_free and pool_release
+// take NULL.
 int pool_alloc_bytes(void** p, size_t bytes, cudaStream_t st, const char* what);
 void pool_free(void* p, cudaStream_t st);
-void pool_trim();  // gives back what the pools of all devices hold unused
+void pool_release(void* p);  // once nothing on the device uses it any more
+void pool_trim();            // gives back what the pools of all devices hold unused
 
 template <typename T>
 int pool_alloc(T** p, size_t count, cudaStream_t st, const char* what) {

@@ -283,20 +283,19 @@ rmg_map* new_map() {
   return m;
 }
 
-// Waits for the device (work on any stream may use the map), as freeing its
-// arrays one by one did, and hands them back to the pool.
+// Hands a map's arrays back to the pool, after all work on the device (any stream
+// may use the map).  What waits is freeing the status word, which is an allocation
+// of its own for that: cudaDeviceSynchronize would invalidate a capture that is
+// under way in another thread or in a relaxed mode.
 void free_map(rmg_map* m) {
   if (!m) return;
   int cur = m->device;
   cudaGetDevice(&cur);
   if (cur != m->device) cudaSetDevice(m->device);
-  cudaDeviceSynchronize();
+  cudaFree(m->d_status);
   wide_free(m);
-  pool_free(m->d_arena, nullptr);
-  if (g_live_maps.fetch_sub(1) == 1) {
-    cudaStreamSynchronize(nullptr);
-    pool_trim();
-  }
+  pool_release(m->d_arena);
+  if (g_live_maps.fetch_sub(1) == 1) pool_trim();
   if (cur != m->device) cudaSetDevice(cur);
   delete m;
 }
@@ -306,14 +305,15 @@ int alloc_arrays(rmg_map* m, cudaStream_t st) {
   const size_t nv = m->n_vertices, nf = m->n_faces, nn = m->n_nodes;
   size_t off = 0;
   auto carve = [&](size_t bytes) { const size_t at = off; off = (off + bytes + 255) & ~size_t(255); return at; };
-  const size_t o_status = carve(sizeof(unsigned int)), o_vert = carve(12 * nv), o_face = carve(12 * nf),
+  const size_t o_vert = carve(12 * nv), o_face = carve(12 * nf),
                o_node = carve(sizeof(Node) * nn), o_tri = carve(sizeof(Tri) * nf), o_order = carve(4 * nf),
                o_parent = carve(4 * nf), o_flag = carve(4 * nn);
+  int s = dev_alloc(&m->d_status, 1, "status");
+  if (s != RMG_OK) return s;
   unsigned char* base = nullptr;
-  const int s = pool_alloc(&base, off, st, "map");
+  s = pool_alloc(&base, off, st, "map");
   if (s != RMG_OK) return s;
   m->d_arena = base;
-  m->d_status = reinterpret_cast<unsigned int*>(base + o_status);
   m->d_vertices = reinterpret_cast<float*>(base + o_vert);
   m->d_faces = reinterpret_cast<uint32_t*>(base + o_face);
   m->d_nodes = reinterpret_cast<Node*>(base + o_node);

@@ -224,6 +224,11 @@ void pool_free(void* p, cudaStream_t st) {
   if (p) cudaFreeAsync(p, st);
 }
 
+// cudaFree takes pool memory too, and then waits for nothing.
+void pool_release(void* p) {
+  if (p) cudaFree(p);
+}
+
 void pool_trim() {
   std::lock_guard<std::mutex> lock(g_work_pool_mu);
   for (int d = 0; d < kPoolDevices; ++d)

@@ -191,7 +191,7 @@ __global__ void k_wide_refit(const Node* __restrict__ bn, const int* __restrict_
 
 void wide_free(rmg_map* m) {
   wide8_free(m);
-  pool_free(m->d_nodes4, nullptr);  // the caller has waited for the device
+  pool_release(m->d_nodes4);  // the caller has waited for the device
   m->d_nodes4 = nullptr;
   m->d_src4 = nullptr;
   m->n_nodes4 = 0;
