@@ -627,7 +627,9 @@ extern "C" int rmg_map_export(const rmg_map* m, void* nodes, void* tris, uint32_
 // (children, parents, face ids, leaf order, face vertex indices) on the host
 // before anything reaches the device, so a damaged or crafted file is
 // rejected with RMG_ERR_INVALID_ARG instead of steering a kernel out of bounds;
-// the tree depth is recomputed from the links.
+// the tree depth is recomputed from the links.  So are the parents that a refit
+// follows from the leaves: the file's need not agree with the links, and a refit
+// would then not come to an end.
 namespace {
 
 constexpr char kMapMagic[8] = {'R', 'M', 'G', 'L', 'B', 'V', 'H', '1'};
@@ -655,9 +657,9 @@ uint64_t payload_size(uint64_t nv, uint64_t nf, uint64_t nn) {
   return 12 * nv + 12 * nf + sizeof(Node) * nn + sizeof(Tri) * nf + 4 * nf + 4 * nf;
 }
 
-// Index checks and depth of a loaded tree; returns RMG_OK or INVALID_ARG.
-int check_tree(const MapFileHeader& h, const uint32_t* faces, const Node* nodes, const Tri* tris,
-               const uint32_t* order, const int* leaf_parent, uint32_t* depth_out) {
+// Index checks, depth and parents of a loaded tree; returns RMG_OK or INVALID_ARG.
+int check_tree(const MapFileHeader& h, const uint32_t* faces, Node* nodes, const Tri* tris,
+               const uint32_t* order, int* leaf_parent, uint32_t* depth_out) {
   const uint32_t nv = h.n_vertices, nf = h.n_faces, nn = h.n_nodes;
   const uint32_t want_nodes = nf >= 2 ? nf - 1 : (nf == 1 ? 1 : 0);
   if (nn != want_nodes) return fail(RMG_ERR_INVALID_ARG, "rmg_map_load: node count does not match the face count");
@@ -708,6 +710,14 @@ int check_tree(const MapFileHeader& h, const uint32_t* faces, const Node* nodes,
       }
     }
     if (visited != nn) return fail(RMG_ERR_INVALID_ARG, "rmg_map_load: unreachable nodes");
+  }
+  if (nf == 1) leaf_parent[0] = -1;
+  for (uint32_t i = 0; nf >= 2 && i < nn; ++i) {
+    const int c[2] = {nodes[i].d.x, nodes[i].d.y};
+    for (int k = 0; k < 2; ++k) {
+      if (c[k] >= 0) nodes[c[k]].d.z = (int)i;
+      else leaf_parent[~c[k]] = (int)i;
+    }
   }
   *depth_out = depth;
   return RMG_OK;
