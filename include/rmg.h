@@ -217,7 +217,8 @@ int rmg_map_status(rmg_map* map, int clear);
  * to check that a corrupt tree ends in RMG_ERR_TRAVERSAL_BUDGET, not a
  * fault; values are range-checked so every link stays inside the arrays.
  * which 0 / 1: left / right link of binary node `node` (the map's 4-wide tree
- * is walked no longer, so the damaged binary tree is the one walked);
+ * is walked no longer and its 8-wide tree is dropped, so the damaged binary tree
+ * is the one walked);
  * which 2..5: slot which-2 of 4-wide node `node` (the node's slots are put in
  * order again, internal children first, and those children are copied behind
  * the last node). */

@@ -867,7 +867,10 @@ extern "C" int rmg_map_debug_set_child(rmg_map* m, uint32_t node, uint32_t which
     const size_t off = offsetof(Node, d) + (which ? sizeof(int) : 0);
     RMG_CUDA_TRY(cudaMemcpy(reinterpret_cast<char*>(m->d_nodes + node) + off, &child, sizeof(int),
                             cudaMemcpyHostToDevice));
-    m->depth4 = 0xffffffffu;  // the binary tree is the one damaged: walk it from now on (see have_wide4)
+    // the binary tree is the one damaged: walk it from now on (see have_wide4; scenes
+    // made before keep the 4-wide nodes that they name)
+    m->depth4 = 0xffffffffu;
+    wide8_free(m);
     return RMG_OK;
   });
 }
