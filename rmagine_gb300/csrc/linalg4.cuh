@@ -97,10 +97,8 @@ __device__ __forceinline__ void quat_f(const float w0[3], const float w1[3], con
   for (int k = 0; k < 4; ++k) q[k] *= r;
 }
 
-// Whether any lane of a group says so, in its lanes.
-__device__ __forceinline__ bool any4(bool x) {
-  return (__ballot_sync(0xffffffffu, x) >> (threadIdx.x & 28) & 15u) != 0;
-}
+// Whether any lane of this lane's group is in a warp's vote.
+__device__ __forceinline__ bool any4(uint32_t vote) { return (vote >> (threadIdx.x & 28) & 15u) != 0; }
 
 __device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 
@@ -125,10 +123,10 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   int e = __double2hiint(pick(j, a[0], a[1], a[2])) & 0x7ff00000;
   e = max(max(of4(e, 0), of4(e, 1)), of4(e, 2));
   // (no exchange inside a choice: every lane of the warp takes part in all of them)
-  const bool mixed = any4(!is_zero(pick(j, a[1], a[2], a[0])) || !is_zero(pick(j, a[2], a[0], a[1])));
-  const bool some = any4(!is_zero(pick(j, a[0], a[1], a[2])));
-  const bool diagonal = !mixed, zero = !mixed && !some;
-  if (__all_sync(0xffffffffu, zero)) {
+  const uint32_t mixed = __ballot_sync(0xffffffffu, !is_zero(pick(j, a[1], a[2], a[0])) || !is_zero(pick(j, a[2], a[0], a[1])));
+  const uint32_t some = __ballot_sync(0xffffffffu, !is_zero(pick(j, a[0], a[1], a[2])));
+  const bool diagonal = !any4(mixed), zero = !any4(mixed | some);
+  if ((mixed | some) == 0) {
     U = V = m3_eye();
     s[0] = s[1] = s[2] = 0.0;
     return true;
@@ -141,7 +139,7 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   const double a00 = of4(a[0], 0), a01 = of4(a[0], 1), a02 = of4(a[0], 2);
   const double a11 = of4(a[1], 1), a12 = of4(a[1], 2), a22 = of4(a[2], 2);
   float f00 = (float)a00, f01 = (float)a01, f02 = (float)a02, f11 = (float)a11, f12 = (float)a12, f22 = (float)a22;
-  double v[3], y[3], z[3];  // this lane's column of V, the columns n1 and n2
+  double v[3] = {0.0, 0.0, 0.0}, y[3], z[3];  // this lane's column of V, the columns n1 and n2
   double d, off, g;         // elements (j, j) and (j, n1) of A in V's frame, and the gap of their eigenvalues
   float X, fg;
   // One pass, and up to two more for the groups with small eigenvalues closer than a
@@ -150,9 +148,8 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   // other groups keep their frame meanwhile and form the same numbers from it again,
   // so that a problem's result does not depend on its neighbours.
   bool again = true;
-  const bool passes = !__all_sync(0xffffffffu, diagonal || bad);
 #pragma unroll 1
-  for (int pass = 0; passes; ++pass) {
+  for (int pass = 0; mixed != 0; ++pass) {
     float w0[3] = {1.f, 0.f, 0.f}, w1[3] = {0.f, 1.f, 0.f}, w2[3] = {0.f, 0.f, 1.f};
     const float tol = pass == 0 ? 1e-13f : 1e-34f;
 #pragma unroll 1
@@ -197,8 +194,9 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
       far = false;
       X = 0.0f;
     }
-    again = any4(far && !bad && !diagonal);
-    if (pass == 2 || !__any_sync(0xffffffffu, again)) {
+    const uint32_t away = __ballot_sync(0xffffffffu, far && !bad && !diagonal);
+    again = any4(away);
+    if (pass == 2 || away == 0) {
       bad = bad || (far && !diagonal);
       break;
     }
@@ -207,7 +205,7 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
     f01 = of4(fo, 0); f12 = of4(fo, 1); f02 = of4(fo, 2);
     if (!again) f01 = f12 = f02 = 0.0f;
   }
-  if (passes) {
+  if (mixed != 0) {
     const float Xa = of4(X, n1), Xb = of4(X, n2), ga = of4(fg, n1), gb = of4(fg, n2);
     const float rest = (float)(off - g * (double)X) + 0.5f * Xa * Xb * (ga - gb);
     const float Xc = fabsf(rest) <= 4e-16f && !(fabsf(rest) < 1e-8f * fabsf(fg)) ? 0.0f : rest / fg;
@@ -218,7 +216,7 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] += p0 * v[k] + p1 * y[k] + p2 * z[k];
   }
-  if (diagonal || !passes) {
+  if (diagonal) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] = k == j ? 1.0 : 0.0;
   }
@@ -277,7 +275,7 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
     U.a[k][0] = u0[k]; U.a[k][1] = u1[k]; U.a[k][2] = u2[k];
     s[k] = of4(sj, k);
   }
-  if (any4(bad)) svd3_rot(C, U, s, V);
+  if (any4(__ballot_sync(0xffffffffu, bad))) svd3_rot(C, U, s, V);
   if (zero) {
     U = V;
     s[0] = s[1] = s[2] = 0.0;

@@ -382,15 +382,16 @@ __global__ void __launch_bounds__(kStatsThreads) k_umeyama_bwd_stream(const BwdP
   const uint32_t c = blockIdx.x - b * P.chunks;
   const uint64_t base = (uint64_t)b * P.n_per;
   const uint32_t lo = c * P.chunk_len;
-  const uint32_t hi = lo + min(P.n_per - lo, P.chunk_len);  // lo < n_per, see fill_params
+  const uint32_t hi = P.n_per - lo < P.chunk_len ? P.n_per : lo + P.chunk_len;  // lo < n_per, see fill_params
   const Tf pre = batch_pre(P, b);
   const Q preinv = qconj(pre.R);
   __shared__ Coef cf;
   if (threadIdx.x == 0) cf = B.coef[b];
   __syncthreads();
   const V zero{0.f, 0.f, 0.f};
-  for (uint32_t j = threadIdx.x; j < hi - lo; j += blockDim.x) {
-    const uint64_t i = base + lo + j;
+  if (threadIdx.x >= hi - lo) return;
+  for (uint32_t j = lo + threadIdx.x; j < hi; j += blockDim.x) {
+    const uint64_t i = base + j;
     V D, M;
     const bool ok = correspondence<false>(P, pre, i, ldv(P.dp, i), ldv(P.mp, i), zero, D, M);
     float gm[3] = {0.f, 0.f, 0.f}, gdv[3] = {0.f, 0.f, 0.f};
@@ -406,6 +407,7 @@ __global__ void __launch_bounds__(kStatsThreads) k_umeyama_bwd_stream(const BwdP
     }
     if (B.gm) { B.gm[3 * i] = gm[0]; B.gm[3 * i + 1] = gm[1]; B.gm[3 * i + 2] = gm[2]; }
     if (B.gd) { B.gd[3 * i] = gdv[0]; B.gd[3 * i + 1] = gdv[1]; B.gd[3 * i + 2] = gdv[2]; }
+    if (hi - j <= blockDim.x) break;  // j + blockDim.x may pass 2^32
   }
 }
 
