@@ -65,26 +65,26 @@ WORK_PER_RAY = {
 # from one ncu capture of the workload (profiles/).
 TRAFFIC: dict = {
     # captured on 100 poses (13.1 M rays) and scaled by the ray count to the 1,000-pose launch
-    "terrain1m_spherical": 10 * (273549568 + 414917376),
+    "terrain1m_spherical": 10 * (249177344 + 412728320),
     # captured on 512 batches (16.8 M correspondences) and scaled by 16 to the 8,192-batch launch
     "icp_stats_fwd": 16 * (402915328 + 3088384),
     "icp_stats_bwd": 16 * (403369216 + 357416960),
     # captured on 64 poses (4.19 M rays) and scaled by 64 to the 4,096-pose launch
-    "pose_grad": 64 * (213367296 + 10159616),
+    "pose_grad": 64 * (195585024 + 10249472),
     # captured on 50 poses (15.4 M rays) / 100 poses (13.1 M rays) and scaled to the 1,000-pose launch
-    "terrain1m_pinhole": 20 * (81764096 + 479327232),
-    "terrain2m_spherical": 10 * (525986560 + 432446976),
+    "terrain1m_pinhole": 20 * (76448256 + 478631936),
+    "terrain2m_spherical": 10 * (481427200 + 429165824),
     # captured on 100 poses (13.1 M rays) and scaled by the ray count to the 1,000-pose launch
-    "rcc_fused": 10 * (278349824 + 14763264),
+    "rcc_fused": 10 * (260233472 + 13442048),
     # full-size launch (131,072,000 ranges)
     "noise": 524465664 + 463988224,
     # captured on 100 poses (13.1 M rays) and scaled by the ray count to the 1,000-pose launch
-    "scene_terrain1m": 10 * (353755904 + 663259392),
+    "scene_terrain1m": 10 * (321539328 + 653904896),
     # the whole 1,024-sensor launch (780,800 rays)
-    "batched_small": 179047936 + 12244736,
+    "batched_small": 168597248 + 11310336,
     # captured with every sensor cut to 16 poses (143,238,688 rays) and scaled by the ray count to the
     # full 64-sensor launch (9,025,081,856 rays)
-    "batched": round(9025081856 / 143238688 * (2113643008 + 794353664)),
+    "batched": round(9025081856 / 143238688 * (1912611584 + 789447424)),
 }
 
 SRC_COUNTERS = "profiles/traversal_counters_by_workload.md (small cases)"
@@ -92,17 +92,17 @@ SRC_COUNTERS = "profiles/traversal_counters_by_workload.md (small cases)"
 # Warp instructions per unit (ray) of the dominant kernel, `smsp__inst_executed.sum` of one ncu
 # capture on the small case of the workload divided by its rays (profiles/), keyed by kernel walk.
 ISSUE: dict = {
-    "terrain1m_spherical/wide4": {"warp_inst_per_unit": 1336972581 / 13107200, "source":
+    "terrain1m_spherical/wide4": {"warp_inst_per_unit": 1286613899 / 13107200, "source":
                                   "profiles/k_trace_terrain1m_spherical.md (100 poses, 13,107,200 rays)"},
-    "pose_grad/k_range_grad": {"warp_inst_per_unit": 500072639 / 4194304, "source":
+    "pose_grad/k_range_grad": {"warp_inst_per_unit": 479228468 / 4194304, "source":
                                "profiles/k_range_grad_terrain2m_posegrad.md (64 poses, 4,194,304 rays)"},
-    "terrain1m_pinhole/wide4": {"warp_inst_per_unit": 1108598517 / 15360000, "source": SRC_COUNTERS},
-    "terrain2m_spherical/wide4": {"warp_inst_per_unit": 1431417870 / 13107200, "source": SRC_COUNTERS},
-    "room_vlp16/wide4": {"warp_inst_per_unit": 97591585 / 1440000, "source": SRC_COUNTERS},
-    "rcc_fused/k_trace_stats": {"warp_inst_per_unit": 1110709255 / 13107200, "source": SRC_COUNTERS},
-    "scene_terrain1m/k_trace_scene": {"warp_inst_per_unit": 1819218053 / 13107200, "source": SRC_COUNTERS},
-    "batched_small/k_trace_batched": {"warp_inst_per_unit": 148012101 / 780800, "source": SRC_COUNTERS},
-    "batched/k_trace_batched": {"warp_inst_per_unit": 13162807329 / 143238688, "source":
+    "terrain1m_pinhole/wide4": {"warp_inst_per_unit": 1081814016 / 15360000, "source": SRC_COUNTERS},
+    "terrain2m_spherical/wide4": {"warp_inst_per_unit": 1377411403 / 13107200, "source": SRC_COUNTERS},
+    "room_vlp16/wide4": {"warp_inst_per_unit": 91305312 / 1440000, "source": SRC_COUNTERS},
+    "rcc_fused/k_trace_stats": {"warp_inst_per_unit": 1064000456 / 13107200, "source": SRC_COUNTERS},
+    "scene_terrain1m/k_trace_scene": {"warp_inst_per_unit": 1767754597 / 13107200, "source": SRC_COUNTERS},
+    "batched_small/k_trace_batched": {"warp_inst_per_unit": 141116218 / 780800, "source": SRC_COUNTERS},
+    "batched/k_trace_batched": {"warp_inst_per_unit": 12638607499 / 143238688, "source":
                                 "profiles/k_trace_batched_mixed64.md (16 poses per sensor, 143,238,688 rays)"},
 }
 

@@ -230,7 +230,7 @@ bool own_tiles(const rmg_batch_config& c) {
 
 // The walk of a plan, as kernel_ptr takes it: the default's stack depth is the
 // 4-wide tree, 16 the binary one with a full stack, 0 (and trees too deep for
-// either) the short-stack walk.  512 sensors, 590,000 rays: 193, 208 and 345 us.
+// either) the short-stack walk.  512 sensors, 590,000 rays: 174, 208 and 345 us.
 int batch_walk(const rmg_batch* b) {
   if (b->cfg.stack_depth == default_batch_config().stack_depth && have_wide4(b->map)) return kWideTB;
   if (b->cfg.stack_depth > 0 && b->map->depth <= (unsigned)kFullStack) return 0;
@@ -243,8 +243,8 @@ int build_jobs(rmg_batch* b) {
   uint64_t begin = 0, rays = 0;
   for (const rmg_batch_entry& e : b->entries) rays += (uint64_t)e.sensor->width * e.sensor->height * e.n_poses;
   // few rays: tiles of 4 to 16 (see lanes_for).  24,600 rays of 64 scattered and
-  // camera sensors on a 30,000-triangle terrain: 79 us with whole warps, 56 so;
-  // 590,000 rays keep whole warps (231 us, 272 with 16).
+  // camera sensors on a 30,000-triangle terrain: 55 us with whole warps, 47 so;
+  // 590,000 rays keep whole warps (174 us, 226 with 16).
   const uint32_t lanes = own_tiles(b->cfg) ? lanes_for(rays) : 32;
   for (const rmg_batch_entry& e : b->entries) {
     JobDev J;
@@ -297,8 +297,8 @@ BatchParams params(const rmg_batch* b, uint64_t warps) {
   B.counter = b->counter;
   // Left to the library, a warp takes `grab` tiles at a time only where there are
   // many times as many: a tile of scattered rays lasts 60 us, and 3.4 tiles for each
-  // warp in twos make four (590,000 rays of 512 sensors: 266 -> 231 us; 161,000
-  // rays 165 -> 103).
+  // warp in twos make four (590,000 rays of 512 sensors: 202 -> 174 us; 172,000
+  // rays 107 -> 74).
   B.grab = b->cfg.grab;
   if (own_tiles(b->cfg)) B.grab = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(B.grab, b->total_tiles / (16 * warps)));
   B.budget = 2u * b->map->n_nodes + 64u;

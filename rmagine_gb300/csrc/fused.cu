@@ -35,9 +35,9 @@ namespace {
 // Tiles (32 rays) that a warp reduces before its CTA writes one partial record.
 // Fewer make more CTAs, of which the last, partly idle wave is a smaller part;
 // more make fewer records and less final work.  8 / 4 / 2 / 1 tiles, us: 256 poses
-// x 180 tiles 279 / 259 / 246 / 238, 1 pose 123 / 101 / 79 / 67, 48 x 656 500 / 347 /
-// 334 / 328, 4,000 x 180 2,668 / 2,687 / 2,747 / 2,877, 300 x 4,096 4,201 / 4,203 /
-// 4,254 / 4,512.  The number depends on the sensor alone, so that a pose's sums
+// x 180 tiles 201 / 178 / 167 / 169, 1 pose 90 / 59 / 45 / 39, 48 x 656 416 / 291 /
+// 230 / 212, 4,000 x 180 1,953 / 1,960 / 2,000 / 2,094, 300 x 4,096 3,993 / 3,998 /
+// 4,093 / 4,322.  The number depends on the sensor alone, so that a pose's sums
 // do not depend on how many poses a launch holds.
 constexpr uint32_t tiles_per_warp(uint32_t tiles_per_pose) { return tiles_per_pose >= 1024 ? 4 : 2; }
 
@@ -64,7 +64,7 @@ struct FusedParams {
 // A binary64 instruction takes 64 cycles for a warp, however many of its lanes
 // are on, so every lane does the same three, on its own operands.  With branches
 // on k there were some 15, and the 16 sums took 80 shuffles: 256 poses of 16 x 360
-// rays 240 us a call, now 235.
+// rays 240 -> 235 us a call.
 __device__ __forceinline__ double add_moment(double acc, float x, float n, const V& sd, const V& sm) {
   const uint32_t k = (threadIdx.x & 31) >> 1;
   const uint32_t e = k < 7 ? 0 : k - 7, i = e / 3, j = e - 3 * i;

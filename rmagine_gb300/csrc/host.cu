@@ -32,8 +32,8 @@ constexpr size_t kDefaultChunkBytes = size_t(128) << 20;
 constexpr int kDefaultCompute = 2;
 // A launch lasts as long as its slowest rays (60 to 100 us) however few poses it
 // has, while 8 MiB cross the link in 45 us.  64 poses of 10,000 directions with
-// 17 bytes a ray: 427 / 331 / 284 / 281 / 287 us with least chunks of 1 / 4 / 8 /
-// 16 / 32 MiB; 200 poses 558 / 520 / 511 / 515 / 596.
+// 17 bytes a ray: 295 / 263 / 247 / 249 / 248 us with least chunks of 1 / 4 / 8 /
+// 16 / 32 MiB; 200 poses 486 / 472 / 460 / 477 / 537.
 constexpr size_t kLeastChunkBytes = size_t(8) << 20;
 std::atomic<size_t> g_chunk_bytes{kDefaultChunkBytes};
 std::atomic<int> g_compute{kDefaultCompute};

@@ -31,7 +31,7 @@
 // the first's in range and face and lose the tie to its smaller index.
 //
 // Traversal (k_trace_scene): the top tree is walked with a full stack, the lanes
-// of a warp entering instances together (walk4_gather: 1,275 -> 1,239 us on the
+// of a warp entering instances together (walk4_gather: 1,213 -> 1,175 us on the
 // terrain under 2,000 boxes); at an instance leaf the ray is taken into the instance's mesh frame,
 //     o_l = s^-1 (.) R^T (o - t),   d_l = s^-1 (.) R^T d   (R^T as conj(q) sandwich),
 // which keeps the ray parameter t, and the geometry's tree is walked by the
@@ -218,8 +218,8 @@ __device__ __forceinline__ void trace_scene(const SceneParams& S, const V& o, co
 }
 
 // 64 registers: the instance walk nested in the top-level one keeps both levels'
-// state (1M-triangle terrain under 2,000 boxes: 1,336 / 1,239 / 1,260 us with 56 /
-// 64 / 72, 1,344 with the binary walks on both levels).
+// state (1M-triangle terrain under 2,000 boxes: 1,257 / 1,175 / 1,179 us with 56 /
+// 64 / 72; 1,344 with the binary walks on both levels).
 template <int OK, bool WIDE, bool TOP>
 __global__ void __maxnreg__(64) k_trace_scene(const SceneParams S) {
   const TraceParams& P = S.T;

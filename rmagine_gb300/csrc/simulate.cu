@@ -78,10 +78,11 @@ void fit_tile(uint32_t W, uint32_t H, uint32_t& tw, uint32_t& th) {
 // still find room on the GPU, 36 per SM at the 4-wide walk's 56 registers and a
 // few more.  A launch of few warps is a latency chain as long as the longest path
 // of a warp's rays, and fewer rays share fewer detours: one 16 x 900 scan of the
-// box room 28.6 -> 20.7 us (4 rays a warp), of the 1M-triangle terrain 59.6 ->
-// 42.5, 3 x 32 x 513 there 84.8 -> 62.4 (8), 4 x 10,000 scattered directions 73.5
-// -> 57.6.  Larger launches fill the SMs with whole warps: with room for 120 per
-// SM eight room scans take 48 us instead of 37.
+// box room 20.5 -> 16.5 us (4 rays a warp), of the 1M-triangle terrain 49.2 ->
+// 32.8, 3 x 32 x 513 there 63.5 -> 54.0 (8), 4 x 10,000 scattered directions 57.4
+// -> 45.1.  Larger launches fill the SMs with whole warps: with room for 120 per
+// SM eight room scans take 37.8 us instead of 24.6, with room for 20 the three
+// terrain launches 36.9, 63.5 and 53.6.
 constexpr uint32_t kWarpRoom = 42;
 
 uint32_t lanes_for(uint64_t n_rays) {

@@ -12,7 +12,7 @@
 // pre-transformed dataset point and first model point), binary32 sums of
 // d', m' and m' d'^T over runs of at most 32 correspondences; the warp sums its
 // 32 runs pairwise in binary32 and folds the result into binary64 accumulators
-// (one lane, one fold per 1024 correspondences); the CTA combines in binary64, and
+// (a lane for each sum, one fold per 1024 correspondences); the CTA combines in binary64, and
 // batches split over several CTAs are combined in a fixed order by the last
 // CTA to finish, so results are deterministic.  The mean and covariance are
 // formed in binary64 (cov = E[m' d'^T] - E[m'] E[d']^T), then rounded to the

@@ -1,11 +1,14 @@
-// Per-ray closest-hit traversal of the LBVH and the attribute epilogue.
+// Per-ray closest-hit traversal of a map's trees and the attribute epilogue.
 //
 // This is the GPU restatement of the per-ray body of rmagine's simulators:
 //   SphereSimulatorEmbree.tcc:69-249 (ray setup, rtcIntersect1, attributes)
 //   O1DnSimulatorEmbree.tcc:84-132, OnDnSimulatorEmbree.tcc:86-134 (origins)
 // with the BVH query done by this file instead of Embree/OptiX.
 //
-// Traversal ("short stack + parent pointers"):
+// The default walk is that of the 4-wide tree (trace_ray4 below).  The binary
+// tree's ("short stack + parent pointers", or a full stack for trees of up to 32
+// levels) is taken where it is asked for or the 4-wide tree has more than 21
+// levels:
 //   * Every internal node carries both child boxes; a visit tests the two
 //     boxes, intersects leaf children (one triangle each) on the spot and
 //     descends into the nearer hit internal child.
@@ -19,7 +22,10 @@
 //   * Box tests widen every plane distance outward by |o/d| 2^-21 and the
 //     interval by 2^-22 relative (RayBox); triangle tests are the
 //     watertight test of common.cuh.  Closest-hit ties are broken by the
-//     smaller face id, so the result does not depend on traversal order.
+//     smaller face id, so the result does not depend on traversal order -- but
+//     for (nearly) coplanar triangles met at a grazing angle: their ranges differ
+//     by the rounding of the triangle test, which there is more than the box
+//     tests are widened by, and which of them is found may differ by walk.
 //   * Every ray has a step budget (2 * internal nodes + 64 node visits and
 //     parent climbs, more than any valid tree needs).  Exceeding it records
 //     RMG_ERR_TRAVERSAL_BUDGET in the map's device status word and ends the
@@ -554,19 +560,18 @@ __device__ __forceinline__ void walk4_gather(const Node4* nodes, int node, const
 // identical; only the order of visits differs.
 //
 // What bounds it is instruction issue and the half-rate min/max/compare pipe
-// (65% and 54% busy on the 1M-triangle terrain; L1 68%), so a visit is built to
+// (70% and 60% busy on the 1M-triangle terrain; L1 73%), so a visit is built to
 // spend little there: the near and far planes are picked by address from the
 // ray's signs (no min/max of a plane pair), two children share an FMA
 // (fma.rn.f32x2), the hits are a 4-bit mask, and entry distances are ordered
 // only where two or more internal children are hit (23% of the visits).  Internal
 // children are consecutive nodes, so no link is read for them.  12.7 visits per
 // ray against 24.9 binary ones there.  Both walks, us a pass: that terrain with
-// a 128 x 1024 lidar 3,140 (binary) / 3,030, a 2.1M-triangle terrain with a
-// 640 x 480 camera 1,513 / 1,414, the box room with a 16 x 360 lidar 312 / 292,
-// one 16 x 900 scan there 32.1 / 27.8 (tiles of 32), scattered directions 202 /
-// 178.  Postponing
-// the leaf tests until every lane has one, 32-bit node offsets and a pointer per
-// plane all measured slower.
+// a 128 x 1024 lidar 3,013 (binary) / 2,751, a 2.1M-triangle terrain with a
+// 640 x 480 camera 1,515 / 1,382, the box room with a 16 x 360 lidar 305 / 263,
+// one 16 x 900 scan there 30.7 / 24.3 (tiles of 32), scattered directions 160 /
+// 132.  Postponing the leaf tests until every lane has one, 32-bit node offsets and
+// a pointer per plane all measured slower.
 __device__ __forceinline__ void trace_ray4(const DeviceMap& map, const V& o, const V& d, float tfar,
                                            unsigned budget, Hit& h, bool& over_budget) {
   h.t = tfar;
@@ -1021,8 +1026,8 @@ __device__ __forceinline__ void reread_ray(const SensorDev& sen, uint32_t loc, V
 // per SM, a few bytes of spills to L1-cached local memory) is 9% faster than
 // unconstrained at 62 (1M-triangle terrain, 5,661 -> 6,179 Mrays/s then), 40
 // registers lose again.  The 4-wide walk holds twice the planes per visit; on
-// the same terrain 48 / 56 / 64 registers take 3,573 / 3,040 / 3,195 us, in the
-// box room 341 / 292 / 301.  The 8-wide walk holds a
+// the same terrain 48 / 56 / 64 registers take 3,281 / 2,797 / 2,946 us, in the
+// box room 311 / 266 / 274.  The 8-wide walk holds a
 // node's twenty words and three axes of plane addends at once.
 template <int TB>
 constexpr int trace_regs() { return TB == kWide8TB ? 64 : (TB == kWideTB ? 56 : 48); }
