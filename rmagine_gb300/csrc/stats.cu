@@ -389,8 +389,7 @@ __global__ void __launch_bounds__(kStatsThreads) k_umeyama_bwd_stream(const BwdP
   if (threadIdx.x == 0) cf = B.coef[b];
   __syncthreads();
   const V zero{0.f, 0.f, 0.f};
-  if (threadIdx.x >= hi - lo) return;
-  for (uint32_t j = lo + threadIdx.x; j < hi; j += blockDim.x) {
+  for (uint32_t j = lo + threadIdx.x; j < hi; j += blockDim.x) {  // ends: hi <= 2^32 - kStatsThreads
     const uint64_t i = base + j;
     V D, M;
     const bool ok = correspondence<false>(P, pre, i, ldv(P.dp, i), ldv(P.mp, i), zero, D, M);
@@ -407,7 +406,6 @@ __global__ void __launch_bounds__(kStatsThreads) k_umeyama_bwd_stream(const BwdP
     }
     if (B.gm) { B.gm[3 * i] = gm[0]; B.gm[3 * i + 1] = gm[1]; B.gm[3 * i + 2] = gm[2]; }
     if (B.gd) { B.gd[3 * i] = gdv[0]; B.gd[3 * i + 1] = gdv[1]; B.gd[3 * i + 2] = gdv[2]; }
-    if (hi - j <= blockDim.x) break;  // j + blockDim.x may pass 2^32
   }
 }
 
@@ -624,6 +622,9 @@ extern "C" int rmg_umeyama_backward(const rmg_transform* pre_transforms, uint32_
     if (n_batches == 0) return RMG_OK;
     if (!stats) return fail(RMG_ERR_INVALID_ARG, "rmg_umeyama_backward: stats is NULL");
     if (!grad_dataset && !grad_model) return RMG_OK;
+    // the stream kernel counts in 32 bits, a CTA's width at a time
+    if (n_per_batch > 0xffffffffu - (kStatsThreads - 1))
+      return fail(RMG_ERR_INVALID_ARG, "rmg_umeyama_backward: too many correspondences per batch");
     BwdParams B;
     int s = fill_params(pre_transforms, pre_transform_stride, dataset_points, dataset_mask, dataset_ids, model_points,
                         nullptr, model_mask, model_ids, params, n_batches, n_per_batch, B.S);

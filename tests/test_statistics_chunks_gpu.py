@@ -45,3 +45,17 @@ def test_every_correspondence_counts_once(rs, which, shift):
     for part in (slice(0, n // 3), slice(n // 3, n)):
         for a, b in zip(whole, rs.umeyama_backward(d[None, part], m[None, part], st, gR, gt)):
             assert torch.equal(a[:, part], b)
+
+
+def test_backward_of_more_than_it_can_count_is_refused(rs):
+    """Within a CTA's width of 2^32 the stream kernel's count would not come to an end."""
+    from rmagine_gb300 import _lib as L
+
+    x = torch.zeros(64, device="cuda")
+    pc = rs.UmeyamaReductionConstraints().to_c()
+    import ctypes as C
+
+    for n in (0xFFFFFF01, 0xFFFFFFFF):
+        st = L.load().rmg_umeyama_backward(None, 0, rs._ptr(x), None, None, rs._ptr(x), None, None, C.byref(pc), 1, n,
+                                           rs._ptr(x), None, None, rs._ptr(x), rs._ptr(x), rs._stream())
+        assert st == L.RMG_ERR_INVALID_ARG
