@@ -126,7 +126,10 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
   const uint32_t mixed = __ballot_sync(0xffffffffu, !is_zero(pick(j, a[1], a[2], a[0])) || !is_zero(pick(j, a[2], a[0], a[1])));
   const uint32_t some = __ballot_sync(0xffffffffu, !is_zero(pick(j, a[0], a[1], a[2])));
   const bool diagonal = !any4(mixed), zero = !any4(mixed | some);
-  if ((mixed | some) == 0) {
+  uint32_t groups = mixed | mixed >> 1;
+  groups |= groups >> 2;
+  const bool plain = (groups & 0x11111111u) == 0x11111111u;  // none of the warp's is diagonal
+  if (!plain && (mixed | some) == 0) {
     U = V = m3_eye();
     s[0] = s[1] = s[2] = 0.0;
     return true;
@@ -216,7 +219,7 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] += p0 * v[k] + p1 * y[k] + p2 * z[k];
   }
-  if (diagonal) {
+  if (!plain && diagonal) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] = k == j ? 1.0 : 0.0;
   }
@@ -250,10 +253,10 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
 #pragma unroll
   for (int k = 0; k < 3; ++k) u1[k] -= d01 * u0[k];
   double q1 = dot(u1, u1);
-  if (!(q1 > 1e-24 * q0)) {
-    if (!diagonal) {
-      bad = true;
-    } else {  // rank one: any unit vector orthogonal to u0
+  const bool flat = !(q1 > 1e-24 * q0);
+  bad = bad || (flat && !diagonal);
+  if (!plain) {
+    if (flat && diagonal) {  // rank one: any unit vector orthogonal to u0
       const int k = (fabs(u0[0]) <= fabs(u0[1]) && fabs(u0[0]) <= fabs(u0[2])) ? 0 : (fabs(u0[1]) <= fabs(u0[2]) ? 1 : 2);
       const double u0k = pick(k, u0[0], u0[1], u0[2]);
 #pragma unroll
@@ -276,7 +279,7 @@ __device__ __forceinline__ bool svd3_lanes(const M3d& C, M3d& U, double s[3], M3
     s[k] = of4(sj, k);
   }
   if (any4(__ballot_sync(0xffffffffu, bad))) svd3_rot(C, U, s, V);
-  if (zero) {
+  if (!plain && zero) {
     U = V;
     s[0] = s[1] = s[2] = 0.0;
   }
